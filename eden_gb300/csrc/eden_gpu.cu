@@ -157,6 +157,22 @@ struct EdenGpuCtx {
 #include "eden_codegen.cuh"
 
 namespace {
+// Raises a kernel's dynamic shared-memory limit on a device to at least
+// `bytes`.  The limit belongs to the kernel, which the contexts of a process
+// share (a compiled one with every context of the same source), so it is
+// never lowered: a context created later with smaller cells must not take it
+// below what an earlier one launches with.
+cudaError_t raise_smem_limit(const void *fn, int device, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, size_t> limit;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t &have = limit[{fn, device}];
+    if (bytes <= have) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) have = bytes;
+    return e;
+}
+
 // Launch of a kernel given by handle (a built-in __global__ function or a
 // kernel loaded from the model's compiled library).
 template <typename... A>
@@ -1630,10 +1646,10 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             if (codegen == 1) return ctx->fail(EDEN_GPU_E_CUDA, "code generation failed: %s", why.c_str());
         }
     }
-    CUDA_TRY(ctx, cudaFuncSetAttribute(k_hines_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_hines));
+    CUDA_TRY(ctx, raise_smem_limit((const void *)k_hines_t, ctx->device, ctx->smem_hines));
     if (ctx->smem_window)
-        CUDA_TRY(ctx, cudaFuncSetAttribute(ctx->fn_cells, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)std::min<size_t>(max_smem_class, (size_t)ctx->smem_optin)));
+        CUDA_TRY(ctx, raise_smem_limit(ctx->fn_cells, ctx->device,
+                                       std::min<size_t>(max_smem_class, (size_t)ctx->smem_optin)));
     {
         // resident input blocks only: each warp then walks several chunks
         int per_sm = 1;

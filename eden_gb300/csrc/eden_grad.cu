@@ -1100,8 +1100,10 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
         return g->fail(EDEN_GPU_E_INVALID, "largest cell (%d compartments, %d gates) needs %zu bytes of shared memory, "
                                            "the device allows %d", dm.c, dm.g, g->smem, optin);
     if (g->smem > 48 * 1024) {
-        GTRY(g, cudaFuncSetAttribute(k_grad_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g->smem));
-        GTRY(g, cudaFuncSetAttribute(k_grad_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g->smem));
+        // (the limit belongs to the kernels, which every context launches: the
+        // device's own, so that no context lowers another's)
+        GTRY(g, cudaFuncSetAttribute(k_grad_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        GTRY(g, cudaFuncSetAttribute(k_grad_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     }
     std::vector<EdenGpuChannelType> types(m->chan_types, m->chan_types + m->n_chan_types);
     int rc;
