@@ -102,6 +102,7 @@ struct EdenGpuCtx {
     int gcap = 0, forest_cap = 0;           // largest cell / compartments per staged forest
     bool smem_window = false;              // groups fit shared memory
     int max_cell_blocks = 0;               // most blocks of a k_cells_t launch
+    int cell_threads = 128;                // threads of a k_cells_t block
     std::vector<int64_t> h_ext_step;       // logging steps of the spike sources' events
     size_t smem_hines = 0;
     struct CellClass { int cta_begin, cta_end; size_t smem; };
@@ -599,24 +600,22 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // window -- a forest of physical cells (joint breadth-first numbering,
     // at most kForestWidth nodes per depth level, at most kForestNodes nodes) or a batch
     // of up to 32 izhikevich neurons.  Targets are numbered unit by unit.
-    // Small networks get smaller forests, so that at least about four units
-    // per SM run (a window's time is that of its slowest warp); large ones
-    // fill forests up to kForestNodes.
+    // Small networks get smaller forests, so that about twelve units per SM run
+    // (a window's time is that of its slowest warp, and a step's chain leaves
+    // room for as many: 30,011 cells of one compartment took 5.3 us a step in
+    // units of 50, 3.3 in units of 16); large ones fill forests up to
+    // kForestNodes.
     int forest_node_cap = kForestNodes;
     const int forest_width = (opt && opt->segments_per_depth > 0) ? std::min(opt->segments_per_depth, 1023) : kForestWidth;
     if (opt && opt->segments_per_warp > 0) {
         forest_node_cap = std::min(opt->segments_per_warp, 1023);
     } else {
         int64_t n_phys_comp = 0;
-        int largest = 1;
         for (int k = 0; k < n_cells; k++)
-            if (cell_phys[k] >= 0) {
-                n_phys_comp += cell_n[k];
-                largest = std::max(largest, cell_n[k]);
-            }
-        const int64_t units = 4 * (int64_t)std::max(ctx->n_sm, 1);
+            if (cell_phys[k] >= 0) n_phys_comp += cell_n[k];
+        const int64_t units = 12 * (int64_t)std::max(ctx->n_sm, 1);
         const int64_t even = (n_phys_comp + units - 1) / units;
-        forest_node_cap = (int)std::min<int64_t>(kForestNodes, std::max<int64_t>({even, (int64_t)largest, 8}));
+        forest_node_cap = (int)std::min<int64_t>(kForestNodes, std::max<int64_t>(even, 8));
     }
     std::vector<int32_t> u2i(nt, -1), i2u(nt, -1);
     std::vector<int32_t> c_parent(nt, -1), c_child0(nt, 0), c_nchild(nt, 0), t_izh(nt, -1);
@@ -850,7 +849,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // the same every step and are computed here once, deepest first
     std::vector<char> nonflat(nt, 1);
     std::vector<float> c_kc(nt, 0.f), c_pv0(nt, 0.f), c_rt0(nt, 0.f);
-    std::vector<uint32_t> c_cep(nt, 0);
     {
         std::vector<char> is_src(nt, 0);
         for (int s = 0; s < m->n_src; s++)
@@ -871,35 +869,174 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                     c_pv0[it] = inv;
                     c_rt0[it] = c_l[it] * inv;
                 }
-                const uint32_t cb = k1 > k0 ? (uint32_t)(k0 - a) : 0u, ce = k1 > k0 ? (uint32_t)(k1 - a) : 0u;
-                const uint32_t pp = c_parent[it] >= 0 ? (uint32_t)(c_parent[it] - a + 1) : 0u;
-                c_cep[it] = ce | (cb << kCepBeginShift) | (pp << kCepParentShift) | (nonflat[it] ? kCepNonFlat : 0u);
             }
         }, 32);
     }
-    // a flat compartment's pre-update increment, or a non-flat one's L
-    std::vector<float> c_kl(nt, 0.f);
-    for (int it = 0; it < nt; it++) c_kl[it] = nonflat[it] ? c_l[it] : c_kc[it];
-
-    // per forest depth (parallel to lvl): non-flat flag
-    std::vector<uint8_t> lvl_info(lvl.size(), 0);
-    for (size_t f = 0; f < fo_t0.size(); f++)
-        for (int l = 0; l < fo_nlev[f]; l++)
-            for (int it = lvl[fo_l0[f] + l]; it < lvl[fo_l0[f] + l + 1]; it++)
-                if (nonflat[it]) lvl_info[fo_l0[f] + l] = 0x80;
-    // gate parameter records per channel type and gate (gate_next_p)
-    std::vector<float> gate_par((size_t)std::max(m->n_chan_types, 1) * EDEN_MAX_GATES * kGateWords, 0.f);
-    for (int k = 0; k < m->n_chan_types; k++) {
-        const EdenGpuChannelType &ty = m->chan_types[k];
-        for (int g = 0; g < ty.n_gates; g++) {
-            float *r = &gate_par[((size_t)k * EDEN_MAX_GATES + g) * kGateWords];
-            int32_t fk = ty.fwd_kind[g], rk = ty.rev_kind[g];
-            if (ty.gate_kind[g] != EDEN_GATE_RATES) fk |= (1 + k * EDEN_MAX_GATES + g) << 8;
-            memcpy(&r[0], &fk, 4); r[1] = ty.fwd_rate[g]; r[2] = ty.fwd_mid[g]; r[3] = ty.fwd_scale[g];
-            memcpy(&r[4], &rk, 4); r[5] = ty.rev_rate[g]; r[6] = ty.rev_mid[g]; r[7] = ty.rev_scale[g];
-            r[8] = ty.q10[g];
+    // ---- nodes and twigs of each forest (DevModel::c_rec, hines_window), forests
+    // on the host's threads.  A twig is a flat subtree of at most `most`
+    // compartments; the twigs go to the lanes, large ones first, each to the
+    // lane with the fewest so far, a lane's places filled from the bottom row.
+    // `most` is the one of a few sizes with the cheapest step, by the
+    // instructions of a depth, a child and a row that hines_window counts.
+    auto bits = [](int32_t x) { float f; memcpy(&f, &x, 4); return f; };
+    struct ForestRec {
+        std::vector<float4> node, place;
+        std::vector<float> rt;
+        std::vector<int32_t> nd_t, tw_t, ps;
+        std::vector<uint32_t> adr;
+    };
+    std::vector<ForestRec> frec(fo_t0.size());
+    std::vector<int32_t> node_of(nt, -1), place_of(nt, -1);  // each compartment's node or twig place
+    std::vector<char> no_pass(nt, 0);
+    const bool make_twigs = !opt || opt->mode == EDEN_MODE_BATCHED;
+    parallel_for((int64_t)fo_t0.size(), [&](int64_t f) {
+        const int a = fo_t0[f], n = fo_t1[f] - a;
+        if (n > 1023) return;  // (such a forest runs the per-step kernels)
+        ForestRec &fr = frec[f];
+        std::vector<int32_t> size(n, 1), depth(n, 0);  // (non-flat compartments: size over any limit)
+        for (int i = n - 1; i >= 0; i--) {
+            if (nonflat[a + i]) size[i] = 1 << 20;
+            if (c_parent[a + i] >= 0) size[c_parent[a + i] - a] += size[i];
         }
+        for (int i = 0; i < n; i++)
+            if (c_parent[a + i] >= 0) depth[i] = depth[c_parent[a + i] - a] + 1;
+        // 0: a node, 1: a twig's topmost compartment, 2: below it
+        auto part = [&](int most, int i) {
+            if (size[i] > most) return 0;
+            return size[c_parent[a + i] - a] > most ? 1 : 2;
+        };
+        int best = 0;
+        if (!fo_f64[f] && make_twigs) {
+            int64_t cheapest = INT64_MAX;
+            for (int most : {0, 3, 6, 9, 12, 16, 20, 26, 32, 40, 50, 64}) {
+                std::vector<int32_t> count(fo_nlev[f], 0), kids(fo_nlev[f], 0);
+                std::vector<int32_t> twigs;
+                for (int i = 0; i < n; i++) {
+                    const int q = part(most, i);
+                    if (q == 0) { count[depth[i]]++; kids[depth[i]] = std::max(kids[depth[i]], c_nchild[a + i]); }
+                    else if (q == 1) twigs.push_back(size[i]);
+                }
+                std::sort(twigs.begin(), twigs.end(), std::greater<int>());
+                int rows = 0;
+                {
+                    std::vector<int> load(32, 0);
+                    for (int t : twigs) {
+                        auto l = std::min_element(load.begin(), load.end());
+                        *l += t;
+                        rows = std::max(rows, *l);
+                    }
+                }
+                int64_t cost = 22 * (int64_t)rows;
+                for (int l = 0; l < fo_nlev[f]; l++) cost += (count[l] + 31) / 32 * (42 + 5 * kids[l]);
+                // (addresses of twig places have 15 bits)
+                const int words = twig_words(n + 1) + 64 * rows;
+                if (cost < cheapest && words < (int)kTwigTop) { cheapest = cost; best = most; }
+            }
+        }
+        // nodes, in the compartments' order: a depth's are consecutive, and a node's children
+        std::vector<int32_t> nodes, tops;
+        for (int i = 0; i < n; i++) {
+            const int q = part(best, i);
+            if (q < 2) { node_of[a + i] = (int)nodes.size(); nodes.push_back(i); }
+            if (q == 1) tops.push_back(i);
+        }
+        for (int i : nodes) {
+            const int it = a + i, q = part(best, i);
+            const uint32_t nk = q == 0 ? (uint32_t)c_nchild[it] : 0u;
+            const uint32_t cb = nk > 0 ? (uint32_t)node_of[c_child0[it]] : 0u;
+            const uint32_t pp = c_parent[it] >= 0 ? (uint32_t)node_of[c_parent[it]] : 0u;
+            const uint32_t w = nk | (cb << kCepBeginShift) | (pp << kCepParentShift) | (nonflat[it] ? kCepNonFlat : 0u) |
+                               (q == 1 ? kCepTwig : 0u);
+            fr.node.push_back(make_float4(nonflat[it] ? c_l[it] : c_kc[it], c_u[it],
+                                          fo_f64[f] ? (nonflat[it] ? 0.0f : flat_d0[it]) : c_pv0[it], bits((int32_t)w)));
+            fr.rt.push_back(c_rt0[it]);
+            fr.nd_t.push_back(q == 1 ? -1 - i : i);
+        }
+        // passes over the depths with a node that is no twig's
+        for (size_t j0 = 0; j0 < nodes.size();) {
+            size_t j1 = j0;
+            while (j1 < nodes.size() && depth[nodes[j1]] == depth[nodes[j0]]) j1++;
+            const size_t first = fr.ps.size();
+            for (size_t j = j0; j < j1; j += 32) {
+                const int cnt = (int)std::min<size_t>(32, j1 - j);
+                int32_t d = (int32_t)j | (cnt << kPassCountShift), kids = 0;
+                bool done = depth[nodes[j0]] == 0 && !fo_f64[f], any = false;
+                for (size_t k = j; k < j + cnt; k++) {
+                    const int it = a + nodes[k];
+                    if (part(best, nodes[k]) == 0) {
+                        any = true;
+                        kids = std::max(kids, c_nchild[it]);
+                    }
+                    if (nonflat[it]) d |= kPassNonFlat;
+                    done = done && nonflat[it] && c_nchild[it] == 0;
+                }
+                // (cells of one compartment are finished with their currents)
+                for (size_t k = j; done && k < j + cnt; k++) no_pass[a + nodes[k]] = 1;
+                if (depth[nodes[j0]] == 0) d |= kPassRoot;
+                if (any && !done) fr.ps.push_back(d | kids << kPassKidsShift);
+            }
+            if (fr.ps.size() > first) {
+                fr.ps[first] |= kPassFirst;
+                fr.ps.back() |= kPassLast;
+            }
+            j0 = j1;
+        }
+        // the twigs' places
+        std::stable_sort(tops.begin(), tops.end(), [&](int x, int y) { return size[x] > size[y]; });
+        std::vector<std::vector<int32_t>> lane(32);
+        for (int t : tops) {
+            auto l = std::min_element(lane.begin(), lane.end(), [](const auto &x, const auto &y) { return x.size() < y.size(); });
+            // children first, in increasing order
+            std::vector<std::pair<int32_t, int32_t>> stack{{t, 0}};
+            while (!stack.empty()) {
+                auto &[i, k] = stack.back();
+                if (k < c_nchild[a + i]) {
+                    const int c = c_child0[a + i] - a + k++;
+                    stack.push_back({c, 0});
+                } else {
+                    l->push_back(i);
+                    stack.pop_back();
+                }
+            }
+        }
+        size_t rows = 0;
+        for (auto &l : lane) rows = std::max(rows, l.size());
+        const int base = twig_words((int)nodes.size() + 1), tv = base + 32 * (int)rows;
+        for (int l = 0; l < 32; l++)
+            for (size_t r = 0; r < lane[l].size(); r++) place_of[a + lane[l][r]] = (int32_t)(32 * r + l);
+        fr.place.assign(32 * rows, make_float4(0.f, 0.f, 0.f, 0.f));
+        fr.tw_t.assign(32 * rows, -1);
+        // (an empty place works on itself, with zeros)
+        for (size_t k = 0; k < 32 * rows; k++) fr.adr.push_back((uint32_t)(base + k) | (uint32_t)(tv + k) << 16);
+        for (int l = 0; l < 32; l++)
+            for (size_t r = 0; r < lane[l].size(); r++) {
+                const size_t k = 32 * r + l;
+                const int i = lane[l][r], it = a + i, up = c_parent[it];
+                const bool top = part(best, i) == 1;
+                fr.place[k] = make_float4(c_kc[it], c_u[it], c_pv0[it], c_rt0[it]);
+                fr.tw_t[k] = i;
+                fr.adr[k] = top ? (uint32_t)(2 * node_of[it]) | kTwigTop | (uint32_t)(2 * node_of[up]) << 16
+                                : (uint32_t)(base + place_of[up]) | (uint32_t)(tv + place_of[up]) << 16;
+            }
+    }, 32);
+    std::vector<float4> c_rec, tw_rec;
+    std::vector<float> nd_rt;
+    std::vector<int32_t> fo_n0(fo_t0.size() + 1, 0), fo_w0(fo_t0.size() + 1, 0), fo_p0(fo_t0.size() + 1, 0), nd_t, tw_t, ps;
+    std::vector<uint32_t> tw_adr;
+    for (size_t f = 0; f < fo_t0.size(); f++) {
+        const ForestRec &fr = frec[f];
+        c_rec.insert(c_rec.end(), fr.node.begin(), fr.node.end());
+        nd_rt.insert(nd_rt.end(), fr.rt.begin(), fr.rt.end());
+        nd_t.insert(nd_t.end(), fr.nd_t.begin(), fr.nd_t.end());
+        ps.insert(ps.end(), fr.ps.begin(), fr.ps.end());
+        tw_rec.insert(tw_rec.end(), fr.place.begin(), fr.place.end());
+        tw_t.insert(tw_t.end(), fr.tw_t.begin(), fr.tw_t.end());
+        tw_adr.insert(tw_adr.end(), fr.adr.begin(), fr.adr.end());
+        fo_n0[f + 1] = (int32_t)c_rec.size();
+        fo_w0[f + 1] = (int32_t)(tw_t.size() / 32);
+        fo_p0[f + 1] = (int32_t)ps.size();
     }
+    frec.clear();
 
     // kinds and timeCourse / steadyState forms of the gates of other kinds
     // than gateHHrates, by channel type and gate (gate_next_p)
@@ -1123,6 +1260,17 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         ck_info[c] = (bk_kind[ck_blk[c]] == BK_CLAMPV ? BK_PULSE : (bk_kind[ck_blk[c]] & BK_KIND_MASK)) |
                      ((int32_t)bk_type[ck_blk[c]] << 2) | (ck_n[c] << 8);
 
+    // each block's record in the windowed kernel, its chunks counted in its unit
+    std::vector<int4> bk_rec(n_block);
+    for (size_t u = 0; u < un_t0.size(); u++) {
+        const int b0 = t_blk0[un_t0[u]], b1 = t_blk0[un_t1[u]];
+        for (int b = b0; b < b1; b++) {
+            int32_t e;
+            memcpy(&e, &bk_erev[b], 4);
+            bk_rec[b] = make_int4(bk_c0[b] - bk_c0[b0], bk_c0[b + 1] - bk_c0[b0], bk_kind[b], e);
+        }
+    }
+
     // ---- window length: every delay must cover the window (see k_window)
     int kmax = kMaxWindow;
     if (ns > 0) {
@@ -1179,51 +1327,58 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // ---- per-unit lists of the windowed kernel: spike sources and recorded
     // targets (unit-local indices), gates, and each unit's shared-memory words
     const int n_unit = (int)un_t0.size();
-    std::vector<int32_t> un_gt0(n_unit), un_ngt(n_unit), un_s0(n_unit), un_s1(n_unit), un_r0(n_unit), un_r1(n_unit);
-    std::vector<int32_t> gs_t, gs_src, gr_t, gr_col;
-    std::vector<float> gs_thr;
-    std::vector<int32_t> un_nf0(n_unit), un_nf1(n_unit), nf_t;
+    std::vector<int32_t> un_gt0(n_unit), un_ngt(n_unit), un_r0(n_unit), un_r1(n_unit);
+    std::vector<int32_t> gr_t, gr_col;
+    std::vector<int32_t> un_nf0(n_unit), un_nf1(n_unit), un_ch0(n_unit), un_ch1(n_unit), nf_t;
     std::vector<int> un_words(n_unit);
-    {
-        std::vector<int32_t> slot_of(nt, -1);
-        for (int u = 0; u < n_unit; u++) {
-            const int a = un_t0[u], b = un_t1[u];
-            un_nf0[u] = (int)nf_t.size();
-            if (un_f[u] >= 0)
-                for (int t = a; t < b; t++)
-                    if (nonflat[t]) { slot_of[t] = (int)nf_t.size() - un_nf0[u]; nf_t.push_back(t - a); }
-            un_nf1[u] = (int)nf_t.size();
-        }
-        for (int u = 0; u < n_unit; u++) {
-            const int a = un_t0[u], b = un_t1[u];
-            un_s0[u] = (int)gs_t.size();
-            if (un_f[u] >= 0)
-                for (int t = a; t < b; t++)
-                    if (t_src[t] >= 0) { gs_t.push_back(slot_of[t]); gs_src.push_back(t_src[t]); gs_thr.push_back(src_thr[t_src[t]]); }
-            un_s1[u] = (int)gs_t.size();
-        }
+    for (int u = 0; u < n_unit; u++) {
+        const int a = un_t0[u], b = un_t1[u];
+        un_nf0[u] = (int)nf_t.size();
+        if (un_f[u] >= 0)
+            for (int t = a; t < b; t++)
+                if (nonflat[t]) nf_t.push_back(t - a);
+        un_nf1[u] = (int)nf_t.size();
     }
-    // channels of each unit's non-flat compartments, in slot order, and the
-    // channel set of each (the generated code has one routine per set)
-    std::vector<int32_t> nf_c0(nf_t.size()), nf_c1(nf_t.size()), nfc_q, nfc_i, nf_sig(nf_t.size(), -1);
+    // the records of each unit's non-flat compartments (slots) and gates, and
+    // the slots' channels, in slot order, with the channel set of each (the
+    // generated code has one routine per set)
+    std::vector<float4> nf_rec(kSlotRecs * nf_t.size()), gate_tab((size_t)kGateRecs * EDEN_MAX_GATES * std::max(m->n_chan_types, 1));
+    std::vector<int32_t> gt_idx(n_gate);
+    std::vector<float2> nf_ts(nf_t.size());
+    std::vector<int32_t> nfc_q, nfc_i;
     std::map<std::vector<int>, int> set_id;
     std::vector<std::vector<int>> chan_sets;
     std::vector<float> nfc_g, nfc_e;
     for (int u = 0; u < n_unit; u++) {
         const int a = un_t0[u];
         const int gbase = ch_gate0[c_chan0[a]];
+        un_ch0[u] = (int)nfc_g.size();
         for (int k = un_nf0[u]; k < un_nf1[u]; k++) {
             const int t = a + nf_t[k];
-            nf_c0[k] = (int)nfc_g.size();
             std::vector<int> set;
             for (int ch = c_chan0[t]; ch < c_chan0[t + 1]; ch++) set.push_back(ch_type[ch]);
+            int32_t sig = -1;
             auto found = set_id.find(set);
             if (found != set_id.end()) {
-                nf_sig[k] = found->second;
+                sig = found->second;
             } else if (chan_sets.size() < 64) {
-                nf_sig[k] = (int)chan_sets.size();
-                set_id[set] = nf_sig[k];
+                sig = (int)chan_sets.size();
+                set_id[set] = sig;
                 chan_sets.push_back(set);
+            }
+            // (blocks and channels counted in the unit: a unit's slice of shared
+            // memory holds fewer than 65536 of either)
+            const int32_t b0 = t_blk0[t] - t_blk0[a], b1 = t_blk0[t + 1] - t_blk0[a];
+            const int32_t c0 = (int32_t)nfc_g.size() - un_ch0[u], nc = c_chan0[t + 1] - c_chan0[t];
+            const int32_t flags = no_pass[t] ? kSlotDone : 0;
+            nf_rec[kSlotRecs * k] = make_float4(bits(node_of[t] | flags), c_area[t], c_cm[t], known_reciprocal(c_cm[t]));
+            nf_rec[kSlotRecs * k + 1] = make_float4(c_inv[t], bits((int32_t)((uint32_t)b0 | (uint32_t)b1 << 16)),
+                                                    bits((int32_t)((uint32_t)c0 | (uint32_t)nc << 16)), bits(sig));
+            nf_ts[k] = make_float2(t_src[t] >= 0 ? src_thr[t_src[t]] : NAN, bits(t_src[t]));
+            for (int ch = c_chan0[t]; ch < c_chan0[t + 1]; ch++) {
+                const EdenGpuChannelType &ty = m->chan_types[ch_type[ch]];
+                for (int g = 0; g < ty.n_gates; g++)
+                    gt_idx[ch_gate0[ch] + g] = (k - un_nf0[u]) | (ch_type[ch] * EDEN_MAX_GATES + g) << 10;
             }
             for (int ch = c_chan0[t]; ch < c_chan0[t + 1]; ch++) {
                 const EdenGpuChannelType &ty = m->chan_types[ch_type[ch]];
@@ -1232,17 +1387,33 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                 nfc_g.push_back(ch_g[ch]); nfc_e.push_back(ch_e[ch]);
                 nfc_q.push_back(ch_gate0[ch] - gbase); nfc_i.push_back(pack);
             }
-            nf_c1[k] = (int)nfc_g.size();
+        }
+        un_ch1[u] = (int)nfc_g.size();
+    }
+    for (int k = 0; k < m->n_chan_types; k++) {
+        const EdenGpuChannelType &ty = m->chan_types[k];
+        for (int g = 0; g < ty.n_gates; g++) {
+            float4 *r = &gate_tab[(size_t)kGateRecs * (k * EDEN_MAX_GATES + g)];
+            // (a gate of another kind: 1 + its row of gate_ext)
+            const int32_t row = ty.gate_kind[g] != EDEN_GATE_RATES ? 1 + k * EDEN_MAX_GATES + g : 0;
+            r[0] = make_float4(bits((ty.fwd_kind[g] & 15) | (ty.rev_kind[g] & 15) << 4 | row << 8), ty.fwd_rate[g],
+                               ty.fwd_mid[g], ty.fwd_scale[g]);
+            r[1] = make_float4(0.f, ty.rev_rate[g], ty.rev_mid[g], ty.rev_scale[g]);
+            r[2] = make_float4(ty.q10[g], known_reciprocal(ty.fwd_scale[g]), known_reciprocal(ty.rev_scale[g]), 0.f);
         }
     }
     for (int u = 0; u < n_unit; u++) {
         const int a = un_t0[u], b = un_t1[u];
         un_gt0[u] = ch_gate0[c_chan0[a]];
-        // a unit's trace columns: its local target, or -1 - its local gate slot
+        // a unit's trace columns: a node or a twig place (a point neuron's local
+        // target), or -1 - its local gate slot
         un_r0[u] = (int)gr_t.size();
         for (int t = a; t < b; t++)
             for (int k = t_trace0[t]; k < t_trace0[t + 1]; k++) {
-                gr_t.push_back(trace_gate[k] < 0 ? t - a : -1 - (trace_gate[k] - un_gt0[u]));
+                gr_t.push_back(trace_gate[k] >= 0   ? -1 - (trace_gate[k] - un_gt0[u])
+                               : un_f[u] < 0        ? t - a
+                               : place_of[t] >= 0   ? place_of[t] << 1 | 1
+                                                    : node_of[t] << 1);
                 gr_col.push_back(trace_col[k]);
             }
         un_r1[u] = (int)gr_t.size();
@@ -1250,35 +1421,47 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         if (un_f[u] >= 0) {
             const int nblk = t_blk0[b] - t_blk0[a];
             const int nck = bk_c0[t_blk0[b]] - bk_c0[t_blk0[a]];
-            const int nfch = un_nf1[u] > un_nf0[u] ? nf_c1[un_nf1[u] - 1] - nf_c0[un_nf0[u]] : 0;
-            un_words[u] = forest_words(b - a, un_nf1[u] - un_nf0[u], nfch, un_ngt[u], fo_nlev[un_f[u]],
-                                       un_s1[u] - un_s0[u], nblk, nck, std::max(ctx->K, 4), fo_f64[un_f[u]] != 0);
+            const int f = un_f[u];
+            un_words[u] = forest_words(fo_n0[f + 1] - fo_n0[f], fo_w0[f + 1] - fo_w0[f], un_nf1[u] - un_nf0[u], un_ch1[u] - un_ch0[u], un_ngt[u],
+                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, nck, std::max(ctx->K, 4),
+                                       fo_f64[un_f[u]] != 0);
         } else {
             un_words[u] = izh_words(b - a);
         }
     }
     phase("packing");
-    // CTAs of up to four units, packed longest-first onto the CTA with the
-    // fewest words so that every CTA needs about the same shared memory; a
-    // network of more CTAs than SMs gets a multiple of the SM count of them
-    // (some then hold three units), so that every SM runs as many (1 % faster
-    // on C2).  (Packing by an estimate of each unit's work instead measured
-    // 3 % slower.)
-    const int upc = kCellThreads / 32;
-    int n_cta = (n_unit + upc - 1) / upc;
-    if (n_cta > ctx->n_sm) n_cta = std::min(n_unit, (n_cta + ctx->n_sm - 1) / ctx->n_sm * ctx->n_sm);
+    // CTAs: a window's time is that of its slowest SM, so where all units fit the
+    // SMs' shared memory at once, every SM gets the same number of CTAs, as many
+    // as they can be (at most six) and still be resident together; else CTAs of
+    // up to four units take turns.  Units go longest-first onto the CTA with the
+    // fewest words.  (On the batched multicompartment network, 10,000 cells in
+    // 35 MB, CTAs of four needed a second round for a quarter of them.)
+    const int most = (int)(ctx->smem_optin / sizeof(float)) - 4 * kPassPad;  // words of one block
     std::vector<int> uorder(n_unit);
     std::iota(uorder.begin(), uorder.end(), 0);
     std::stable_sort(uorder.begin(), uorder.end(), [&](int x, int y) { return un_words[x] > un_words[y]; });
-    std::vector<std::vector<int>> cta_units(n_cta);
-    std::vector<int> cta_words(n_cta, 0);
-    {
+    std::vector<std::vector<int>> cta_units;
+    std::vector<int> cta_words;
+    int n_cta = 0;
+    // true if no CTA holds more than `limit` words and `upc` units (more CTAs
+    // where `grow`)
+    auto pack = [&](int ctas, int upc, int limit, bool grow) {
+        n_cta = ctas;
+        cta_units.assign(n_cta, {});
+        cta_words.assign(n_cta, 0);
         // min-heap of (words, cta) over CTAs that still have room
         std::vector<std::pair<int, int>> heap;
         for (int c = 0; c < n_cta; c++) heap.push_back({0, c});
         auto cmp = [](const std::pair<int, int> &x, const std::pair<int, int> &y) { return x > y; };
         std::make_heap(heap.begin(), heap.end(), cmp);
         for (int uu : uorder) {
+            if (heap.empty() || (heap.front().first > 0 && heap.front().first + un_words[uu] > limit)) {
+                if (!grow) return false;
+                heap.push_back({0, n_cta++});
+                cta_units.emplace_back();
+                cta_words.push_back(0);
+                std::push_heap(heap.begin(), heap.end(), cmp);
+            }
             std::pop_heap(heap.begin(), heap.end(), cmp);
             auto top = heap.back();
             heap.pop_back();
@@ -1289,7 +1472,27 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                 std::push_heap(heap.begin(), heap.end(), cmp);
             }
         }
+        for (int w : cta_words)
+            if (w > limit) return grow;
+        return true;
+    };
+    {
+        const int sms = std::max(ctx->n_sm, 1), warps = kCellThreads / 32;
+        bool fits = false;
+        if (n_unit <= sms) fits = pack(n_unit, 1, most, true);
+        for (int per_sm = 6; !fits && per_sm >= 1; per_sm--) {
+            const int upc = warps / per_sm;
+            if ((int64_t)sms * per_sm * upc < n_unit) continue;
+            const int ctas = std::min(sms * per_sm, n_unit);
+            // (a block's own share of the SM: its words, padding and 1 KB of the system's)
+            const int share = (int)(ctx->smem_per_sm / per_sm / sizeof(float)) - 4 * kPassPad - 256;
+            fits = pack(ctas, upc, std::min(most, share), false);
+        }
+        if (!fits) pack((n_unit + 3) / 4, 4, most, true);
     }
+    int max_units = 1;
+    for (auto &c : cta_units) max_units = std::max(max_units, (int)c.size());
+    ctx->cell_threads = 32 * max_units;
     std::vector<int32_t> cta_u0, un_off(n_unit, 0), unit_of_slot;
     for (int c = 0; c < n_cta; c++) {
         cta_u0.push_back((int)unit_of_slot.size());
@@ -1302,7 +1505,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         for (size_t j = 0; j < unit_of_slot.size(); j++) o[j] = v[unit_of_slot[j]];
         v.swap(o);
     };
-    for (auto *v : {&un_t0, &un_t1, &un_f, &un_gt0, &un_ngt, &un_s0, &un_s1, &un_r0, &un_r1, &un_nf0, &un_nf1}) perm(*v);
+    for (auto *v : {&un_t0, &un_t1, &un_f, &un_gt0, &un_ngt, &un_ch0, &un_ch1, &un_r0, &un_r1, &un_nf0, &un_nf1}) perm(*v);
     {
         std::vector<int> w2(n_unit);
         for (int j = 0; j < n_unit; j++) w2[j] = un_words[unit_of_slot[j]];
@@ -1317,6 +1520,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     {
         int mx = 1;
         for (int c = 0; c < n_cta; c++) mx = std::max(mx, cta_words[c]);
+        mx += 4 * kPassPad;
         ctx->classes.push_back({0, n_cta, (size_t)mx * sizeof(float)});
     }
     size_t max_smem_class = 0;
@@ -1359,19 +1563,15 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         }
         TRY(upload_c(ctx, &d.c_rax, c_rax)); TRY(upload_c(ctx, &d.c_kb, c_kb));
     }
-    TRY(upload_c(ctx, &d.c_kl, c_kl)); TRY(upload_c(ctx, &d.c_pv0, c_pv0));
-    TRY(upload_c(ctx, &d.c_rt0, c_rt0)); TRY(upload_c(ctx, &d.c_cep, c_cep)); TRY(upload_c(ctx, &d.t_izh, t_izh));
+    TRY(upload_c(ctx, &d.c_rec, c_rec)); TRY(upload_c(ctx, &d.nd_rt, nd_rt)); TRY(upload_c(ctx, &d.nd_t, nd_t));
+    TRY(upload_c(ctx, &d.fo_n0, fo_n0)); TRY(upload_c(ctx, &d.fo_w0, fo_w0)); TRY(upload_c(ctx, &d.tw_rec, tw_rec));
+    TRY(upload_c(ctx, &d.tw_t, tw_t)); TRY(upload_c(ctx, &d.tw_adr, tw_adr)); TRY(upload_c(ctx, &d.t_izh, t_izh));
     TRY(upload_c(ctx, &d.fo_t0, fo_t0)); TRY(upload_c(ctx, &d.fo_t1, fo_t1)); TRY(upload_c(ctx, &d.fo_l0, fo_l0));
     TRY(upload_c(ctx, &d.fo_nlev, fo_nlev)); TRY(upload_c(ctx, &d.lvl, lvl));
-    {
-        // double-precision forests: flags, the flat compartments' constant
-        // diagonal terms, and the per-step path's double scratch
-        std::vector<float> c_d0(nt, 0.0f);
-        for (int it = 0; it < nt; it++)
-            if (!nonflat[it]) c_d0[it] = flat_d0[it];
-        TRY(upload_c(ctx, &d.fo_f64, fo_f64)); TRY(upload_c(ctx, &d.c_d0, c_d0));
-        TRY(upload(ctx, &d.dscr, (const double *)nullptr, ctx->n_f64_cells > 0 ? (size_t)2 * nt : (size_t)1));
-    }
+    TRY(upload_c(ctx, &d.fo_p0, fo_p0)); TRY(upload_c(ctx, &d.ps, ps));
+    // double-precision forests: flags and the per-step path's double scratch
+    TRY(upload_c(ctx, &d.fo_f64, fo_f64));
+    TRY(upload(ctx, &d.dscr, (const double *)nullptr, ctx->n_f64_cells > 0 ? (size_t)2 * nt : (size_t)1));
     {
         // gap-junction ends per internal target, in the model's order
         std::vector<int32_t> t_gap0(nt + 1, 0), gj_peer(m->n_gap);
@@ -1504,14 +1704,14 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     d.trace_cap = ctx->trace_cap;
     TRY(upload_c(ctx, &d.un_t0, un_t0)); TRY(upload_c(ctx, &d.un_t1, un_t1)); TRY(upload_c(ctx, &d.un_f, un_f));
     TRY(upload_c(ctx, &d.un_off, un_off)); TRY(upload_c(ctx, &d.un_gt0, un_gt0)); TRY(upload_c(ctx, &d.un_ngt, un_ngt));
-    TRY(upload_c(ctx, &d.un_s0, un_s0)); TRY(upload_c(ctx, &d.un_s1, un_s1));
+    TRY(upload_c(ctx, &d.un_ch0, un_ch0)); TRY(upload_c(ctx, &d.un_ch1, un_ch1));
     TRY(upload_c(ctx, &d.un_r0, un_r0)); TRY(upload_c(ctx, &d.un_r1, un_r1)); TRY(upload_c(ctx, &d.cta_u0, cta_u0));
-    TRY(upload_c(ctx, &d.gs_t, gs_t)); TRY(upload_c(ctx, &d.gs_src, gs_src)); TRY(upload_c(ctx, &d.gs_thr, gs_thr));
     TRY(upload_c(ctx, &d.gr_t, gr_t)); TRY(upload_c(ctx, &d.gr_col, gr_col));
-    TRY(upload_c(ctx, &d.un_nf0, un_nf0)); TRY(upload_c(ctx, &d.un_nf1, un_nf1)); TRY(upload_c(ctx, &d.nf_t, nf_t));
-    TRY(upload_c(ctx, &d.lvl_info, lvl_info)); TRY(upload_c(ctx, &d.gate_par, gate_par));
+    TRY(upload_c(ctx, &d.un_nf0, un_nf0)); TRY(upload_c(ctx, &d.un_nf1, un_nf1));
+    TRY(upload_c(ctx, &d.nf_rec, nf_rec)); TRY(upload_c(ctx, &d.nf_ts, nf_ts));
+    TRY(upload_c(ctx, &d.gt_idx, gt_idx)); TRY(upload_c(ctx, &d.gate_tab, gate_tab));
+    TRY(upload_c(ctx, &d.bk_rec, bk_rec));
     TRY(upload_c(ctx, &d.gate_ext, gate_ext));
-    TRY(upload_c(ctx, &d.nf_c0, nf_c0)); TRY(upload_c(ctx, &d.nf_c1, nf_c1)); TRY(upload_c(ctx, &d.nf_sig, nf_sig));
     TRY(upload_c(ctx, &d.nfc_g, nfc_g)); TRY(upload_c(ctx, &d.nfc_e, nfc_e));
     TRY(upload_c(ctx, &d.nfc_q, nfc_q)); TRY(upload_c(ctx, &d.nfc_i, nfc_i));
     TRY(upload(ctx, &d.status, (const int32_t *)nullptr, 1));
@@ -1663,7 +1863,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         fprintf(stderr, "libeden_gpu: set-up %s\n", timing.c_str());
         int occ_cells = 0, occ_inputs = 0;
         if (ctx->smem_window)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cells, ctx->fn_cells, kCellThreads, max_smem_class);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cells, ctx->fn_cells, ctx->cell_threads, max_smem_class);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_inputs, ctx->fn_inputs, kInputThreads, 0);
         fprintf(stderr, "libeden_gpu: kernels %s%s%s (%.0f ms)\n",
                 ctx->codegen_used ? "compiled for this model" : "built in",
@@ -1676,7 +1876,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                 "(%.1f nodes, %.1f levels avg)\n"
                 "libeden_gpu: %d units, %zu size classes; inputs grid %d (%d/SM)\n",
                 nt, m->n_src, (long long)ns, (long long)m->n_pois, n_block, (int)in_tgt.size(), ctx->K,
-                (int)cta_words.size(), kCellThreads, max_smem_class, occ_cells, fo_t0.size(),
+                (int)cta_words.size(), ctx->cell_threads, max_smem_class, occ_cells, fo_t0.size(),
                 fo_t0.empty() ? 0.0 : (double)fnodes / fo_t0.size(), fo_t0.empty() ? 0.0 : (double)flev / fo_t0.size(),
                 n_unit, ctx->classes.size(), ctx->grid_inputs, occ_inputs);
     }
@@ -1850,7 +2050,7 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
         tmark(ctx, EDEN_KERNEL_CELLS, true);
         for (const auto &cl : ctx->classes) {
             const int nb = std::min(cl.cta_end - cl.cta_begin, ctx->max_cell_blocks);
-            launch_k(ctx->fn_cells, nb, kCellThreads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
+            launch_k(ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
                      (const WindowTimes *)ctx->d_wtimes, base, idx, cl.cta_begin, cl.cta_end);
             n++;
         }
@@ -2159,7 +2359,7 @@ static int launch_window_static(EdenGpuCtx *ctx, const DevModel &dm, const Windo
         int n = 1;
         for (const auto &cl : ctx->classes) {
             const int nb = std::min(cl.cta_end - cl.cta_begin, ctx->max_cell_blocks);
-            launch_k(ctx->fn_cells, nb, kCellThreads, cl.smem, s, dm, tab, times, zero, idx, cl.cta_begin,
+            launch_k(ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, dm, tab, times, zero, idx, cl.cta_begin,
                      cl.cta_end);
             n++;
         }

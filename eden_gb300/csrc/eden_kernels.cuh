@@ -113,18 +113,38 @@ struct DevModel {
     // windowed-path constants of each physical compartment.  A "flat"
     // compartment has one gateless channel, no inputs, is no spike source and
     // has only flat compartments below it; everything else is "non-flat".
-    //   c_kl   flat: the pre-update increment dt*(G*E)/C (V' = V + c_kl, the
-    //          reference's V + dt*(I + V*G)/C with I = G*(E - V)); non-flat:
-    //          its L (its elimination factor is L / pivot, rebuilt each step)
-    //   c_pv0  flat: reciprocal of its Hines pivot, which is the same every
-    //          step because nothing below it changes; non-flat: unused
-    //   c_rt0  flat: L / pivot, its elimination factor into its parent
-    //   c_cep  child-range end | child-range begin << 10 | (parent + 1) << 20
-    //          | non-flat << 30, all local to the compartment's forest
-    const float *c_kl, *c_pv0, *c_rt0;
-    const uint32_t *c_cep;
+    // c_rec, one 16-byte record:
+    //   x  flat: the pre-update increment dt*(G*E)/C (V' = V + x, the
+    //      reference's V + dt*(I + V*G)/C with I = G*(E - V)); non-flat:
+    //      its L (its elimination factor is L / pivot, rebuilt each step)
+    //   y  U
+    //   z  flat: reciprocal of its Hines pivot, which is the same every
+    //      step because nothing below it changes (in a double-precision
+    //      forest its constant diagonal term G/C + sum 1/(R C)); non-flat:
+    //      written each step
+    //   w  children | first child << 10 | parent (a root: 0) << 20
+    //      | non-flat << 30 | a twig's topmost << 31, as nodes of the
+    //      compartment's forest
+    // A forest's compartments are its nodes -- the non-flat ones and the flat
+    // ones over a large subtree, solved depth by depth -- and its twigs: flat
+    // subtrees, each walked by one lane (hines_window).  A twig's topmost
+    // compartment is a node too, a leaf of them.  Nodes [fo_n0[f], fo_n0[f + 1]):
+    // c_rec; nd_t, the compartment (local to its unit), or -1 - it for a twig's
+    // topmost; nd_rt, flat: L / pivot, the elimination factor into the parent.
+    // Twigs: rows [fo_w0[f], fo_w0[f + 1]) of 32 places, a lane's compartments
+    // children first; per place tw_rec (the pre-update increment, U, reciprocal
+    // pivot, elimination factor), tw_adr (the word its elimination goes to
+    // | kTwigTop | the word of its parent's V << 16, in the unit's slice of
+    // shared memory) and tw_t, the compartment (-1: empty).
+    const float4 *c_rec, *tw_rec;
+    const float *nd_rt;
+    const int32_t *fo_n0, *nd_t, *fo_w0, *tw_t;
+    const uint32_t *tw_adr;
     // forests: physical compartments [fo_t0, fo_t1), depth boundaries lvl[fo_l0 .. fo_l0 + fo_nlev]
     const int32_t *fo_t0, *fo_t1, *fo_l0, *fo_nlev, *lvl;
+    // the windowed path's warp passes over forest f, ps[fo_p0[f] .. fo_p0[f + 1]),
+    // roots first: up to 32 consecutive compartments of one depth (kPass*)
+    const int32_t *fo_p0, *ps;
     // channels
     const int32_t *c_chan0, *ch_type, *ch_gate0;
     const float *ch_gbase, *ch_erev;
@@ -213,38 +233,40 @@ struct DevModel {
     int64_t trace_cap;
     // units of the windowed kernel, one warp each: targets [un_t0, un_t1),
     // forest un_f (-1: a batch of izhikevich neurons), shared-memory slice at
-    // word un_off of its CTA, gates [un_gt0, un_gt0 + un_ngt), spike sources
-    // gs_*[un_s0 .. un_s1) and recorded targets gr_*[un_r0 .. un_r1)
-    // (target indices local to the unit); CTA c runs units [cta_u0[c], cta_u0[c+1])
+    // word un_off of its CTA, gates [un_gt0, un_gt0 + un_ngt) and recorded
+    // targets gr_*[un_r0 .. un_r1) (target indices local to the unit); CTA c
+    // runs units [cta_u0[c], cta_u0[c+1])
     int32_t n_unit;
-    const int32_t *un_t0, *un_t1, *un_f, *un_off, *un_gt0, *un_ngt, *un_s0, *un_s1, *un_r0, *un_r1;
+    const int32_t *un_t0, *un_t1, *un_f, *un_off, *un_gt0, *un_ngt, *un_r0, *un_r1;
     const int32_t *cta_u0;
-    // per unit: spike sources (gs_*) and trace columns [un_r0, un_r1): gr_t is
-    // the unit-local target, or -1 - the unit-local gate slot of a gate's
-    // state; gr_col the column
-    const int32_t *gs_t, *gs_src, *gr_t, *gr_col;
-    const float *gs_thr;
-    // non-flat compartments of forest units: nf_t[un_nf0[u] .. un_nf1[u]) are
-    // unit-local indices; spike sources (gs_t) and gates refer to these slots
-    const int32_t *un_nf0, *un_nf1, *nf_t;
-    // per forest depth (parallel to lvl): 0x80 if it holds a non-flat compartment
-    const uint8_t *lvl_info;
-    // channels of the non-flat compartments, per non-flat compartment
-    // [nf_c0, nf_c1): conductivity, reversal potential, first gate (index in
-    // the unit's gates) and gate count | instances << (3 + 5 * gate)
-    const int32_t *nf_c0, *nf_c1;
-    const int32_t *nf_sig;            // channel set of each non-flat compartment (generated code), -1: none
+    // per unit: trace columns [un_r0, un_r1): gr_t is the node << 1 or the twig
+    // place << 1 | 1 (of a point neuron the unit-local target), or -1 - the
+    // unit-local gate slot of a gate's state; gr_col the column
+    const int32_t *gr_t, *gr_col;
+    // non-flat compartments ("slots") of forest units, [un_nf0[u], un_nf1[u]):
+    // nf_rec, two 16-byte records a slot (forest_window: node | kSlot*, area,
+    // C, 1/C; sum 1/(R C), block range, channel range, channel set), and nf_ts,
+    // its spike threshold (NaN: no spike source) and source
+    const int32_t *un_nf0, *un_nf1;
+    const float4 *nf_rec;
+    const float2 *nf_ts;
+    // channels of the slots, [un_ch0[u], un_ch1[u]): conductivity, reversal
+    // potential, first gate (index in the unit's gates) and gate count
+    // | instances << (3 + 5 * gate)
+    const int32_t *un_ch0, *un_ch1;
     const float *nfc_g, *nfc_e;
     const int32_t *nfc_q, *nfc_i;
-    // per channel type and gate, the 9-word gate parameter record (gate_next_p)
-    const float *gate_par;
+    // per gate, its slot | row of gate_tab << 10; gate_tab: the parameters of a
+    // gate of a channel type, three 16-byte records (gate_next_p)
+    const int32_t *gt_idx;
+    const float4 *gate_tab;
+    // per input block: its chunks (counted in its unit), kind and reversal potential
+    const int4 *bk_rec;
     int32_t *status;
     // forests whose cells may lose diagonal dominance: their elimination runs
-    // in double precision (hines_window_f64, hines_forest_f64); c_d0 is a
-    // flat compartment's constant diagonal term G/C + sum 1/(R C); dscr is
+    // in double precision (hines_window_f64, hines_forest_f64); dscr is
     // the per-step path's double scratch (two per target)
     const uint8_t *fo_f64;
-    const float *c_d0;
     double *dscr;
     // gap-junction ends of each target [t_gap0[t], t_gap0[t+1]): the peer
     // (internal target), conductance (uS) and weight
@@ -289,29 +311,45 @@ constexpr uint32_t kCepMask = 0x3ffu;
 constexpr int kCepBeginShift = 10;
 constexpr int kCepParentShift = 20;
 constexpr uint32_t kCepNonFlat = 1u << 30;
-constexpr int kGateWords = 9;  // gate parameter record (gate_next_p)
+constexpr uint32_t kCepTwig = 1u << 31;  // a twig's topmost compartment
+constexpr uint32_t kTwigTop = 1u << 15;
+// a slot's node, with
+constexpr int32_t kSlotDone = 1 << 16;  // a cell of one compartment, in no pass: solved with its currents
+// a warp pass over a forest: first compartment | compartments << 10 | most
+// children of one of them << 16 | flags
+constexpr int32_t kPassStart = 0x3ff;
+constexpr int kPassCountShift = 10;
+constexpr int kPassKidsShift = 16;
+constexpr int32_t kPassFirst = 1 << 26;    // the first pass of its depth
+constexpr int32_t kPassLast = 1 << 27;     // the last pass of its depth
+constexpr int32_t kPassRoot = 1 << 28;     // depth 0
+constexpr int32_t kPassNonFlat = 1 << 29;  // holds a non-flat compartment
+constexpr int kPassPad = 32;               // lanes past a pass's end read, and do not use, up to this many records
+constexpr int kGateRecs = 3;      // 16-byte records of a gate (gate_next_p)
+constexpr int kSlotRecs = 2;      // 16-byte records of a non-flat compartment
 constexpr int kGateExtWords = 9;  // a non-rates gate's kind and timeCourse / steadyState forms
 
-// Shared-memory words of a unit's slice in the windowed kernel (an even
-// count, so that every slice starts 8-byte aligned).  A forest: 6 per
-// compartment in three pairs (V and elimination factor; c_kl and the packed
-// child range/parent/flag; U and pivot), 10 per non-flat compartment (local index, V at
-// the step start, area, C, sum of 1/(R C), input-block range, channel
-// range, channel set), 4 per channel of a non-flat compartment, 11 per gate (value,
-// non-flat slot, parameter record), the depth boundaries, 3 per spike
-// source, 3 per input block (kind, reversal potential, chunk start) plus
-// one, and the window's conductance series of the unit's input chunks
-// (kcap steps).  A batch of izhikevich neurons: V
-// twice and 11 parameter / state words per neuron.
-__host__ __device__ inline int forest_words(int n, int nf, int nfch, int ngt, int nlev, int ns, int nblk, int nck,
-                                            int kcap, bool f64 = false) {
+// Shared-memory words of a unit's slice in the windowed kernel (a multiple of
+// four, so that every slice starts 16-byte aligned).  A forest of n nodes (and
+// one of zeros after them) and nw twig rows, what addresses refer to first:
+// pairs, V and elimination factor per node; two words per twig place, pre-updated V and V; then the 16-byte
+// records: one per node, one per twig place, two per non-flat compartment, one
+// per input block; then pairs: threshold and source per non-flat compartment;
+// then words: a twig place's addresses, V at the step's start per non-flat
+// compartment, four per channel of these, three per gate (its index word, its
+// value in alternate steps), the passes, and the window's conductance series of
+// the unit's input chunks (kcap steps).  A batch of izhikevich neurons: V twice
+// and 19 parameter / state words per neuron.
+__host__ __device__ inline int twig_words(int n) { return (2 * n + 3) & ~3; }  // where the twigs' words start
+__host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int nck, int kcap,
+                                            bool f64 = false) {
     // a double-precision forest adds its eliminated values, pivots and
     // factors in double (6 words per compartment, 8-byte aligned)
-    const int w = 6 * n + 10 * nf + 4 * nfch + (2 + kGateWords) * ngt + (nlev + 1) + 3 * ns + 3 * nblk + 1 + kcap * nck +
-                  (f64 ? 6 * n + 2 : 0);
-    return (w + 1) & ~1;
+    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + 2 * nf + 32 * nw + nf +
+                  4 * nfch + 3 * ngt + np + kcap * nck + (f64 ? 6 * n + 2 : 0);
+    return (w + 3) & ~3;
 }
-__host__ __device__ inline int izh_words(int n) { return ((2 + EDEN_POINT_PARAMS + 3) * n + 1 + 1) & ~1; }
+__host__ __device__ inline int izh_words(int n) { return ((2 + EDEN_POINT_PARAMS + 3) * n + 3) & ~3; }
 
 // Per-window arguments: the window covers steps [step0, step0 + K); steps
 // <= 0 are initialisation passes.  The previous window began at step
@@ -354,6 +392,11 @@ __device__ __forceinline__ void stage_word(void *smem_dst, const void *gmem_src)
     unsigned s;
     asm("{\n .reg .u64 a;\n cvta.to.shared.u64 a, %1;\n cvt.u32.u64 %0, a;\n}" : "=r"(s) : "l"(smem_dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void stage_rec(void *smem_dst, const void *gmem_src) {  // 16 bytes, both sides aligned
+    unsigned s;
+    asm("{\n .reg .u64 a;\n cvta.to.shared.u64 a, %1;\n cvt.u32.u64 %0, a;\n}" : "=r"(s) : "l"(smem_dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -935,6 +978,34 @@ __device__ __forceinline__ void block_currents(const float *Gpk, int b0, int b1,
     }
 }
 
+// block_currents from the unit's block records in shared memory (first chunk,
+// end chunk, kind, reversal potential)
+__device__ __forceinline__ void block_currents_rec(const float *Gk, const int4 *BK, int b0, int b1, float v, float &Iin,
+                                                   float &Gin, float &Isyn, float &Gsyn) {
+    Iin = 0.0f; Gin = 0.0f; Isyn = 0.0f; Gsyn = 0.0f;
+#pragma unroll 1
+    for (int bk = b0; bk < b1; bk++) {
+        const int4 r = BK[bk];
+        float g = Gk[r.x];
+#pragma unroll 1
+        for (int c = r.x + 1; c < r.y; c++) g += Gk[c];
+        const int kind = r.z & BK_KIND_MASK;
+        if (EDEN_KIND_CLAMP && kind == BK_CLAMPV) {
+            Iin -= v * g;
+            continue;
+        }
+        // a current is its value times 1, and adds no conductance; the sums a
+        // block is not part of take 0 * anything finite: no branches
+        const bool current = kind == BK_PULSE || (EDEN_KIND_CURRENT && (r.z & BK_CURRENT));
+        const float t = current ? 1.0f : __int_as_float(r.w) - v;
+        const float gi = kind == BK_SYN ? 0.0f : g, gs = kind == BK_SYN ? g : 0.0f;
+        Iin = fmaf(gi, t, Iin);
+        Isyn = fmaf(gs, t, Isyn);
+        Gin += current ? 0.0f : gi;
+        Gsyn += current ? 0.0f : gs;
+    }
+}
+
 __device__ __forceinline__ float gate_next(const ChanTypeDev &ct, int gi, bool init, float dt, float v, float qo) {
     if (EDEN_KIND_GATEFORMS && ct.gk[gi] != EDEN_GATE_RATES)
         return gate_general(ct.gk[gi], ct.fk[gi], ct.fr[gi], ct.fm[gi], ct.fs[gi], ct.rk[gi], ct.rr[gi], ct.rm[gi],
@@ -945,28 +1016,46 @@ __device__ __forceinline__ float gate_next(const ChanTypeDev &ct, int gi, bool i
     return gate_relax(alpha, beta, ct.q10[gi], init, dt, qo);
 }
 
-// The same from a gate's 9-word parameter record (forward form, rate,
-// midpoint, scale; reverse form, rate, midpoint, scale; q10 factor), kept
-// in shared memory by the windowed kernel.  A gate of another kind than
-// gateHHrates carries 1 + its row of `ext` (kind, timeCourse form and its
-// three values, steadyState form and its three values) in the bits of the
-// first word above the forward form.
+// The same from the three parameter records of the windowed kernel's table:
+//   a  forward form | reverse form << 4 | row << 8, forward rate, midpoint, scale
+//   b  0, reverse rate, midpoint, scale
+//   c  q10 factor, known_reciprocal of the forward and of the reverse scale, 0
+// A gate of another kind than gateHHrates carries 1 + its row of `ext` (kind,
+// timeCourse form and its three values, steadyState form and its three values)
+// in the first word above the forms.
 // An instantaneous gate keeps the steady state at the compartment's
 // potential after the step (`vnew`), which is what the next step's currents
 // read as its value.
-__device__ __forceinline__ float gate_next_p(const float *P, const float *ext, bool init, float dt, float v,
-                                             float vnew, float qo) {
-    const int w0 = __float_as_int(P[0]);
+// The value is gate_next's, operation by operation, with three of its seven
+// divisions known in advance (by the scales, and by alpha + beta once
+// 1 / (alpha + beta) is there) and, of the two that the rate forms may take,
+// only those that some lane's forms do.
+__device__ __forceinline__ float gate_next_p(const float4 &a, const float4 &b, const float4 &c, const float *ext,
+                                             bool init, float dt, float v, float vnew, float qo) {
+    const int w0 = __float_as_int(a.x);
     if (EDEN_KIND_GATEFORMS && (w0 >> 8) != 0) {
         const float *X = ext + (size_t)((w0 >> 8) - 1) * kGateExtWords;
         const int gk = __float_as_int(X[0]);
-        return gate_general(gk, w0 & 0xff, P[1], P[2], P[3], __float_as_int(P[4]), P[5], P[6], P[7],
-                            __float_as_int(X[1]), X[2], X[3], X[4], __float_as_int(X[5]), X[6], X[7], X[8], P[8],
-                            init, dt, gk == EDEN_GATE_INSTANTANEOUS ? vnew : v, qo);
+        return gate_general(gk, w0 & 15, a.y, a.z, a.w, (w0 >> 4) & 15, b.y, b.z, b.w, __float_as_int(X[1]), X[2], X[3],
+                            X[4], __float_as_int(X[5]), X[6], X[7], X[8], c.x, init, dt,
+                            gk == EDEN_GATE_INSTANTANEOUS ? vnew : v, qo);
     }
-    const float alpha = rate_value(w0, P[1], P[2], P[3], v);
-    const float beta = rate_value(__float_as_int(P[4]), P[5], P[6], P[7], v);
-    return gate_relax(alpha, beta, P[8], init, dt, qo);
+    const int fk = w0 & 15, rk = (w0 >> 4) & 15;
+    const bool fq = fk != EDEN_RATE_EXP, rq = rk != EDEN_RATE_EXP;
+    const bool fs = fk == EDEN_RATE_SIGMOID, rs = rk == EDEN_RATE_SIGMOID;
+    const float xf = div_known(v - a.z, a.w, c.y), xr = div_known(v - b.z, b.w, c.z);
+    const float ef = expf(fq ? -xf : xf), er = expf(rq ? -xr : xr);
+    const float fn = fs ? a.y : xf, fd = fs ? 1.0f + ef : 1.0f - ef;
+    const float rn = rs ? b.y : xr, rd = rs ? 1.0f + er : 1.0f - er;
+    // one quotient covers a gate with one exponential form
+    const float q1 = (fq ? fn : rn) / (fq ? fd : rd);
+    const float q2 = fq && rq ? rn / rd : q1;
+    const float alpha = !fq ? a.y * ef : fs ? q1 : a.y * ((v == a.z) ? 1.0f : q1);
+    const float beta = !rq ? b.y * er : rs ? q2 : b.y * ((v == b.z) ? 1.0f : q2);
+    const float sum = alpha + beta;
+    const float tau = 1.0f / sum;
+    const float inf = div_known(alpha, sum, (sum >= 0x1p-60f && sum < 0x1p60f) ? tau : 0.0f);
+    return gate_relax_ti(tau, inf, c.x, init, dt, qo);
 }
 
 // ---------------------------------------------------------------------------
@@ -1300,118 +1389,146 @@ __device__ __forceinline__ void hines_forest_f64(const DevModel &m, bool init, i
 }
 
 // Backward-Euler Hines solve of one forest by one warp for the windowed path,
-// on the unit's shared-memory slice (eden/Eden.cpp:6114-6225), whose
-// compartment terms sit in pairs so that one load brings two: XR (V, the
-// elimination factor), KL (c_kl, the packed child range / parent / non-flat
-// flag) and UP (U, the pivot).  Flat compartments keep the reciprocal pivot
-// and the elimination factor L / pivot computed once, because their
-// diagonals never change, and their pre-update (V += c_kl) is folded into
-// the elimination; a non-flat compartment's pivot is rebuilt every step
-// from its diagonal (UP.y holds G/C + sum 1/(RC) on entry, XR.x its
-// pre-updated V) and its children's factors, in increasing child order as
-// the reference's post-order visits them, and its factor from its L
-// (KL.x).  The forest's levels (LV: each level's first compartment and
-// whether it holds a non-flat one) put every compartment below its parent;
-// the elimination runs from the last level to the roots of level 0, a
-// level's compartments over the lanes, then the back-substitution runs
-// root-first.  XR.x holds V_next on return.
-constexpr int32_t kLvMask = 0xffff;
-constexpr int32_t kLvNonFlat = 1 << 16;
-__device__ __forceinline__ void hines_window(float dt, float2 *XR, const uint2 *KL, float2 *UP, const int32_t *LV,
-                                             int nlev) {
+// on the unit's shared-memory slice S (eden/Eden.cpp:6114-6225).  Flat
+// compartments keep the reciprocal pivot and the elimination factor L / pivot
+// computed once, because their diagonals never change.  Every compartment takes
+// its children in increasing order, as the reference's post-order visits them.
+//
+// Twigs first: each lane walks its own flat subtrees up, every compartment into
+// its parent's word, the topmost into its node's; their pre-update (V + the
+// increment) was written with their V (TX; TV holds V).  Then the nodes, depth
+// by depth (XR: V and the elimination factor; CN: the record): from the last
+// pass (PS) to the roots, which it finishes, a flat node's pre-update (V +=
+// CN.x) folded in, a non-flat node's pivot rebuilt from 1 + dt (G/C + sum
+// 1/(RC)) (CN.z on entry, XR.x its pre-updated V) and its factor from its L;
+// then from pass `p1`, the first below the roots, the back-substitution; then
+// the twigs down again.
+//
+// A unit's step is a chain, and what it costs is the instructions a warp spends
+// along it.  A depth costs 26 + 16 of them and 5 more for each child of its
+// largest family, for as few compartments as there are; a twig row costs 22 for
+// up to 32.  So subtrees up to a size chosen per forest become twigs
+// (build_and_upload weighs the two), and depths remain only above them.  In a
+// pass every lane takes as many children as the pass's largest family (an absent
+// one is node n, all zeros), so the loop over them does not diverge, and lanes
+// past its end load what they do not use.  A lane's places are 32 words apart: no bank
+// conflicts, and no synchronisation within a twig.
+// (Products are fused explicitly, as the compiler fuses them in a plain loop.)
+__device__ __forceinline__ void hines_window(float dt, float *S, float2 *XR, float4 *CN, const int32_t *PS, int np,
+                                             int p1, int n, float *TX, float *TV, const float4 *TR, const uint32_t *TA,
+                                             int nw) {
     const int lane = threadIdx.x & 31;
-    int end = LV[nlev] & kLvMask;
-    for (int lev = nlev - 1; lev >= 0; lev--) {
-        const int32_t lw = LV[lev];
-        // a level wider than the warp takes two or more passes
-        for (int j = (lw & kLvMask) + lane; j < end; j += 32) {
-            const uint2 kl = KL[j];
-            const uint32_t cep = kl.y;
-            const int ke = (int)(cep & kCepMask), kb = (int)((cep >> kCepBeginShift) & kCepMask);
-            if ((lw & kLvNonFlat) && (cep & kCepNonFlat)) {
-                float xj = XR[j].x + 0.0f;
-                float dj = 1.0f + UP[j].y * dt;
-                for (int i = kb; i < ke; i++) {
-                    const float2 c = XR[i];
-                    dj -= c.y * UP[i].x;
-                    xj -= c.y * c.x;
-                }
-                const float inv = __fdividef(1.0f, dj);
-                UP[j].y = inv;
-                XR[j] = make_float2(xj, __uint_as_float(kl.x) * inv);
-            } else {
-                float xj = XR[j].x + __uint_as_float(kl.x);
-                // most compartments have at most two children: take those
-                // without a loop, in order
-                int i = kb;
-                if (i < ke) { const float2 c = XR[i]; xj -= c.y * c.x; }
-                if (i + 1 < ke) { const float2 c = XR[i + 1]; xj -= c.y * c.x; }
-                for (i = kb + 2; i < ke; i++) { const float2 c = XR[i]; xj -= c.y * c.x; }
-                XR[j].x = xj;
+#pragma unroll 1
+    for (int i = lane; i < 32 * nw; i += 32) {
+        const uint32_t a = TA[i];
+        const float x = TX[i];
+        float *to = S + (a & (kTwigTop - 1));
+        const float y = fmaf(-TR[i].w, x, *to);
+        *to = (a & kTwigTop) ? x : y;
+    }
+    if (nw > 0) __syncwarp();
+#pragma unroll 1
+    for (int p = np - 1; p >= 0; p--) {
+        const int32_t d = PS[p];
+        const int j = (d & kPassStart) + lane, kids = (d >> kPassKidsShift) & 0x3ff;
+        const bool on = lane < ((d >> kPassCountShift) & 63);
+        const float4 c = CN[j];
+        float x = XR[j].x;
+        const uint32_t cep = __float_as_uint(c.w);
+        int kb = (int)((cep >> kCepBeginShift) & kCepMask);
+        const int ke = on ? kb + (int)(cep & kCepMask) : 0;
+        // (a twig's topmost compartment among them has done its part)
+        if (d & kPassNonFlat) {
+            const bool nonflat = (cep & kCepNonFlat) != 0;
+            float dj = c.z;
+            x += (cep & (kCepNonFlat | kCepTwig)) ? 0.0f : c.x;
+#pragma unroll 1
+            for (int i = 0; i < kids; i++, kb++) {
+                const int q = kb < ke ? kb : n;
+                const float2 k = XR[q];
+                dj = fmaf(-k.y, CN[q].y, dj);
+                x = fmaf(-k.y, k.x, x);
+            }
+            const float inv = nonflat ? __fdividef(1.0f, dj) : c.z;
+            if (d & kPassRoot) x = x * inv;
+            if (on && nonflat) { CN[j].z = inv; XR[j].y = c.x * inv; }
+        } else {
+            x += (cep & kCepTwig) ? 0.0f : c.x;
+#pragma unroll 1
+            for (int i = 0; i < kids; i += 2, kb += 2) {
+                const float2 k = XR[kb < ke ? kb : n], l = XR[kb + 1 < ke ? kb + 1 : n];
+                x = fmaf(-k.y, k.x, x);
+                x = fmaf(-l.y, l.x, x);
             }
         }
-        end = lw & kLvMask;
-        __syncwarp();
+        if (on) XR[j].x = x;
+        if (d & kPassFirst) __syncwarp();
     }
-    for (int r = (LV[0] & kLvMask) + lane; r < (LV[1] & kLvMask); r += 32) XR[r].x = XR[r].x * UP[r].y;
-    __syncwarp();
-    for (int lev = 1; lev < nlev; lev++) {
-        const int i1 = LV[lev + 1] & kLvMask;
-        for (int i = (LV[lev] & kLvMask) + lane; i < i1; i += 32) {
-            const int p = (int)((KL[i].y >> kCepParentShift) & kCepMask) - 1;
-            const float2 up = UP[i];
-            XR[i].x = (XR[i].x - up.x * XR[p].x) * up.y;
-        }
-        __syncwarp();
+#pragma unroll 1
+    for (int p = p1; p < np; p++) {
+        const int32_t d = PS[p];
+        const int j = (d & kPassStart) + lane;
+        const bool on = lane < ((d >> kPassCountShift) & 63);
+        const float4 c = CN[j];
+        const float x = XR[j].x;
+        const int q = on ? (int)((__float_as_uint(c.w) >> kCepParentShift) & kCepMask) : 0;
+        const float v = fmaf(-c.y, XR[q].x, x) * c.z;
+        if (on) XR[j].x = v;
+        if (d & kPassLast) __syncwarp();
+    }
+#pragma unroll 1
+    for (int i = 32 * (nw - 1) + lane; i >= 0; i -= 32) {
+        const float4 c = TR[i];
+        const float v = fmaf(-c.y, S[TA[i] >> 16], TX[i]) * c.z;
+        TV[i] = v;
+        TX[i] = __fadd_rn(v, c.x);
     }
 }
 
 // hines_window in double precision, for a forest whose rows may lose
 // diagonal dominance: every compartment's pivot is rebuilt each step from
-// its diagonal term (UP.y: G/C + sum 1/(RC), the flat ones' constant one staged
-// from c_d0), and the elimination and back-substitution carry doubles in
+// its diagonal term (CN.z: G/C + sum 1/(RC), constant for the flat ones), and
+// the elimination and back-substitution carry doubles in
 // XD / PVD / RTD; XR.x receives V_next rounded once.  A flat compartment's
-// pre-update is its c_kl, and every compartment's L comes from Lg (global,
+// pre-update is its CN.x, and every compartment's L comes from Lg (global,
 // indexed like the forest).  The operations are hines_window's, in its order.
-__device__ __forceinline__ void hines_window_f64(float dt, float2 *XR, const uint2 *KL, const float2 *UP,
-                                                 const float *Lg, const int32_t *LV, int nlev, double *XD,
-                                                 double *PVD, double *RTD) {
+__device__ __forceinline__ void hines_window_f64(float dt, float2 *XR, const float4 *CN, const float *Lg,
+                                                 const int32_t *PS, int np, int n, double *XD, double *PVD,
+                                                 double *RTD) {
     const int lane = threadIdx.x & 31;
     const double dtd = dt;
-    int end = LV[nlev] & kLvMask;
-    for (int lev = nlev - 1; lev >= 0; lev--) {
-        const int32_t lw = LV[lev];
-        for (int j = (lw & kLvMask) + lane; j < end; j += 32) {
-            const uint2 kl = KL[j];
-            const uint32_t cep = kl.y;
-            const int ke = (int)(cep & kCepMask), kb = (int)((cep >> kCepBeginShift) & kCepMask);
-            const float kc = (cep & kCepNonFlat) ? 0.0f : __uint_as_float(kl.x);
+    for (int p = np - 1; p >= 0; p--) {
+        const int32_t d = PS[p];
+        const int j = (d & kPassStart) + lane;
+        if (lane < ((d >> kPassCountShift) & 63)) {
+            const float4 c = CN[j];
+            const uint32_t cep = __float_as_uint(c.w);
+            const int kb = (int)((cep >> kCepBeginShift) & kCepMask), ke = kb + (int)(cep & kCepMask);
+            const float kc = (cep & kCepNonFlat) ? 0.0f : c.x;
             double xj = (double)XR[j].x + (double)kc;
-            double dj = 1.0 + (double)UP[j].y * dtd;
+            double dj = 1.0 + (double)c.z * dtd;
             for (int i = kb; i < ke; i++) {
                 const double r = RTD[i];
-                dj -= r * (double)UP[i].x;
+                dj -= r * (double)CN[i].y;
                 xj -= r * XD[i];
             }
             const double inv = 1.0 / dj;
             PVD[j] = inv;
             RTD[j] = (double)Lg[j] * inv;
-            XD[j] = xj;
+            XD[j] = (d & kPassRoot) ? xj * inv : xj;
         }
-        end = lw & kLvMask;
-        __syncwarp();
+        if (d & kPassFirst) __syncwarp();
     }
-    for (int r = (LV[0] & kLvMask) + lane; r < (LV[1] & kLvMask); r += 32) XD[r] = XD[r] * PVD[r];
-    __syncwarp();
-    for (int lev = 1; lev < nlev; lev++) {
-        const int i1 = LV[lev + 1] & kLvMask;
-        for (int i = (LV[lev] & kLvMask) + lane; i < i1; i += 32) {
-            const int p = (int)((KL[i].y >> kCepParentShift) & kCepMask) - 1;
-            XD[i] = (XD[i] - (double)UP[i].x * XD[p]) * PVD[i];
+    for (int p = 0; p < np; p++) {
+        const int32_t d = PS[p];
+        const int i = (d & kPassStart) + lane;
+        if (!(d & kPassRoot) && lane < ((d >> kPassCountShift) & 63)) {
+            const float4 c = CN[i];
+            const int q = (int)((__float_as_uint(c.w) >> kCepParentShift) & kCepMask);
+            XD[i] = (XD[i] - (double)c.y * XD[q]) * PVD[i];
         }
-        __syncwarp();
+        if (d & kPassLast) __syncwarp();
     }
-    const int n = LV[nlev] & kLvMask;
     for (int i = lane; i < n; i += 32) XR[i].x = (float)XD[i];
     __syncwarp();
 }

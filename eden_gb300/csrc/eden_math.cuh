@@ -35,6 +35,26 @@ __device__ __forceinline__ float randof(float x, int64_t work_item, int64_t inst
     return x * r;
 }
 
+// x / y, correctly rounded, where r = RN(1 / y) is known in advance (or 0, if
+// |y| is outside [2^-60, 2^60)): Markstein's theorem, as div_by_tau uses it --
+// q = RN(x r) is within an ulp of the quotient, x - y q is exact in one FMA, and
+// RN(q + r (x - y q)) is the correctly rounded quotient.  With |x| and |y| in
+// [2^-60, 2^60) every intermediate is normal; any other operand (zero,
+// infinite and NaN ones among them) is divided.  Four dependent operations and
+// no reciprocal, where a division is about ten with a slow path to branch to.
+static __device__ __noinline__ float div_any(float x, float y) { return x / y; }
+__device__ __forceinline__ float div_known(float x, float y, float r) {
+    const float a = fabsf(x);
+    if (!(a >= 0x1p-60f && a < 0x1p60f) || r == 0.0f) return div_any(x, y);
+    const float q = x * r;
+    return fmaf(fmaf(-q, y, x), r, q);
+}
+// RN(1 / y) for div_known, 0 where it has to divide
+__host__ __device__ __forceinline__ float known_reciprocal(float y) {
+    const float a = y < 0.0f ? -y : y;
+    return a >= 0x1p-60f && a < 0x1p60f ? 1.0f / y : 0.0f;
+}
+
 // HH rate forms (eden/Eden.cpp:5164-5181), evaluated without branching on
 // the form so that the gates of a warp with different forms do not diverge;
 // each form keeps its own operations: EXP r * exp(x), EXPLINEAR

@@ -10,7 +10,7 @@ namespace eden {
 
 constexpr int kThreads = 256;
 constexpr int kInputThreads = 128;  // k_inputs_t: four warps, each with two event tiles
-constexpr int kCellThreads = 128;   // k_cells_t: four warps
+constexpr int kCellThreads = 768;   // k_cells_t: at most, a warp per unit; the registers of 24 warps an SM
 constexpr int kHinesThreads = 128;  // k_hines_t: four warps, each staging one forest
 
 }  // namespace eden
@@ -166,180 +166,222 @@ __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs 
 // staged in the warp's shared-memory slice for the whole window.
 
 // A forest unit over the window.  At the window start the unit stages its
-// compartments, its non-flat compartments' descriptors, its gates with their
-// parameter records, and the conductance series of its input chunks for all
-// K steps (written by k_inputs_t), so that a step reads shared memory only.
-// Per step: trajectory samples of the step's starting V; the non-flat
-// compartments' currents (inputs, channels with the gate values before this
-// step's update), diagonal and pre-update; the cable solve, which also
-// applies the flat compartments' constant pre-update; gate updates from the
-// starting V; threshold crossings.
+// nodes', twigs' and non-flat compartments' records, its gates, its input
+// blocks, and the conductance series of its input chunks for all K steps
+// (written by k_inputs_t), so that a step reads shared memory only.  Per step: trajectory samples of the step's starting V; the
+// non-flat compartments' currents (inputs, channels with the gate values before
+// this step's update), diagonal and pre-update; gate updates from the starting
+// V, into the other of the gates' two buffers; the cable solve; threshold
+// crossings.  A lane with at most one non-flat compartment, or one gate, keeps
+// its record in registers for the whole window.
+//
+// With the unit in shared memory the kernel moves 15 times less than a step
+// over HBM would, and is bound by the length of a step's dependent chain and,
+// with many units, by the instructions issued: hence few instructions a pass,
+// divisions by constants done as div_known, and units sized in edenGpuCreate.
 __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S) {
     const int lane = threadIdx.x & 31;
-    const int t0 = m.un_t0[u], n = m.un_t1[u] - t0, fi = m.un_f[u];
+    const int t0 = m.un_t0[u], fi = m.un_f[u], ub0 = m.t_blk0[t0], nblk = m.t_blk0[m.un_t1[u]] - ub0;
+    const int n0 = m.fo_n0[fi], n = m.fo_n0[fi + 1] - n0, w0 = m.fo_w0[fi], nw = m.fo_w0[fi + 1] - w0;
     const int ngt = m.un_ngt[u], gt0 = m.un_gt0[u];
-    const int s0 = m.un_s0[u], ns = m.un_s1[u] - s0;
     const int r0 = m.un_r0[u], r1 = m.un_r1[u];
     const int nf0 = m.un_nf0[u], nf = m.un_nf1[u] - nf0;
-    const int nlev = m.fo_nlev[fi], l0 = m.fo_l0[fi];
-    const int ub0 = m.t_blk0[t0], nblk = m.t_blk0[t0 + n] - ub0;
+    const int ps0 = m.fo_p0[fi], np = m.fo_p0[fi + 1] - ps0;
     const int uc0 = m.bk_c0[ub0], nck = m.bk_c0[ub0 + nblk] - uc0;
-    // compartment terms in pairs (the slice is 8-byte aligned): V and the
-    // elimination factor, c_kl and the packed child range / parent / flag, U
-    // and the pivot
+    const int uch0 = m.un_ch0[u], nch = m.un_ch1[u] - uch0;
     float2 *XR = reinterpret_cast<float2 *>(S);
-    uint2 *KL = reinterpret_cast<uint2 *>(S + 2 * n);
-    float2 *UP = reinterpret_cast<float2 *>(S + 4 * n);
-    int32_t *NT = (int32_t *)(S + 6 * n);
-    float *VO = (float *)(NT + nf), *NA = VO + nf, *NC = NA + nf, *NIR = NC + nf;
-    int32_t *NB0 = (int32_t *)(NIR + nf), *NB1 = NB0 + nf, *NCH0 = NB1 + nf, *NCH1 = NCH0 + nf;
-    int32_t *NSIG = NCH1 + nf;
-    const int uch0 = nf > 0 ? m.nf_c0[nf0] : 0, nch = nf > 0 ? m.nf_c1[nf0 + nf - 1] - uch0 : 0;
-    float *CHG = (float *)(NSIG + nf), *CHE = CHG + nch;
+    float *TX = S + twig_words(n + 1), *TV = TX + 32 * nw;
+    float4 *CN = reinterpret_cast<float4 *>(TV + 32 * nw), *TR = CN + n + 1;
+    float4 *NF = TR + 32 * nw;
+    int4 *BK = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
+    float2 *TS = reinterpret_cast<float2 *>(BK + nblk);
+    uint32_t *TA = reinterpret_cast<uint32_t *>(TS + nf);
+    float *VO = (float *)(TA + 32 * nw);
+    float *CHG = VO + nf, *CHE = CHG + nch;
     int32_t *CHQ = (int32_t *)(CHE + nch), *CHI = CHQ + nch;
-    float *GT = (float *)(CHI + nch);
-    int32_t *GI_S = (int32_t *)(GT + ngt);
-    float *GP = (float *)(GI_S + ngt);
-    int32_t *LV = (int32_t *)(GP + kGateWords * ngt);
-    int32_t *ST = LV + nlev + 1, *SSRC = ST + ns;
-    float *STHR = (float *)(SSRC + ns);
-    int32_t *BKK = (int32_t *)(STHR + ns);
-    float *BKE = (float *)(BKK + nblk);
-    int32_t *BKC = (int32_t *)(BKE + nblk);
-    float *GS = (float *)(BKC + nblk + 1);
+    int32_t *GI = CHI + nch;
+    float *GT = (float *)(GI + ngt);  // two buffers of ngt
+    int32_t *PS = (int32_t *)(GT + 2 * ngt);
+    float *GS = (float *)(PS + np);
     // a double-precision forest's eliminated values, pivots and factors
     const bool f64 = m.fo_f64[fi] != 0;
     double *XD = reinterpret_cast<double *>((reinterpret_cast<unsigned long long>(GS + w.K * nck) + 7ull) & ~7ull);
     double *PVD = XD + n, *RTD = PVD + n;
+    // the steps of a window are all initialisation passes or none is
+    const bool init = w.step0 <= 0;
     // ---- stage the unit
     const float *vsrc = m.v[w.par];
-    const float *pv0 = f64 ? m.c_d0 : m.c_pv0;
     for (int i = lane; i < n; i += 32) {
-        const int t = t0 + i;
-        stage_word(&XR[i].x, &vsrc[t]); stage_word(&XR[i].y, &m.c_rt0[t]);
-        stage_word(&KL[i].x, &m.c_kl[t]); stage_word(&KL[i].y, &m.c_cep[t]);
-        stage_word(&UP[i].x, &m.c_u[t]); stage_word(&UP[i].y, &pv0[t]);
+        const int t = m.nd_t[n0 + i];
+        stage_rec(&CN[i], &m.c_rec[n0 + i]);
+        stage_word(&XR[i].x, &vsrc[t0 + (t >= 0 ? t : -1 - t)]); stage_word(&XR[i].y, &m.nd_rt[n0 + i]);
     }
+    if (lane == 0) {
+        XR[n] = make_float2(0.0f, 0.0f);
+        CN[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    for (int i = lane; i < 32 * nw; i += 32) {
+        const int t = m.tw_t[32 * w0 + i];
+        stage_rec(&TR[i], &m.tw_rec[32 * w0 + i]);
+        stage_word(&TA[i], &m.tw_adr[32 * w0 + i]);
+        stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
+    }
+    for (int i = lane; i < kSlotRecs * nf; i += 32) stage_rec(&NF[i], &m.nf_rec[(size_t)kSlotRecs * nf0 + i]);
+    for (int i = lane; i < nblk; i += 32) stage_rec(&BK[i], &m.bk_rec[ub0 + i]);
     for (int j = lane; j < nf; j += 32) {
-        const int ti = m.nf_t[nf0 + j], t = t0 + ti;
-        NT[j] = ti;
-        stage_word(&NA[j], &m.c_area[t]); stage_word(&NC[j], &m.c_cm[t]); stage_word(&NIR[j], &m.c_inv_rc[t]);
-        NB0[j] = m.t_blk0[t] - ub0; NB1[j] = m.t_blk0[t + 1] - ub0;
-        const int ch0 = m.c_chan0[t], ch1 = m.c_chan0[t + 1];
-        NCH0[j] = m.nf_c0[nf0 + j] - uch0; NCH1[j] = m.nf_c1[nf0 + j] - uch0;
-        stage_word(&NSIG[j], &m.nf_sig[nf0 + j]);
-        // gate update items: the non-flat slot and the gate's parameter record
-        for (int ch = ch0; ch < ch1; ch++) {
-            const int q0 = m.ch_gate0[ch] - gt0, q1 = m.ch_gate0[ch + 1] - gt0;
-            const float *src = m.gate_par + (size_t)m.ch_type[ch] * EDEN_MAX_GATES * kGateWords;
-            for (int q = q0; q < q1; q++) {
-                GI_S[q] = j;
-                for (int k = 0; k < kGateWords; k++) stage_word(&GP[q * kGateWords + k], &src[(q - q0) * kGateWords + k]);
-            }
-        }
+        stage_word(&TS[j].x, &m.nf_ts[nf0 + j].x); stage_word(&TS[j].y, &m.nf_ts[nf0 + j].y);
     }
     for (int c = lane; c < nch; c += 32) {
         stage_word(&CHG[c], &m.nfc_g[uch0 + c]); stage_word(&CHE[c], &m.nfc_e[uch0 + c]);
         stage_word(&CHQ[c], &m.nfc_q[uch0 + c]); stage_word(&CHI[c], &m.nfc_i[uch0 + c]);
     }
-    for (int i = lane; i < ngt; i += 32) stage_word(&GT[i], &m.gate[gt0 + i]);
-    for (int i = lane; i <= nlev; i += 32) {
-        const int info = m.lvl_info[l0 + i];
-        LV[i] = (m.lvl[l0 + i] - t0) | ((info & 0x80) ? kLvNonFlat : 0);
-    }
-    for (int i = lane; i < ns; i += 32) {
-        stage_word(&ST[i], &m.gs_t[s0 + i]); stage_word(&SSRC[i], &m.gs_src[s0 + i]); stage_word(&STHR[i], &m.gs_thr[s0 + i]);
-    }
-    for (int b = lane; b <= nblk; b += 32) {
-        BKC[b] = m.bk_c0[ub0 + b] - uc0;
-        if (b < nblk) { stage_word(&BKK[b], &m.bk_kind[ub0 + b]); stage_word(&BKE[b], &m.bk_erev[ub0 + b]); }
-    }
+    for (int i = lane; i < ngt; i += 32) { stage_word(&GT[i], &m.gate[gt0 + i]); stage_word(&GI[i], &m.gt_idx[gt0 + i]); }
+    for (int i = lane; i < np; i += 32) stage_word(&PS[i], &m.ps[ps0 + i]);
     for (int k = 0; k < w.K; k++)
         for (int c = lane; c < nck; c += 32) stage_word(&GS[k * nck + c], &m.Gp[(size_t)k * m.n_chunk + uc0 + c]);
     stage_wait();
     __syncwarp();
+    for (int j = lane; j < nf; j += 32) VO[j] = XR[__float_as_int(NF[kSlotRecs * j].x) & kPassStart].x;
+    for (int i = lane; i < 32 * nw; i += 32) TX[i] = TV[i] + TR[i].x;  // the first step's pre-update
+    int p1 = 0;  // the first pass below the roots
+    while (p1 < np && (PS[p1] & kPassRoot)) p1++;
+    __syncwarp();
     const float dt = m.dt;
-    double tstep = w.t0;  // this step's time, accumulated in double as the host does
+    int row = 0;  // the first step's row of the trajectory buffer
+    if (r1 > r0) row = (int)((w.step0 + m.trace_cap - 1) % m.trace_cap);
+    float *Gq = GT, *Gn = GT + ngt;  // gate values at the step's start, and at the next's
+    float4 sa, sb, ga, gb, gc;       // the lane's only slot and gate, where it has no more
+    float2 ts;
+    int gs = 0;
+#pragma unroll 1
     for (int k = 0; k < w.K; k++) {
-        const int64_t step = w.step0 + k;
-        const bool init = step <= 0;
-        if (!init && r1 > r0) {
+        if (r1 > r0) {
             // trajectory samples of this step's starting state
-            const int64_t row = (step - 1) % m.trace_cap;
-            for (int q = r0 + lane; q < r1; q += 32) {
-                const int32_t tq = m.gr_t[q];  // a compartment, or -1 - a gate slot
-                m.trace_buf[row * m.n_trace + m.gr_col[q]] = tq >= 0 ? XR[tq].x : GT[-1 - tq];
+            if (!init) {
+#pragma unroll 1
+                for (int q = r0 + lane; q < r1; q += 32) {
+                    const int32_t tq = m.gr_t[q];
+                    m.trace_buf[(size_t)row * m.n_trace + m.gr_col[q]] =
+                        tq < 0 ? Gq[-1 - tq] : (tq & 1) ? TV[tq >> 1] : XR[tq >> 1].x;
+                }
+                row = row + 1 == (int)m.trace_cap ? 0 : row + 1;
             }
+            __syncwarp();
         }
-        __syncwarp();
         const float *Gk = GS + k * nck;
+#pragma unroll 1
         for (int j = lane; j < nf; j += 32) {
             // channels + voltage pre-update (eden/Eden.cpp:5013-6107)
-            const int ti = NT[j];
-            const float v = XR[ti].x;
-            VO[j] = v;
+            if (k == 0 || nf > 32) { sa = NF[kSlotRecs * j]; sb = NF[kSlotRecs * j + 1]; }
+            const int slot = __float_as_int(sa.x), ti = slot & kPassStart;
+            const int brange = __float_as_int(sb.y), crange = __float_as_int(sb.z);
+            const int ch0 = crange & 0xffff;
+            const float v = VO[j];
             float Iin, Gin, Isyn, Gsyn;
-            block_currents(Gk, NB0[j], NB1[j], BKK, BKE, BKC, 0, v, Iin, Gin, Isyn, Gsyn);
+            block_currents_rec(Gk, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
             // (a model with gap junctions runs one-step windows: vsrc holds
             // every target's potential at this step's start)
-            if (EDEN_KIND_GAP) Isyn += gap_current(m, t0 + ti, v, vsrc, init);
-            const float A = NA[j];
+            if (EDEN_KIND_GAP) Isyn += gap_current(m, t0 + m.nd_t[n0 + ti], v, vsrc, init);
+            const float A = sa.y;
             float Ich = 0.f, Gch = 0.f;
 #ifdef EDEN_RTC_CHANNELS
             // the routine generated for this compartment's channel set
-            if (!rtc_channels(NSIG[j], GT + CHQ[NCH0[j]], CHG, CHE, NCH0[j], v, A, Ich, Gch))
+            if (!rtc_channels(__float_as_int(sb.w), Gq + CHQ[ch0], CHG, CHE, ch0, v, A, Ich, Gch))
 #endif
-            for (int c = NCH0[j]; c < NCH1[j]; c++) {
+#pragma unroll 1
+            for (int c = ch0; c < ch0 + (int)((uint32_t)crange >> 16); c++) {
                 const int gi_pack = CHI[c];
-                const float *q = GT + CHQ[c];
+                const float *q = Gq + CHQ[c];
                 float fopen = 1.0f;
                 for (int gi = 0; gi < (gi_pack & 7); gi++) {
                     const float qo = q[gi];
                     const int inst = (gi_pack >> (3 + 5 * gi)) & 31;
                     for (int rr = 0; rr < inst; rr++) fopen = fopen * qo;
                 }
-                const float gs = CHG[c] * fopen;
-                Ich += (gs * (CHE[c] - v) * 1e-5f) * A;
-                Gch += (gs * 1e-5f) * A;
+                const float g = CHG[c] * fopen;
+                Ich += (g * (CHE[c] - v) * 1e-5f) * A;
+                Gch += (g * 1e-5f) * A;
             }
             const float I = Ich + Iin + Isyn;
             const float G = Gch + Gin + Gsyn;
-            const float C = NC[j];
-            UP[ti].y = 1.0f * (G / C) + NIR[j];
-            XR[ti].x = init ? v : v + (dt * (I + (v * G))) / C;
+            const float C = sa.z, rC = sa.w;
+            float d = 1.0f * div_known(G, C, rC) + sb.x;
+            float x = init ? v : v + div_known(dt * (I + (v * G)), C, rC);
+            if (!f64) {
+                d = 1.0f + d * dt;
+                if ((slot & kSlotDone) && !init) x = x * __fdividef(1.0f, d);
+            }
+            CN[ti].z = d;
+            XR[ti].x = x;
         }
+        // gate updates from this step's starting V and gate values; an
+        // instantaneous gate takes the potential after the step, so a model
+        // with other kinds of gates updates them after the solve
+        auto update_gates = [&]() {
+#pragma unroll 1
+            for (int q = lane; q < ngt; q += 32) {
+                if (k == 0 || ngt > 32) {
+                    gs = GI[q];
+                    const float4 *r = m.gate_tab + kGateRecs * (gs >> 10);
+                    ga = r[0]; gb = r[1]; gc = r[2];
+                    gs &= kPassStart;
+                }
+                Gn[q] = gate_next_p(ga, gb, gc, m.gate_ext, init, dt, VO[gs],
+                                    EDEN_KIND_GATEFORMS ? XR[__float_as_int(NF[kSlotRecs * gs].x) & kPassStart].x : 0.0f,
+                                    Gq[q]);
+            }
+        };
+        if (!EDEN_KIND_GATEFORMS) update_gates();
         __syncwarp();
         if (!init) {
-            if (f64) hines_window_f64(dt, XR, KL, UP, m.c_l + t0, LV, nlev, XD, PVD, RTD);
-            else hines_window(dt, XR, KL, UP, LV, nlev);
+            // (a double-precision forest has no twigs: its nodes are its compartments)
+            if (f64) hines_window_f64(dt, XR, CN, m.c_l + t0, PS, np, n, XD, PVD, RTD);
+            else hines_window(dt, S, XR, CN, PS, np, p1, n, TX, TV, TR, TA, nw);
         }
-        // gate updates from this step's starting V and gate values (the
-        // currents above used the values before the update, as the reference does)
-        for (int q = lane; q < ngt; q += 32)
-            GT[q] = gate_next_p(GP + q * kGateWords, m.gate_ext, init, dt, VO[GI_S[q]],
-                                EDEN_KIND_GATEFORMS ? XR[NT[GI_S[q]]].x : 0.0f, GT[q]);
-        // threshold crossings of the unit's spike sources (eden/Eden.cpp:6247-6252)
-        for (int q0 = 0; q0 < ns; q0 += 32) {
-            const int q = q0 + lane;
+        if (EDEN_KIND_GATEFORMS) {
+            update_gates();
+            __syncwarp();
+        }
+        // threshold crossings of the unit's spike sources (eden/Eden.cpp:6247-6252),
+        // and V for the next step
+#pragma unroll 1
+        for (int j0 = 0; j0 < nf; j0 += 32) {
+            const int j = j0 + lane;
             bool spk = false;
-            int src = -1;
-            double tc = 0.0;
-            if (q < ns) {
-                const int sl = ST[q];
-                src = SSRC[q];
-                const float vo = VO[sl], vn = XR[NT[sl]].x;
-                spk = vo < STHR[q] && STHR[q] < vn;
-                if (spk) tc = crossing_time(tstep, dt, vo, vn, STHR[q]);
+            float vo = 0.0f, vn = 0.0f;
+            if (j < nf) {
+                if (nf > 32) sa.x = NF[kSlotRecs * j].x;
+                if (k == 0 || nf > 32) ts = TS[j];
+                vo = VO[j];
+                vn = XR[__float_as_int(sa.x) & kPassStart].x;
+                spk = vo < ts.x && ts.x < vn;
+                VO[j] = vn;
             }
-            push_spike(m, spk, src, (int32_t)(step + 1), w.wpar, tc);
+            if (__any_sync(0xffffffffu, spk)) {
+                // (this step's time, accumulated in double as the host does)
+                double t = w.t0;
+                if (!init)
+                    for (int i = 0; i < k; i++) t += (double)dt;
+                push_spike(m, spk, spk ? __float_as_int(ts.y) : -1, (int32_t)(w.step0 + k + 1), w.wpar,
+                           spk ? crossing_time(t, dt, vo, vn, ts.x) : 0.0);
+            }
         }
         __syncwarp();
-        if (!init) tstep += (double)dt;
+        float *g = Gq;
+        Gq = Gn;
+        Gn = g;
     }
     // ---- write the unit back into the buffer that holds the window's final state
     float *vdst = m.v[w.par ^ (w.K & 1)];
-    for (int i = lane; i < n; i += 32) vdst[t0 + i] = XR[i].x;
-    for (int i = lane; i < ngt; i += 32) m.gate[gt0 + i] = GT[i];
+    for (int i = lane; i < n; i += 32) {
+        const int t = m.nd_t[n0 + i];
+        if (t >= 0) vdst[t0 + t] = XR[i].x;
+    }
+    for (int i = lane; i < 32 * nw; i += 32) {
+        const int t = m.tw_t[32 * w0 + i];
+        if (t >= 0) vdst[t0 + t] = TV[i];
+    }
+    for (int i = lane; i < ngt; i += 32) m.gate[gt0 + i] = Gq[i];
 }
 
 // A batch of up to 32 point neurons over the window (izhikevich2007Cell,
@@ -406,7 +448,7 @@ __device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &
 // A block runs several CTAs in turn when there are more CTAs than blocks;
 // their units are laid out differently in shared memory, so every warp of
 // the block finishes its unit before any starts on the next CTA.
-__global__ void __launch_bounds__(kCellThreads, 8) k_cells_t(DevModel m, const WindowArgs *tab, const WindowTimes *ttab,
+__global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(DevModel m, const WindowArgs *tab, const WindowTimes *ttab,
                                                           const int *base, int idx, int cta_begin, int cta_end) {
     extern __shared__ __align__(16) float sm[];
     const WindowArgs w = tab[*base + idx];
