@@ -38,14 +38,20 @@
 // synapse's current and conductance by its weight), summed per synapse in
 // double by k_grad_weights.
 //
-// Cells are independent, so one warp carries one cell through the whole run
-// in one launch, synchronising only within the warp.  The forward kernel
-// writes the trace and a checkpoint of (V, q) every S steps; the backward
-// kernel walks the segments last to first, recomputes each from its
-// checkpoint into a trajectory buffer and runs the adjoint steps back
-// through it.  Parameter contributions accumulate per lane in double, in a
-// fixed order, and are summed per cell and then per parameter in a fixed
-// order, so gradients are deterministic.
+// Cells are independent, and a run of one is a chain of steps, so what a step
+// must do one thing after another decides its time.  The forward kernel gives a
+// cell a block: a few warps compute the currents and one of them solves the
+// cable, while the others update the gates, which the next step is the first to
+// need.  It writes the trace, a checkpoint of (V, q) every S steps and, where
+// they fit the trajectory buffer, every step's V, q and pivots; where they do
+// not, the backward recomputes as many segments as fit at a time from their
+// checkpoints, all at once.  Of the adjoint, only the recurrence
+//   mu = M^-T lV,  lV' = mu + sum lq cv,  lq' = lq b + mu kq
+// goes back step by step; its coefficients (the factors of M^T from the
+// forward's pivots, b, cv = dQ/dV, kq = dt (E - V^{n+1}) / C gbase 1e-5 A
+// dfopen/dq) come from a kernel parallel over all steps, and the parameters'
+// terms, sums over steps of mu times known factors, from another.  They
+// accumulate in double in a fixed order, so gradients are deterministic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -105,58 +111,83 @@ struct GradDev {
     const GradSyn *syn;
     float *it_a, *it_b;      // unit-weight synapse state while tabulating
     int64_t *it_cur;         // its next event
+    float *ex;               // [ex_rows][n_item] unit-weight exposures of some steps
     float *gtab;             // [N + 1][n_grp] group conductance at step n (weights applied)
     float *gbar;             // [N + 1][n_grp] its adjoint
     double *item_grad;       // [n_item] d loss / d weight
     const float *params;
     float *ck_v, *ck_q;  // checkpoints [n_ck][n_comp], [n_ck][n_gate]
-    float *tr_v, *tr_q;  // one segment's trajectory [S + 1][n_comp], [S + 1][n_gate]
+    // trajectory of the steps from tr_n0 on: V and q at their starts (and after
+    // the last), and the reciprocal pivots of their solves
+    float *tr_v, *tr_q, *tr_d;
+    int64_t tr_n0 = 1;
+    // adjoint coefficients of the steps from co_n0 on: a row of co_len floats a
+    // step, a cell's [factor up, factor down, reciprocal pivot][nc], [b, cv, kq][ng]
+    // from cell_k0; mu, the solved adjoints of the same steps; the adjoints of
+    // the state between launches
+    const int32_t *cell_k0, *comp_cell, *gate_map, *comp_g0, *comp_rc0;
+    int32_t co_len = 0;
+    float *co, *mu;
+    int64_t co_n0 = 1;
+    float *lv, *lq;
+    double *part;        // [slots][chunks of kSumSteps steps]
+    int32_t n_part = 0;
     float *trace;        // [N][n_rec]
     const float *trace_grad;
     double *slot_grad;   // per cell and slot
 };
+
+constexpr int kSumSteps = 32;  // steps whose parameter terms one block sums
+constexpr int kRing = 4;       // steps of coefficients in flight
+constexpr int kFwdWarps = 16;  // most warps of a forward block
+constexpr int kBlock = 4;      // nodes of a chain loaded at a time, and the padding of its arrays
 
 // Largest cell, for the shared-memory layout.
 struct Dims {
     int slots, c, g, ch;
 };
 
-// One warp's shared memory: parameter accumulators, the channel types, the
-// cell's state and solve arrays, and its constants staged once per launch
-// (axial terms already scaled by the cell's resistivity parameter).
+// A block's shared memory in the forward kernel: the channel types, the cell's
+// state and solve arrays, and its constants staged once per launch (axial
+// terms already scaled by the cell's resistivity parameter).
 struct Cell {
-    double *acc;  // [slots][32]
+    // the solve's pairs, kBlock before and after the cell's: pre-updated V and
+    // 1 + dt d, by the solve the eliminated V and the reciprocal pivot; U and L
+    float2 *XD, *UL;
     EdenGpuChannelType *types;
-    float *V, *VN, *X, *D, *LV, *q, *LQ;
-    float *Us, *Ls, *Cc, *Ac, *IRCs;
+    float *Va, *Vb, *qa, *qb;  // V (kBlock after) and q: two buffers each, by turns
+    float *Cc, *Ac, *IRCs;
     int32_t *P, *CB, *CE, *ch0;
-    int32_t *ctype, *cg0, *cslot;
+    int32_t *ctype, *cg0;
+    int32_t *gmap;  // per gate: compartment | (channel type << 2 | gate of it) << 16
     float *cgb, *cerev;
-    int c0, g0, nc, ng, nch, nlev, ra_slot;
+    int c0, g0, nc, ng, nch, nlev;
     const int32_t *lev;
     bool serial;  // solve by one lane (cells with few compartments per depth)
     bool chain;   // an unbranched cable: node j's only child is j + 1
 };
 
+// A cell's axial scale Ra_ref / Ra.
+__device__ __forceinline__ float axial_scale(const GradDev &m, int cell) {
+    const int rp = m.cell_ra_param[cell];
+    return rp >= 0 ? m.cell_ra[cell] / m.params[rp] : 1.0f;
+}
+
 __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dims &dm) {
-    extern __shared__ double smem_d[];
-    const int lane = threadIdx.x & 31;
+    extern __shared__ __align__(16) double smem_d[];
+    const int tid = threadIdx.x, nt = blockDim.x;
     Cell c;
-    c.acc = smem_d;
-    c.types = reinterpret_cast<EdenGpuChannelType *>(smem_d + (size_t)dm.slots * 32);
+    c.XD = reinterpret_cast<float2 *>(smem_d) + kBlock;
+    c.UL = c.XD + dm.c + 2 * kBlock;
+    c.types = reinterpret_cast<EdenGpuChannelType *>(c.UL + dm.c + kBlock);
     float *f = reinterpret_cast<float *>(c.types + m.n_types);
-    c.V = f; f += dm.c;
-    c.VN = f; f += dm.c;
-    c.X = f; f += dm.c;
-    c.D = f; f += dm.c;
-    c.LV = f; f += dm.c;
-    c.Us = f; f += dm.c;
-    c.Ls = f; f += dm.c;
+    c.Va = f; f += dm.c + kBlock;
+    c.Vb = f; f += dm.c + kBlock;
     c.Cc = f; f += dm.c;
     c.Ac = f; f += dm.c;
     c.IRCs = f; f += dm.c;
-    c.q = f; f += dm.g;
-    c.LQ = f; f += dm.g;
+    c.qa = f; f += dm.g;
+    c.qb = f; f += dm.g;
     c.cgb = f; f += dm.ch;
     c.cerev = f; f += dm.ch;
     int32_t *i = reinterpret_cast<int32_t *>(f);
@@ -166,7 +197,7 @@ __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dim
     c.ch0 = i; i += dm.c + 1;
     c.ctype = i; i += dm.ch;
     c.cg0 = i; i += dm.ch;
-    c.cslot = i;
+    c.gmap = i;
     c.c0 = m.cell_c0[cell];
     c.nc = m.cell_c0[cell + 1] - c.c0;
     c.g0 = m.cell_g0[cell];
@@ -175,18 +206,15 @@ __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dim
     c.nch = m.cell_ch0[cell + 1] - h0;
     c.lev = m.lev + m.cell_l0[cell];
     c.nlev = m.cell_l0[cell + 1] - m.cell_l0[cell] - 1;
-    c.ra_slot = m.cell_ra_slot[cell];
     c.serial = c.nc <= 6 * c.nlev;
     c.chain = m.cell_chain[cell] != 0;
-    const int rp = m.cell_ra_param[cell];
-    const float s = rp >= 0 ? m.cell_ra[cell] / m.params[rp] : 1.0f;
+    const float s = axial_scale(m, cell);
     const int words = (int)(sizeof(EdenGpuChannelType) / 4) * m.n_types;
-    for (int k = lane; k < words; k += 32)
+    for (int k = tid; k < words; k += nt)
         reinterpret_cast<int32_t *>(c.types)[k] = reinterpret_cast<const int32_t *>(m.types)[k];
-    for (int j = lane; j < c.nc; j += 32) {
+    for (int j = tid; j < c.nc; j += nt) {
         const int gc = c.c0 + j;
-        c.Us[j] = m.U[gc] * s;
-        c.Ls[j] = m.L[gc] * s;
+        c.UL[j] = make_float2(m.U[gc] * s, m.L[gc] * s);
         c.IRCs[j] = m.IRC[gc] * s;
         c.Cc[j] = m.C[gc];
         c.Ac[j] = m.A[gc];
@@ -195,17 +223,22 @@ __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dim
         c.CE[j] = m.CE[gc];
         c.ch0[j] = m.comp_ch0[gc];
     }
-    if (lane == 0) c.ch0[c.nc] = c.nch;
-    for (int k = lane; k < c.nch; k += 32) {
+    // (what the padding holds is computed with, and not used)
+    if (tid < kBlock) {
+        c.XD[-1 - tid] = c.XD[c.nc + tid] = make_float2(0.0f, 1.0f);
+        c.UL[-1 - tid] = c.UL[c.nc + tid] = make_float2(0.0f, 0.0f);
+    }
+    if (tid == 0) c.ch0[c.nc] = c.nch;
+    for (int k = tid; k < c.nch; k += nt) {
         const int ch = h0 + k;
         const int p = m.ch_param[ch];
         c.ctype[k] = m.ch_type[ch];
         c.cg0[k] = m.ch_g0[ch];
-        c.cslot[k] = m.ch_slot[ch];
         c.cgb[k] = p >= 0 ? m.params[p] : m.ch_gbase[ch];
         c.cerev[k] = m.ch_erev[ch];
     }
-    __syncwarp();
+    for (int k = tid; k < c.ng; k += nt) c.gmap[k] = m.gate_map[c.g0 + k];
+    __syncthreads();
     return c;
 }
 
@@ -233,22 +266,28 @@ __device__ __forceinline__ float rate_slope(int kind, float r, float mid, float 
     return r * fp / s;
 }
 
-// Channels and V pre-update of compartment j at time t: advances its gates
-// in place and returns the pre-updated V (x) and the diagonal term d, with
-// the plain path's operations (target_step).
-__device__ __forceinline__ void comp_pre(const GradDev &m, const Cell &c, int j, int64_t n, float t, float v,
-                                         bool init, float &x, float &d) {
+// A gate's next value (gate_relax, as the plain path's target_step).
+__device__ __forceinline__ float gate_step(const GradDev &m, const Cell &c, int k, float v, float qo, bool init) {
+    const EdenGpuChannelType &ct = c.types[(uint32_t)c.gmap[k] >> 18];
+    const int g = (c.gmap[k] >> 16) & 3;
+    const float al = rate_value(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v);
+    const float be = rate_value(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v);
+    return gate_relax(al, be, ct.q10[g], init, m.dt, qo);
+}
+
+// Channel currents and V pre-update of compartment j at time t, from the gates
+// at the step's start: the pre-updated V (x) and the diagonal term d, with the
+// plain path's operations (target_step).
+__device__ __forceinline__ void comp_pre(const GradDev &m, const Cell &c, const float *q, int j, int64_t n, float t, float v,
+                                         float &x, float &d) {
     const float A = c.Ac[j];
     float Ich = 0.0f, Gch = 0.0f;
     for (int k = c.ch0[j]; k < c.ch0[j + 1]; k++) {
         const EdenGpuChannelType &ct = c.types[c.ctype[k]];
-        float *qq = c.q + c.cg0[k];
+        const float *qq = q + c.cg0[k];
         float fopen = 1.0f;
         for (int g = 0; g < ct.n_gates; g++) {
             const float qo = qq[g];
-            const float al = rate_value(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v);
-            const float be = rate_value(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v);
-            qq[g] = gate_relax(al, be, ct.q10[g], init, m.dt, qo);
             for (int r = 0; r < ct.gate_instances[g]; r++) fopen = fopen * qo;
         }
         const float gs = c.cgb[k] * fopen;
@@ -263,74 +302,76 @@ __device__ __forceinline__ void comp_pre(const GradDev &m, const Cell &c, int j,
     }
     // synaptic drive: inputs, then connections (eden/Eden.cpp:6057-6060)
     float Gin = 0.0f, Isyn = 0.0f, Gsyn = 0.0f;
-    if (!init)
-        for (int k = m.comp_gr0[gc]; k < m.comp_gr0[gc + 1]; k++) {
-            const float g = m.gtab[n * m.n_grp + k];
-            if (m.gr_kind[k] == 0) {
-                Iin += g * (m.gr_erev[k] - v);
-                Gin += g;
-            } else {
-                Isyn += g * (m.gr_erev[k] - v);
-                Gsyn += g;
-            }
+    for (int k = m.comp_gr0[gc]; k < m.comp_gr0[gc + 1]; k++) {
+        const float g = m.gtab[n * m.n_grp + k];
+        if (m.gr_kind[k] == 0) {
+            Iin += g * (m.gr_erev[k] - v);
+            Gin += g;
+        } else {
+            Isyn += g * (m.gr_erev[k] - v);
+            Gsyn += g;
         }
+    }
     const float I = Ich + Iin + Isyn;
     const float G = Gch + Gin + Gsyn;
     const float C = c.Cc[j];
     d = 1.0f * (G / C) + c.IRCs[j];
-    x = init ? v : v + (m.dt * (I + (v * G))) / C;
+    x = v + (m.dt * (I + (v * G))) / C;
 }
 
-// The total conductance of compartment gc at step n, its channels' Gch
-// plus its drive groups', summed in comp_pre's order.
-__device__ __forceinline__ float total_g(const GradDev &m, int gc, int64_t n, float Gch) {
-    float Gin = 0.0f, Gsyn = 0.0f;
-    for (int k = m.comp_gr0[gc]; k < m.comp_gr0[gc + 1]; k++) {
-        const float g = m.gtab[n * m.n_grp + k];
-        if (m.gr_kind[k] == 0) Gin += g;
-        else Gsyn += g;
-    }
-    return Gch + Gin + Gsyn;
-}
-
-// Backward-Euler Hines solve of the cell (eden/Eden.cpp:6114-6225): D holds
-// the diagonal terms on entry and the reciprocal pivots on return, X the
-// pre-updated V on entry and V_next on return; every node pulls its children
-// in order, deepest first, then back-substitution runs root first.  With
-// `transposed` it solves M^T y = X: the same pivots, the right-hand side
-// eliminated with U and back-substituted with L.  Cells with few
-// compartments per depth (chains, ball-and-stick) are solved by one lane in
-// reverse breadth-first order with the last node's values in registers; the
-// others depth by depth across the warp.  Both do the same operations.
-__device__ __forceinline__ void hines_cell(float dt, const Cell &c, bool transposed) {
+// Backward-Euler Hines solve of the cell (eden/Eden.cpp:6114-6225) by one warp,
+// from XD, which keeps the eliminated V and the reciprocal pivots, into VN;
+// every node pulls its children in order, deepest first, then back-substitution
+// runs root first.  Cells with few compartments per depth (chains,
+// ball-and-stick) are solved by one lane in reverse breadth-first order with the
+// last node's values in registers; the others depth by depth across the warp.
+// Both do the same operations.
+__device__ __forceinline__ void hines_cell(const Cell &c, float *VN) {
     const int lane = threadIdx.x & 31;
-    float *D = c.D, *X = c.X;
+    float2 *XD = c.XD;
+    const float2 *UL = c.UL;
     if (c.chain) {
-        // the same operations with every value of the previous node in registers
+        // the next nodes are loaded before these are stored: left to itself the
+        // compiler keeps a load behind a store that might be to the same place.
+        // The last block runs into the padding.
         if (lane == 0) {
             const int n = c.nc;
-            float rc = __fdividef(1.0f, 1.0f + D[n - 1] * dt);
-            float xc = X[n - 1];
-            D[n - 1] = rc;
-#pragma unroll 4
-            for (int j = n - 2; j >= 0; j--) {
-                const float Ui = c.Us[j + 1];
-                const float ratio = c.Ls[j + 1] * rc;
-                float dj = 1.0f + D[j] * dt;
-                dj -= ratio * Ui;
-                const float xj = X[j] - (transposed ? Ui * rc : ratio) * xc;
-                X[j] = xj;
-                rc = __fdividef(1.0f, dj);
-                D[j] = rc;
-                xc = xj;
+            float rc = pivot(XD[n - 1].y), xc = XD[n - 1].x;
+            XD[n - 1].y = rc;
+            float2 xd[kBlock], ul[kBlock];
+#pragma unroll
+            for (int k = 0; k < kBlock; k++) { xd[k] = XD[n - 2 - k]; ul[k] = UL[n - 1 - k]; }
+            for (int j = n - 2; j >= 0; j -= kBlock) {
+                float2 out[kBlock];
+#pragma unroll
+                for (int k = 0; k < kBlock; k++) {
+                    const float ratio = ul[k].y * rc;
+                    rc = pivot(fmaf(-ratio, ul[k].x, xd[k].y));
+                    xc = fmaf(-ratio, xc, xd[k].x);
+                    out[k] = make_float2(xc, rc);
+                }
+                if (j >= kBlock)
+#pragma unroll
+                    for (int k = 0; k < kBlock; k++) { xd[k] = XD[j - kBlock - k]; ul[k] = UL[j + 1 - kBlock - k]; }
+#pragma unroll
+                for (int k = 0; k < kBlock; k++) XD[j - k] = out[k];
             }
-            float xp = X[0] * D[0];
-            X[0] = xp;
-#pragma unroll 4
-            for (int j = 1; j < n; j++) {
-                const float off = transposed ? c.Ls[j] : c.Us[j];
-                xp = (X[j] - off * xp) * D[j];
-                X[j] = xp;
+            float xp = XD[0].x * XD[0].y;
+            VN[0] = xp;
+#pragma unroll
+            for (int k = 0; k < kBlock; k++) { xd[k] = XD[1 + k]; ul[k] = UL[1 + k]; }
+            for (int j = 1; j < n; j += kBlock) {
+                float out[kBlock];
+#pragma unroll
+                for (int k = 0; k < kBlock; k++) {
+                    xp = fmaf(-ul[k].x, xp, xd[k].x) * xd[k].y;
+                    out[k] = xp;
+                }
+                if (j + kBlock < n)
+#pragma unroll
+                    for (int k = 0; k < kBlock; k++) { xd[k] = XD[j + kBlock + k]; ul[k] = UL[j + kBlock + k]; }
+#pragma unroll
+                for (int k = 0; k < kBlock; k++) VN[j + k] = out[k];
             }
         }
         __syncwarp();
@@ -342,271 +383,456 @@ __device__ __forceinline__ void hines_cell(float dt, const Cell &c, bool transpo
             int last = -1;
             for (int j = c.nc - 1; j >= 0; j--) {
                 const int kb = c.CB[j], ke = c.CE[j];
-                float dj = 1.0f + D[j] * dt;
-                float xj = X[j];
-                if (ke > kb) {
-                    for (int i = kb; i < ke; i++) {
-                        const float xi = i == last ? xc : X[i];
-                        const float ri = i == last ? rc : D[i];
-                        const float Ui = c.Us[i];
-                        const float ratio = c.Ls[i] * ri;
-                        dj -= ratio * Ui;
-                        xj -= (transposed ? Ui * ri : ratio) * xi;
-                    }
-                    X[j] = xj;
+                float2 v = XD[j];
+                for (int i = kb; i < ke; i++) {
+                    const float2 k = i == last ? make_float2(xc, rc) : XD[i];
+                    const float ratio = UL[i].y * k.y;
+                    v.y = fmaf(-ratio, UL[i].x, v.y);
+                    v.x = fmaf(-ratio, k.x, v.x);
                 }
-                rc = __fdividef(1.0f, dj);
-                D[j] = rc;
-                xc = xj;
+                rc = pivot(v.y);
+                xc = v.x;
+                XD[j] = make_float2(xc, rc);
                 last = j;
             }
-            float xp = X[0] * D[0];
-            X[0] = xp;
+            float xp = XD[0].x * XD[0].y;
+            VN[0] = xp;
             for (int j = 1; j < c.nc; j++) {
                 const int p = c.P[j];
-                const float off = transposed ? c.Ls[j] : c.Us[j];
-                const float xpar = p == j - 1 ? xp : X[p];
-                xp = (X[j] - off * xpar) * D[j];
-                X[j] = xp;
+                xp = fmaf(-UL[j].x, p == j - 1 ? xp : VN[p], XD[j].x) * XD[j].y;
+                VN[j] = xp;
             }
         }
         __syncwarp();
         return;
     }
-    for (int j = lane; j < c.nc; j += 32) D[j] = 1.0f + D[j] * dt;
-    __syncwarp();
     for (int l = c.nlev - 1; l >= 0; l--) {
         for (int j = c.lev[l] + lane; j < c.lev[l + 1]; j += 32) {
-            const int kb = c.CB[j], ke = c.CE[j];
-            float dj = D[j];
-            if (ke > kb) {
-                float xj = X[j];
-                for (int i = kb; i < ke; i++) {
-                    const float Ui = c.Us[i];
-                    const float ratio = c.Ls[i] * D[i];
-                    dj -= ratio * Ui;
-                    xj -= (transposed ? Ui * D[i] : ratio) * X[i];
-                }
-                X[j] = xj;
+            float2 v = XD[j];
+            for (int i = c.CB[j]; i < c.CE[j]; i++) {
+                const float2 k = XD[i];
+                const float ratio = UL[i].y * k.y;
+                v.y = fmaf(-ratio, UL[i].x, v.y);
+                v.x = fmaf(-ratio, k.x, v.x);
             }
-            D[j] = __fdividef(1.0f, dj);
+            XD[j] = make_float2(v.x, pivot(v.y));
         }
         __syncwarp();
     }
-    for (int r = c.lev[0] + lane; r < c.lev[1]; r += 32) X[r] = X[r] * D[r];
+    for (int r = c.lev[0] + lane; r < c.lev[1]; r += 32) VN[r] = XD[r].x * XD[r].y;
     __syncwarp();
     for (int l = 1; l < c.nlev; l++) {
-        for (int i = c.lev[l] + lane; i < c.lev[l + 1]; i += 32) {
-            const float off = transposed ? c.Ls[i] : c.Us[i];
-            X[i] = (X[i] - off * X[c.P[i]]) * D[i];
-        }
+        for (int i = c.lev[l] + lane; i < c.lev[l + 1]; i += 32) VN[i] = fmaf(-UL[i].x, VN[c.P[i]], XD[i].x) * XD[i].y;
         __syncwarp();
     }
 }
 
-// One forward step n -> n + 1 of the staged cell.
-__device__ __forceinline__ void forward_step(const GradDev &m, const Cell &c, int64_t n) {
-    const int lane = threadIdx.x & 31;
-    const float t = m.tk[n];
-    for (int j = lane; j < c.nc; j += 32) {
-        float x, d;
-        comp_pre(m, c, j, n, t, c.V[j], false, x, d);
-        c.X[j] = x;
-        c.D[j] = d;
-    }
-    __syncwarp();
-    hines_cell(m.dt, c, false);
-    for (int j = lane; j < c.nc; j += 32) c.V[j] = c.X[j];
-    __syncwarp();
-}
-
-__global__ void __launch_bounds__(32) k_grad_forward(GradDev m, Dims dm) {
-    const int cell = blockIdx.x, lane = threadIdx.x;
+// The run of a cell (block x) over steps [1, N], or, recomputing, over segment
+// seg0 + block y from its checkpoint.  The first `cw` warps compute the currents
+// and the first of them solves the cable; the others update the gates in the
+// meantime, into the other of two buffers, and write the step's records.  A
+// step is the currents and the solve one after the other: on a cable of 51
+// compartments 2,700 cycles of the solve's chain (a product, a fused one and a
+// reciprocal a compartment) and about 500 of the rest, where one warp a cell,
+// taking its 153 gates in turns before the solve, took 16,000.
+template <bool RECOMPUTE>
+__global__ void __launch_bounds__(32 * kFwdWarps) k_grad_forward(GradDev m, Dims dm, int cw, int64_t seg0, int keep) {
+    const int cell = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Cell c = stage_cell(m, cell, dm);
-    for (int j = lane; j < c.nc; j += 32) c.V[j] = m.V0[c.c0 + j];
-    for (int k = lane; k < c.ng; k += 32) c.q[k] = 0.0f;
-    __syncwarp();
-    // the four initialisation passes leave V and set every gate to inf(V)
-    for (int j = lane; j < c.nc; j += 32) {
-        float x, d;
-        comp_pre(m, c, j, 0, 0.0f, c.V[j], true, x, d);
+    const int64_t seg = RECOMPUTE ? seg0 + blockIdx.y : 0;
+    const int64_t first = 1 + seg * m.S, end = RECOMPUTE && first + m.S < m.N ? first + m.S : m.N;
+    float *V = c.Va, *Vn = c.Vb, *q = c.qa, *qn = c.qb;  // at the step's start, and the next's
+    if (RECOMPUTE) {
+        for (int j = tid; j < c.nc; j += blockDim.x) V[j] = m.ck_v[seg * m.n_comp + c.c0 + j];
+        for (int k = tid; k < c.ng; k += blockDim.x) q[k] = m.ck_q[seg * m.n_gate + c.g0 + k];
+    } else {
+        // the four initialisation passes leave V and set every gate to inf(V)
+        for (int j = tid; j < c.nc; j += blockDim.x) V[j] = m.V0[c.c0 + j];
+        __syncthreads();
+        for (int k = tid; k < c.ng; k += blockDim.x) q[k] = gate_step(m, c, k, V[c.gmap[k] & 0xffff], 0.0f, true);
     }
     const int r0 = m.cell_r0[cell], r1 = m.cell_r0[cell + 1];
+    // threads of the gates' share (all of them where there is one share)
+    const int gw = (int)(blockDim.x >> 5) - cw, gt = gw > 0 ? tid - 32 * cw : tid, gn = gw > 0 ? 32 * gw : (int)blockDim.x;
     int64_t ck = 0;
     int to_ck = 0;  // steps until the next checkpoint
-    for (int64_t n = 1; n <= m.N; n++) {
-        __syncwarp();
-        if (to_ck == 0 && n < m.N) {
-            for (int j = lane; j < c.nc; j += 32) m.ck_v[ck * m.n_comp + c.c0 + j] = c.V[j];
-            for (int k = lane; k < c.ng; k += 32) m.ck_q[ck * m.n_gate + c.g0 + k] = c.q[k];
+    __syncthreads();
+    for (int64_t n = first; n <= end; n++) {
+        if (gt >= 0) {
+            if (!RECOMPUTE && to_ck == 0 && n < m.N) {
+                for (int j = gt; j < c.nc; j += gn) m.ck_v[ck * m.n_comp + c.c0 + j] = V[j];
+                for (int k = gt; k < c.ng; k += gn) m.ck_q[ck * m.n_gate + c.g0 + k] = q[k];
+            }
+            // (a segment's last state is the next one's first, which writes it)
+            if (RECOMPUTE ? n < end || blockIdx.y + 1 == gridDim.y : keep) {
+                const int64_t row = n - m.tr_n0;
+                for (int j = gt; j < c.nc; j += gn) m.tr_v[row * m.n_comp + c.c0 + j] = V[j];
+                for (int k = gt; k < c.ng; k += gn) m.tr_q[row * m.n_gate + c.g0 + k] = q[k];
+            }
+            if (!RECOMPUTE)
+                for (int r = r0 + gt; r < r1; r += gn) m.trace[(n - 1) * m.n_rec + m.rec_col[r]] = V[m.rec_local[r]];
+        }
+        if (to_ck == 0) {
             ck++;
             to_ck = m.S;
         }
         to_ck--;
-        for (int r = r0 + lane; r < r1; r += 32) m.trace[(n - 1) * m.n_rec + m.rec_col[r]] = c.V[m.rec_local[r]];
-        if (n < m.N) forward_step(m, c, n);
+        if (n == end) break;
+        if (warp < cw) {
+            const float t = m.tk[n];
+            for (int j = tid; j < c.nc; j += 32 * cw) {
+                float x, d;
+                comp_pre(m, c, q, j, n, t, V[j], x, d);
+                c.XD[j] = make_float2(x, fmaf(d, m.dt, 1.0f));
+            }
+            // (the warps of the currents only: named barrier 1)
+            if (cw > 1) asm volatile("bar.sync 1, %0;" ::"r"(32 * cw) : "memory");
+            else __syncwarp();
+            if (warp == 0) {
+                hines_cell(c, Vn);
+                if (RECOMPUTE || keep)
+                    for (int j = lane; j < c.nc; j += 32) m.tr_d[(n - m.tr_n0) * m.n_comp + c.c0 + j] = c.XD[j].y;
+            }
+        }
+        if (gt >= 0)
+            for (int k = gt; k < c.ng; k += gn) qn[k] = gate_step(m, c, k, V[c.gmap[k] & 0xffff], q[k], false);
+        __syncthreads();
+        float *x = V;
+        V = Vn;
+        Vn = x;
+        x = q;
+        q = qn;
+        qn = x;
     }
 }
 
-// lV += the trace gradient of step n (one lane: recorded columns may share
-// a compartment).
-__device__ __forceinline__ void add_trace_grad(const GradDev &m, int cell, int64_t n, float *LV) {
-    if ((threadIdx.x & 31) == 0)
-        for (int r = m.cell_r0[cell]; r < m.cell_r0[cell + 1]; r++)
-            LV[m.rec_local[r]] += m.trace_grad[(n - 1) * m.n_rec + m.rec_col[r]];
-    __syncwarp();
+// The adjoint's coefficients of `rows` steps from co_n0 on, a thread per step and
+// compartment.  dQ/dq = b and dQ/dV = cv where the gate did not clamp, 0 where
+// it did; d fopen / dq_g = inst q_g^(inst-1) * prod over the other gates.
+__global__ void __launch_bounds__(128) k_grad_coef(GradDev m, int64_t rows) {
+    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= rows * m.n_comp) return;
+    const int64_t row = id / m.n_comp;
+    const int gc = (int)(id - row * m.n_comp);
+    const int64_t tr = m.co_n0 + row - m.tr_n0;
+    const int cell = m.comp_cell[gc], c0 = m.cell_c0[cell], nc = m.cell_c0[cell + 1] - c0, j = gc - c0;
+    const int g0 = m.cell_g0[cell], ng = m.cell_g0[cell + 1] - g0;
+    float *co = m.co + row * m.co_len + m.cell_k0[cell];
+    const float dt = m.dt, s = axial_scale(m, cell);
+    const float rc = m.tr_d[tr * m.n_comp + gc];
+    co[j] = (m.U[gc] * s) * rc;
+    co[nc + j] = (m.L[gc] * s) * rc;
+    co[2 * nc + j] = rc;
+    co += 3 * nc;
+    const float v = m.tr_v[tr * m.n_comp + gc], vn = m.tr_v[(tr + 1) * m.n_comp + gc];
+    const float *q = m.tr_q + tr * m.n_gate + g0;
+    const float C = m.C[gc], A = m.A[gc];
+    const int h0 = m.cell_ch0[cell], hend = j + 1 < nc ? h0 + m.comp_ch0[gc + 1] : m.cell_ch0[cell + 1];
+    for (int h = h0 + m.comp_ch0[gc]; h < hend; h++) {
+        const EdenGpuChannelType &ct = m.types[m.ch_type[h]];
+        const int q0 = m.ch_g0[h], p = m.ch_param[h];
+        float qo[EDEN_MAX_GATES], pw[EDEN_MAX_GATES];
+#pragma unroll
+        for (int g = 0; g < EDEN_MAX_GATES; g++) {
+            qo[g] = 1.0f;
+            pw[g] = 1.0f;
+            if (g < ct.n_gates) {
+                qo[g] = q[q0 + g];
+                float x = 1.0f;
+                for (int r = 0; r < ct.gate_instances[g]; r++) x = x * qo[g];
+                pw[g] = x;
+            }
+        }
+        // d(loss)/d(conductance) is mu times this
+        const float gb = p >= 0 ? m.params[p] : m.ch_gbase[h];
+        const float fb = ((-dt * vn + dt * m.ch_erev[h]) / C) * gb * 1e-5f * A;
+#pragma unroll
+        for (int g = 0; g < EDEN_MAX_GATES; g++) {
+            if (g >= ct.n_gates) break;
+            const int inst = ct.gate_instances[g];
+            float dfdq = 0.0f;
+            if (inst > 0) {
+                dfdq = (float)inst;
+                for (int r = 1; r < inst; r++) dfdq = dfdq * qo[g];
+#pragma unroll
+                for (int h2 = 0; h2 < EDEN_MAX_GATES; h2++)
+                    if (h2 != g) dfdq = dfdq * pw[h2];
+            }
+            const float al = rate_value(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v);
+            const float be = rate_value(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v);
+            const float sum = al + be;
+            const float tau = 1.0f / sum;
+            const float inf = al / sum;
+            const float b = expf(-((dt * ct.q10[g]) / tau));
+            const float qn = b * qo[g] + (1.0f - b) * inf;
+            const bool clamped = !(qn > 1e-6f) || !(qn < (float)(1 - 1e-6));
+            float cv = 0.0f;
+            if (!clamped) {
+                const float dal = rate_slope(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v, al);
+                const float dbe = rate_slope(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v, be);
+                const float db = -(dt * ct.q10[g]) * (dal + dbe) * b;
+                const float dinf = (dal * be - al * dbe) / (sum * sum);
+                cv = db * (qo[g] - inf) + (1.0f - b) * dinf;
+            }
+            co[q0 + g] = clamped ? 0.0f : b;
+            co[ng + q0 + g] = cv;
+            co[2 * ng + q0 + g] = fb * dfdq;
+        }
+    }
 }
 
-// Adjoint of step n -> n + 1: on entry V = V^n, VN = V^{n+1}, q = q^n, LV and
-// LQ the adjoints of V^{n+1} and q^{n+1}; on return LV and LQ are those of
-// V^n and q^n, and the parameter terms of the step are in acc.
-__device__ __forceinline__ void adjoint_step(const GradDev &m, const Cell &c, int64_t n) {
+// M^T y = X for the staged cell, from the factors of M^T: y up, F = U / pivot of
+// the child, down, A = L / pivot of the node, D the reciprocal pivots.  X is
+// replaced by the solution.
+__device__ __forceinline__ void adjoint_solve(float *X, const float *F, const float *A, const float *D, int nc, bool chain,
+                                              bool serial, const int32_t *P, const int32_t *CB, const int32_t *CE,
+                                              const int32_t *lev, int nlev) {
     const int lane = threadIdx.x & 31;
-    const float dt = m.dt;
-    for (int j = lane; j < c.nc; j += 32) {
-        const float A = c.Ac[j];
-        float Gch = 0.0f;
-        for (int k = c.ch0[j]; k < c.ch0[j + 1]; k++) {
-            const EdenGpuChannelType &ct = c.types[c.ctype[k]];
-            const float *qq = c.q + c.cg0[k];
-            float fopen = 1.0f;
-            for (int g = 0; g < ct.n_gates; g++)
-                for (int r = 0; r < ct.gate_instances[g]; r++) fopen = fopen * qq[g];
-            Gch += ((c.cgb[k] * fopen) * 1e-5f) * A;
+    if (chain) {
+        // both sweeps are first-order recurrences: each lane composes its own
+        // consecutive nodes' maps, a scan over the lanes composes those, and
+        // the lane runs its nodes from what the scan gives (51 nodes: about 200
+        // cycles a sweep, where a node after the other takes twice that, and
+        // longer cables more)
+        const int L = (nc + 31) / 32, ja = lane * L < nc ? lane * L : nc, jb = ja + L < nc ? ja + L : nc;
+        // up: x_j = X_j - F_{j+1} x_{j+1}; the lane's map of the x below it
+        float a = 1.0f, b = 0.0f;
+        for (int j = jb - 1; j >= ja; j--) {
+            const float f = j + 1 < nc ? -F[j + 1] : 0.0f;
+            b = X[j] + f * b;
+            a = f * a;
         }
-        const float G = m.n_grp ? total_g(m, c.c0 + j, n, Gch) : Gch;
-        c.D[j] = 1.0f * (G / c.Cc[j]) + c.IRCs[j];
-        c.X[j] = c.LV[j];
-    }
-    __syncwarp();
-    hines_cell(dt, c, true);  // X = mu
-    double *acc = c.acc + lane;
-    for (int j = lane; j < c.nc; j += 32) {
-        const float mu = c.X[j], v = c.V[j], vn = c.VN[j];
-        const float dbar = -dt * mu * vn;
-        float vbar = mu;
-        if (c.ra_slot >= 0) {
-            double r = (double)mu * (double)(dt * c.IRCs[j]) * vn;
-            const int p = c.P[j];
-            if (p >= 0) r += (double)mu * (double)c.Us[j] * c.VN[p] + (double)c.X[p] * (double)c.Ls[j] * vn;
-            acc[c.ra_slot * 32] += r;
-        }
-        const float C = c.Cc[j], A = c.Ac[j];
-        // the drive groups' conductance adjoints, for the weight gradients
-        for (int k = m.comp_gr0[c.c0 + j]; k < m.comp_gr0[c.c0 + j + 1]; k++)
-            m.gbar[n * m.n_grp + k] = (dbar + mu * dt * m.gr_erev[k]) / C;
-        for (int k = c.ch0[j]; k < c.ch0[j + 1]; k++) {
-            const EdenGpuChannelType &ct = c.types[c.ctype[k]];
-            const int q0 = c.cg0[k];
-            float qo[EDEN_MAX_GATES], pw[EDEN_MAX_GATES];
-            float fopen = 1.0f;
 #pragma unroll
-            for (int g = 0; g < EDEN_MAX_GATES; g++) {
-                qo[g] = 1.0f;
-                pw[g] = 1.0f;
-                if (g < ct.n_gates) {
-                    qo[g] = c.q[q0 + g];
-                    float p = 1.0f;
-                    for (int r = 0; r < ct.gate_instances[g]; r++) p = p * qo[g];
-                    pw[g] = p;
-                    fopen = fopen * p;
-                }
-            }
-            const float gb = c.cgb[k];
-            const float gbar = (dbar + mu * dt * c.cerev[k]) / C;
-            const int slot = c.cslot[k];
-            if (slot >= 0) acc[slot * 32] += (double)gbar * (double)(fopen * 1e-5f * A);
-            const float fbar = gbar * gb * 1e-5f * A;
-#pragma unroll
-            for (int g = 0; g < EDEN_MAX_GATES; g++) {
-                if (g >= ct.n_gates) break;
-                // d fopen / d q_g = inst q_g^(inst-1) * prod over the other gates
-                const int inst = ct.gate_instances[g];
-                float dfdq = 0.0f;
-                if (inst > 0) {
-                    dfdq = (float)inst;
-                    for (int r = 1; r < inst; r++) dfdq = dfdq * qo[g];
-#pragma unroll
-                    for (int h = 0; h < EDEN_MAX_GATES; h++)
-                        if (h != g) dfdq = dfdq * pw[h];
-                }
-                const float al = rate_value(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v);
-                const float be = rate_value(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v);
-                const float sum = al + be;
-                const float tau = 1.0f / sum;
-                const float inf = al / sum;
-                const float b = expf(-((dt * ct.q10[g]) / tau));
-                const float qn = b * qo[g] + (1.0f - b) * inf;
-                const bool clamped = !(qn > 1e-6f) || !(qn < (float)(1 - 1e-6));
-                const float lq = c.LQ[q0 + g];
-                float qbar = fbar * dfdq;
-                if (!clamped) {
-                    const float dal = rate_slope(ct.fwd_kind[g], ct.fwd_rate[g], ct.fwd_mid[g], ct.fwd_scale[g], v, al);
-                    const float dbe = rate_slope(ct.rev_kind[g], ct.rev_rate[g], ct.rev_mid[g], ct.rev_scale[g], v, be);
-                    const float db = -(dt * ct.q10[g]) * (dal + dbe) * b;
-                    const float dinf = (dal * be - al * dbe) / (sum * sum);
-                    vbar += lq * (db * (qo[g] - inf) + (1.0f - b) * dinf);
-                    qbar += lq * b;
-                }
-                c.LQ[q0 + g] = qbar;
+        for (int o = 1; o < 32; o <<= 1) {
+            const float a2 = __shfl_down_sync(0xffffffffu, a, o), b2 = __shfl_down_sync(0xffffffffu, b, o);
+            if (lane + o < 32) {
+                b += a * b2;
+                a *= a2;
             }
         }
-        c.LV[j] = vbar;
-    }
-    __syncwarp();
-}
-
-__global__ void __launch_bounds__(32) k_grad_backward(GradDev m, Dims dm) {
-    const int cell = blockIdx.x, lane = threadIdx.x;
-    const Cell c = stage_cell(m, cell, dm);
-    const int s0 = m.cell_s0[cell], ns = m.cell_s0[cell + 1] - s0;
-    for (int k = 0; k < ns; k++) c.acc[k * 32 + lane] = 0.0;
-    for (int j = lane; j < c.nc; j += 32) c.LV[j] = 0.0f;
-    for (int k = lane; k < c.ng; k += 32) c.LQ[k] = 0.0f;
-    __syncwarp();
-    add_trace_grad(m, cell, m.N, c.LV);
-    const int64_t nseg = m.N >= 2 ? (m.N - 2) / m.S + 1 : 0;
-    for (int64_t sg = nseg - 1; sg >= 0; sg--) {
-        const int64_t n0 = 1 + sg * m.S, n1 = n0 + m.S < m.N ? n0 + m.S : m.N;
-        // recompute the segment's states n0 .. n1 from its checkpoint
-        for (int j = lane; j < c.nc; j += 32) {
-            const float v = m.ck_v[sg * m.n_comp + c.c0 + j];
-            c.V[j] = v;
-            m.tr_v[c.c0 + j] = v;
+        float x = __shfl_down_sync(0xffffffffu, b, 1);
+        if (lane == 31) x = 0.0f;
+        for (int j = jb - 1; j >= ja; j--) {
+            x = X[j] - (j + 1 < nc ? F[j + 1] : 0.0f) * x;
+            X[j] = x * D[j];
         }
-        for (int k = lane; k < c.ng; k += 32) {
-            const float q = m.ck_q[sg * m.n_gate + c.g0 + k];
-            c.q[k] = q;
-            m.tr_q[c.g0 + k] = q;
+        // down: v_j = X_j D_j - A_j v_{j-1}
+        a = 1.0f;
+        b = 0.0f;
+        for (int j = ja; j < jb; j++) {
+            const float f = j > 0 ? -A[j] : 0.0f;
+            b = X[j] + f * b;
+            a = f * a;
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float a2 = __shfl_up_sync(0xffffffffu, a, o), b2 = __shfl_up_sync(0xffffffffu, b, o);
+            if (lane >= o) {
+                b += a * b2;
+                a *= a2;
+            }
+        }
+        x = __shfl_up_sync(0xffffffffu, b, 1);
+        if (lane == 0) x = 0.0f;
+        for (int j = ja; j < jb; j++) {
+            x = X[j] - (j > 0 ? A[j] : 0.0f) * x;
+            X[j] = x;
         }
         __syncwarp();
-        for (int64_t n = n0; n < n1; n++) {
-            forward_step(m, c, n);
-            const int64_t k = n + 1 - n0;
-            for (int j = lane; j < c.nc; j += 32) m.tr_v[k * m.n_comp + c.c0 + j] = c.V[j];
-            for (int g = lane; g < c.ng; g += 32) m.tr_q[k * m.n_gate + c.g0 + g] = c.q[g];
-            __syncwarp();
-        }
-        // and run the adjoint back through them
-        for (int64_t n = n1 - 1; n >= n0; n--) {
-            const int64_t k = n - n0;
-            for (int j = lane; j < c.nc; j += 32) {
-                c.V[j] = m.tr_v[k * m.n_comp + c.c0 + j];
-                c.VN[j] = m.tr_v[(k + 1) * m.n_comp + c.c0 + j];
+        return;
+    }
+    if (serial) {
+        if (lane == 0) {
+            for (int j = nc - 1; j >= 0; j--) {
+                float x = X[j];
+                for (int i = CB[j]; i < CE[j]; i++) x -= F[i] * X[i];
+                X[j] = x;
             }
-            for (int g = lane; g < c.ng; g += 32) c.q[g] = m.tr_q[k * m.n_gate + c.g0 + g];
-            __syncwarp();
-            adjoint_step(m, c, n);
-            add_trace_grad(m, cell, n, c.LV);
+            X[0] = X[0] * D[0];
+            for (int j = 1; j < nc; j++) X[j] = X[j] * D[j] - A[j] * X[P[j]];
+        }
+        __syncwarp();
+        return;
+    }
+    for (int l = nlev - 1; l >= 0; l--) {
+        for (int j = lev[l] + lane; j < lev[l + 1]; j += 32) {
+            float x = X[j];
+            for (int i = CB[j]; i < CE[j]; i++) x -= F[i] * X[i];
+            X[j] = x;
+        }
+        __syncwarp();
+    }
+    for (int r = lev[0] + lane; r < lev[1]; r += 32) X[r] = X[r] * D[r];
+    __syncwarp();
+    for (int l = 1; l < nlev; l++) {
+        for (int i = lev[l] + lane; i < lev[l + 1]; i += 32) X[i] = X[i] * D[i] - A[i] * X[P[i]];
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ void copy16(float *smem_dst, const float *gmem_src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gmem_src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy4(float *smem_dst, const float *gmem_src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gmem_src)
+                 : "memory");
+}
+
+// The adjoint recurrence of a cell (a block) back over the steps [n0, n0 + rows)
+// whose coefficients are there; lv and lq hold the adjoints of the state after
+// them and receive those of the state before.  The first warp solves; the others
+// fetch a row of coefficients, `ring` - 1 steps ahead of its use, in the
+// meantime; then every thread takes its compartments and their gates.
+__global__ void __launch_bounds__(256) k_grad_adjoint(GradDev m, Dims dm, int64_t rows, int ring, int stage, int last) {
+    extern __shared__ __align__(16) double smem_d[];
+    const int cell = blockIdx.x, tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5;
+    const int c0 = m.cell_c0[cell], nc = m.cell_c0[cell + 1] - c0, g0 = m.cell_g0[cell], ng = m.cell_g0[cell + 1] - g0;
+    const int r0 = m.cell_r0[cell], nr = m.cell_r0[cell + 1] - r0;
+    const int len = (3 * (nc + ng) + 3) & ~3;
+    float *f = reinterpret_cast<float *>(smem_d);
+    float *R = f; f += (size_t)ring * stage;  // a stage: the row, then the step's trace gradients
+    float *X = f; f += dm.c;
+    float *LQ = f; f += dm.g;
+    int32_t *i32 = reinterpret_cast<int32_t *>(f);
+    int32_t *P = i32; i32 += dm.c;
+    int32_t *CB = i32; i32 += dm.c;
+    int32_t *CE = i32; i32 += dm.c;
+    int32_t *G0 = i32; i32 += dm.c + 1;
+    int32_t *RC = i32;
+    for (int j = tid; j < nc; j += nt) {
+        P[j] = m.P[c0 + j]; CB[j] = m.CB[c0 + j]; CE[j] = m.CE[c0 + j];
+        G0[j] = m.comp_g0[c0 + j]; RC[j] = m.comp_rc0[c0 + j] - r0;
+        X[j] = m.lv[c0 + j];
+    }
+    if (tid == 0) { G0[nc] = ng; RC[nc] = nr; }
+    for (int k = tid; k < ng; k += nt) LQ[k] = m.lq[g0 + k];
+    const int32_t *lev = m.lev + m.cell_l0[cell];
+    const int nlev = m.cell_l0[cell + 1] - m.cell_l0[cell] - 1;
+    const bool chain = m.cell_chain[cell] != 0, serial = nc <= 6 * nlev;
+    auto fetch = [&](int64_t row) {  // by the threads of all warps but the first
+        if (row >= 0) {
+            float *dst = R + (row % ring) * stage;
+            const float *src = m.co + row * m.co_len + m.cell_k0[cell];
+            for (int k = 4 * (tid - 32); k < len; k += 4 * (nt - 32)) copy16(dst + k, src + k);
+            const float *tg = m.trace_grad + (m.co_n0 + row - 1) * m.n_rec;
+            for (int r = tid - 32; r < nr; r += nt - 32) copy4(dst + len + r, tg + m.rec_col[r0 + r]);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncthreads();
+    // the trace gradient of the last state, which no step follows
+    if (last)
+        for (int j = tid; j < nc; j += nt)
+            for (int r = RC[j]; r < RC[j + 1]; r++) X[j] += m.trace_grad[(m.N - 1) * m.n_rec + m.rec_col[r0 + r]];
+    if (warp > 0) {
+        fetch(rows - 1);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int k = 1; k < ring - 1; k++) fetch(rows - 1 - k);
+    }
+    for (int64_t row = rows - 1; row >= 0; row--) {
+        __syncthreads();
+        const float *co = R + (row % ring) * stage;
+        if (warp == 0) {
+            adjoint_solve(X, co, co + nc, co + 2 * nc, nc, chain, serial, P, CB, CE, lev, nlev);
+        } else if (ring > 1) {
+            // into the stage of the row before this one's in time, which is done
+            // with; then the next row is there
+            fetch(row - (ring - 1));
+            if (ring == kRing) asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const float *gb = co + 3 * nc, *tg = co + len;
+        for (int j = tid; j < nc; j += nt) {
+            const float mu = X[j];
+            m.mu[row * m.n_comp + c0 + j] = mu;
+            float x = mu;
+            for (int k = G0[j]; k < G0[j + 1]; k++) {
+                const float lq = LQ[k];
+                x += lq * gb[ng + k];
+                LQ[k] = lq * gb[k] + mu * gb[2 * ng + k];
+            }
+            for (int r = RC[j]; r < RC[j + 1]; r++) x += tg[r];
+            X[j] = x;
+        }
+        if (ring == 1) {  // (one row at a time)
+            __syncthreads();
+            if (warp > 0) {
+                fetch(row - 1);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
         }
     }
-    __syncwarp();
-    for (int k = lane; k < ns; k += 32) {
-        double tot = 0.0;
-        for (int l = 0; l < 32; l++) tot += c.acc[k * 32 + l];
-        if (k == c.ra_slot) tot /= (double)m.params[m.cell_ra_param[cell]];
-        m.slot_grad[s0 + k] = tot;
+    __syncthreads();
+    for (int j = tid; j < nc; j += nt) m.lv[c0 + j] = X[j];
+    for (int k = tid; k < ng; k += nt) m.lq[g0 + k] = LQ[k];
+}
+
+// The parameters' terms of kSumSteps steps of a cell (block x: the cell, y: the
+// steps), from mu and the trajectory, in double per thread and slot, then over
+// the threads in order; and the drive groups' conductance adjoints.
+__global__ void __launch_bounds__(64) k_grad_terms(GradDev m, int64_t rows) {
+    extern __shared__ __align__(16) double smem_d[];
+    const int cell = blockIdx.x, tid = threadIdx.x;
+    const int s0 = m.cell_s0[cell], ns = m.cell_s0[cell + 1] - s0;
+    const int c0 = m.cell_c0[cell], nc = m.cell_c0[cell + 1] - c0, h0 = m.cell_ch0[cell], g0 = m.cell_g0[cell];
+    double *acc = smem_d + tid;
+    for (int k = 0; k < ns; k++) acc[64 * k] = 0.0;
+    const int64_t a = (int64_t)blockIdx.y * kSumSteps, b = a + kSumSteps < rows ? a + kSumSteps : rows;
+    const float dt = m.dt, s = axial_scale(m, cell);
+    const int ra = m.cell_ra_slot[cell];
+    for (int j = tid; j < nc; j += 64) {
+        const int gc = c0 + j;
+        const float C = m.C[gc], A = m.A[gc], Us = m.U[gc] * s, Ls = m.L[gc] * s, irc = m.IRC[gc] * s;
+        const int p = m.P[gc], k0 = m.comp_gr0[gc], k1 = m.comp_gr0[gc + 1];
+        const int ha = h0 + m.comp_ch0[gc], hb = j + 1 < nc ? h0 + m.comp_ch0[gc + 1] : m.cell_ch0[cell + 1];
+        for (int64_t row = a; row < b; row++) {
+            const int64_t n = m.co_n0 + row, tr = n - m.tr_n0;
+            const float mu = m.mu[row * m.n_comp + gc], vn = m.tr_v[(tr + 1) * m.n_comp + gc];
+            const float dbar = -dt * mu * vn;
+            if (ra >= 0) {
+                double r = (double)mu * (double)(dt * irc) * vn;
+                if (p >= 0)
+                    r += (double)mu * (double)Us * m.tr_v[(tr + 1) * m.n_comp + c0 + p] +
+                         (double)m.mu[row * m.n_comp + c0 + p] * (double)Ls * vn;
+                acc[64 * ra] += r;
+            }
+            for (int k = k0; k < k1; k++) m.gbar[n * m.n_grp + k] = (dbar + mu * dt * m.gr_erev[k]) / C;
+            for (int h = ha; h < hb; h++) {
+                const int slot = m.ch_slot[h];
+                if (slot < 0) continue;
+                const EdenGpuChannelType &ct = m.types[m.ch_type[h]];
+                const float *q = m.tr_q + tr * m.n_gate + g0 + m.ch_g0[h];
+                float fopen = 1.0f;
+                for (int g = 0; g < ct.n_gates; g++) {
+                    float x = 1.0f;
+                    for (int r = 0; r < ct.gate_instances[g]; r++) x = x * q[g];
+                    fopen = fopen * x;
+                }
+                const float gbar = (dbar + mu * dt * m.ch_erev[h]) / C;
+                acc[64 * slot] += (double)gbar * (double)(fopen * 1e-5f * A);
+            }
+        }
     }
+    __syncthreads();
+    for (int k = tid; k < ns; k += 64) {
+        double tot = 0.0;
+        for (int l = 0; l < 64; l++) tot += smem_d[64 * k + l];
+        m.part[(int64_t)(s0 + k) * m.n_part + blockIdx.y] = tot;
+    }
+}
+
+// slot_grad += the terms of `chunks` blocks of steps, the latest first; a
+// resistivity's share is complete, and divided by it, once `done`.
+__global__ void k_grad_sum(GradDev m, int n_slot, const int32_t *slot_cell, int chunks, int done) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n_slot) return;
+    double tot = m.slot_grad[k];
+    for (int c = chunks - 1; c >= 0; c--) tot += m.part[(int64_t)k * m.n_part + c];
+    const int cell = slot_cell[k];
+    if (done && k - m.cell_s0[cell] == m.cell_ra_slot[cell]) tot /= (double)m.params[m.cell_ra_param[cell]];
+    m.slot_grad[k] = tot;
 }
 
 // The unit-weight exposure of item s at step n and its state update
@@ -628,54 +854,55 @@ __device__ __forceinline__ void item_update(const GradSyn &st, float dt, bool ev
     }
 }
 
-// gtab[n][k] = sum over the group's items of weight * unit-weight exposure,
-// for steps 1 .. N - 1 (one thread per group; items in group order).
-__global__ void k_grad_drive(GradDev m) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m.n_grp) return;
-    const int i0 = m.gr_it0[k], i1 = m.gr_it0[k + 1];
-    for (int i = i0; i < i1; i++) {
-        m.it_a[i] = 0.0f;
-        m.it_b[i] = 0.0f;
-        m.it_cur[i] = m.it_ev0[i];
-    }
-    m.gtab[k] = 0.0f;
-    for (int64_t n = 1; n <= m.N; n++) {
-        float g = 0.0f;
-        for (int i = i0; i < i1; i++) {
-            const GradSyn st = m.syn[m.it_type[i]];
-            float a = m.it_a[i], b = m.it_b[i];
-            const float w = m.it_param[i] >= 0 ? m.params[m.it_param[i]] : m.it_w[i];
-            g += w * item_exposure(st, a, b);
-            const int64_t e = m.it_cur[i];
-            const bool event = e < m.it_ev0[i + 1] && m.it_ev[e] == (int32_t)n;
-            if (event) m.it_cur[i] = e + 1;
-            item_update(st, m.dt, event, a, b);
-            m.it_a[i] = a;
-            m.it_b[i] = b;
-        }
-        m.gtab[n * m.n_grp + k] = g;
-    }
-}
-
-// d loss / d weight of each item: sum over steps 1 .. N - 1 of the group's
-// conductance adjoint times the item's unit-weight exposure, in double.
-__global__ void k_grad_weights(GradDev m) {
+// Unit-weight exposures of the steps [n0, n0 + rows) into ex, a thread per item;
+// the items' states go on from the call before (n0 = 1: from rest).
+__global__ void k_grad_expose(GradDev m, int64_t n0, int64_t rows) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n_item) return;
-    const int k = m.it_grp[i];
     const GradSyn st = m.syn[m.it_type[i]];
-    float a = 0.0f, b = 0.0f;
-    int64_t e = m.it_ev0[i];
+    float a = n0 == 1 ? 0.0f : m.it_a[i], b = n0 == 1 ? 0.0f : m.it_b[i];
+    int64_t e = n0 == 1 ? m.it_ev0[i] : m.it_cur[i];
     const int64_t e1 = m.it_ev0[i + 1];
-    double acc = 0.0;
-    for (int64_t n = 1; n < m.N; n++) {
-        acc += (double)m.gbar[n * m.n_grp + k] * (double)item_exposure(st, a, b);
-        const bool event = e < e1 && m.it_ev[e] == (int32_t)n;
-        if (event) e++;
+    int32_t next = e < e1 ? m.it_ev[e] : -1;
+    for (int64_t r = 0; r < rows; r++) {
+        m.ex[r * m.n_item + i] = item_exposure(st, a, b);
+        const bool event = next == (int32_t)(n0 + r);
+        if (event) next = ++e < e1 ? m.it_ev[e] : -1;
         item_update(st, m.dt, event, a, b);
     }
-    m.item_grad[i] = acc;
+    m.it_a[i] = a;
+    m.it_b[i] = b;
+    m.it_cur[i] = e;
+}
+
+// gtab[n][k] = sum over the group's items of weight * unit-weight exposure for
+// the steps in ex (a thread per step and group; items in group order).
+__global__ void k_grad_drive(GradDev m, int64_t n0, int64_t rows) {
+    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= rows * m.n_grp) return;
+    const int64_t r = id / m.n_grp;
+    const int k = (int)(id - r * m.n_grp);
+    float g = 0.0f;
+    for (int i = m.gr_it0[k]; i < m.gr_it0[k + 1]; i++) {
+        const float w = m.it_param[i] >= 0 ? m.params[m.it_param[i]] : m.it_w[i];
+        g += w * m.ex[r * m.n_item + i];
+    }
+    m.gtab[(n0 + r) * m.n_grp + k] = g;
+}
+
+// d loss / d weight of each item: sum over the steps in ex, up to N - 1, of the
+// group's conductance adjoint times the item's unit-weight exposure, in double
+// (a warp per item), added to what the steps before gave.
+__global__ void k_grad_weights(GradDev m, int64_t n0, int64_t rows) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= m.n_item) return;
+    const int k = m.it_grp[i];
+    double acc = 0.0;
+    for (int64_t r = lane; r < rows && n0 + r < m.N; r += 32)
+        acc += (double)m.gbar[(n0 + r) * m.n_grp + k] * (double)m.ex[r * m.n_item + i];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) m.item_grad[i] = n0 == 1 ? acc : m.item_grad[i] + acc;
 }
 
 }  // namespace eden_grad
@@ -691,7 +918,15 @@ struct EdenGpuGrad {
     std::vector<void *> allocs;
     int n_params = 0, n_cells = 0, n_rec = 0;
     Dims dims{1, 1, 1, 1};
-    size_t smem = 0;
+    // launch shapes: threads of a forward block and its warps of currents; steps
+    // of coefficients in flight in the adjoint, and the floats of one
+    int fwd_threads = 64, fwd_cw = 1, adj_threads = 64, ring = 1, stage = 4;
+    size_t smem = 0, smem_adj = 0;
+    // rows of the buffers: whether every step's trajectory is kept, the segments
+    // recomputed at a time where not, the steps of coefficients, of exposures
+    bool keep = false;
+    int64_t seg_group = 1, co_rows = 1, ex_rows = 1;
+    int32_t *d_slot_cell = nullptr;
     std::vector<int32_t> slot_param;     // slot -> parameter
     std::vector<int32_t> cell_ra_param;  // host copy, for the forward's checks
     std::vector<int32_t> item_param;     // parameter that is each drive item's weight, or -1
@@ -743,6 +978,13 @@ int alloc(EdenGpuGrad *g, T **dst, size_t n) {
 }
 
 bool finite_pos(float x) { return std::isfinite(x) && x > 0.0f; }
+
+// Most bytes of the trajectory and of the adjoint's coefficients, each: 256
+// cells of 51 compartments over 8,001 steps take 2.1 GB and 5.4 GB, and run in
+// one and in three parts.
+constexpr int64_t kTrajectoryBytes = (int64_t)2200 << 20;
+constexpr int64_t kCoefBytes = (int64_t)2 << 30;
+constexpr int64_t kExposureBytes = (int64_t)256 << 20;
 
 int validate(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     if (m->abi_version != EDEN_GPU_ABI_VERSION)
@@ -893,6 +1135,7 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     std::vector<int32_t> ch_type, ch_g0, ch_param, ch_slot;
     std::vector<float> ch_gbase, ch_erev, pu_start, pu_dur, pu_aw;
     std::vector<int32_t> new_of(m->n_comp);  // model compartment -> breadth-first position
+    std::vector<int32_t> comp_g0, comp_cell, gate_map, cell_k0(nphys + 1, 0), slot_cell;
     // pulses by compartment, in pulse order
     std::vector<std::vector<int64_t>> pulses_of(m->n_comp);
     for (int64_t k = 0; k < m->n_pulse; k++) pulses_of[m->pulse_target[k]].push_back(k);
@@ -951,6 +1194,8 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
                 L[gn] = -dt / (R * m->comp_c[a + p]);
             }
             comp_ch0.push_back((int32_t)ch_type.size() - ch_first);  // local to the cell
+            comp_g0.push_back((int32_t)(n_gate - gbase_cell));
+            comp_cell.push_back(c);
             for (int ch = m->comp_chan_off[gi]; ch < m->comp_chan_off[gi + 1]; ch++) {
                 const int pp = s->chan_param ? s->chan_param[ch] : -1;
                 ch_type.push_back(m->chan_type[ch]);
@@ -959,6 +1204,8 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
                 ch_slot.push_back(pp >= 0 ? slot_of(pp) : -1);
                 ch_gbase.push_back(m->chan_gbase[ch]);
                 ch_erev.push_back(m->chan_erev[ch]);
+                for (int q = 0; q < m->chan_types[m->chan_type[ch]].n_gates; q++)
+                    gate_map.push_back((int32_t)((uint32_t)h | (uint32_t)(m->chan_type[ch] << 2 | q) << 16));
                 n_gate += m->chan_types[m->chan_type[ch]].n_gates;
             }
             for (int64_t k : pulses_of[gi]) {
@@ -975,7 +1222,12 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
         }
         if ((int)slots.size() > kMaxSlots)
             return g->fail(EDEN_GPU_E_INVALID, "cell %d uses %d parameters, at most %d", c, (int)slots.size(), kMaxSlots);
-        for (int32_t p : slots) g->slot_param.push_back(p);
+        for (int32_t p : slots) {
+            g->slot_param.push_back(p);
+            slot_cell.push_back(c);
+        }
+        // (rows of coefficients are copied 16 bytes at a time)
+        cell_k0[c + 1] = cell_k0[c] + (int32_t)((3 * (nc + (n_gate - gbase_cell)) + 3) & ~(int64_t)3);
         cell_c0[c + 1] = b;
         cell_g0[c + 1] = (int32_t)n_gate;
         cell_ch0[c + 1] = (int32_t)ch_type.size();
@@ -993,13 +1245,22 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
         for (int i = m->phys_comp_off[c]; i < m->phys_comp_off[c + 1]; i++) cell_of[i] = c;
     std::vector<std::vector<int32_t>> rec_by_cell(nphys);
     for (int r = 0; r < s->n_rec; r++) rec_by_cell[cell_of[s->rec_comp[r]]].push_back(r);
-    std::vector<int32_t> rec_local, rec_col;
+    std::vector<int32_t> rec_local, rec_col, comp_rc0(m->n_comp, 0);
+    int max_rec = 0;
     for (int c = 0; c < nphys; c++) {
-        for (int32_t r : rec_by_cell[c]) {
-            rec_local.push_back(new_of[s->rec_comp[r]] - cell_c0[c]);
-            rec_col.push_back(r);
+        // by compartment, then column
+        std::stable_sort(rec_by_cell[c].begin(), rec_by_cell[c].end(),
+                         [&](int32_t x, int32_t y) { return new_of[s->rec_comp[x]] < new_of[s->rec_comp[y]]; });
+        size_t k = 0;
+        for (int gc = cell_c0[c]; gc < cell_c0[c + 1]; gc++) {
+            comp_rc0[gc] = (int32_t)rec_local.size();
+            for (; k < rec_by_cell[c].size() && new_of[s->rec_comp[rec_by_cell[c][k]]] == gc; k++) {
+                rec_local.push_back(gc - cell_c0[c]);
+                rec_col.push_back(rec_by_cell[c][k]);
+            }
         }
         cell_r0[c + 1] = (int32_t)rec_local.size();
+        max_rec = std::max(max_rec, (int)rec_by_cell[c].size());
     }
     // step times: the reference accumulates the float dt in double from 0
     // at step 1 and runs each step at that time as a float
@@ -1088,23 +1349,30 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     d.n_item = (int64_t)items.size();
     g->item_param = it_param;
     g->cell_ra_param = cell_ra_param;
-    // shared memory per warp
+    // launch shapes and shared memory
     const Dims &dm = g->dims;
     d.n_types = m->n_chan_types;
-    g->smem = (size_t)dm.slots * 32 * sizeof(double) + (size_t)m->n_chan_types * sizeof(EdenGpuChannelType) +
-              (size_t)(10 * dm.c + 2 * dm.g + 2 * dm.ch) * sizeof(float) +
-              (size_t)(4 * dm.c + 1 + 3 * dm.ch) * sizeof(int32_t);
+    g->fwd_cw = std::min(4, (dm.c + 31) / 32);
+    g->fwd_threads = 32 * (g->fwd_cw + std::min(kFwdWarps - g->fwd_cw, n_gate > 0 ? std::max(1, (dm.g + 31) / 32) : 0));
+    g->smem = (size_t)m->n_chan_types * sizeof(EdenGpuChannelType) +
+              (size_t)(9 * dm.c + 10 * kBlock + 2 * dm.g + 2 * dm.ch) * sizeof(float) +
+              (size_t)(4 * dm.c + 1 + 2 * dm.ch + dm.g) * sizeof(int32_t);
     int optin = 0;
     GTRY(g, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device));
-    if (g->smem > (size_t)optin)
+    g->stage = ((3 * (dm.c + dm.g) + 3) / 4 * 4 + max_rec + 3) / 4 * 4;
+    const size_t adj = ((size_t)6 * dm.c + 2 + dm.g) * sizeof(float);
+    g->adj_threads = std::min(256, std::max(64, (dm.c + 31) / 32 * 32));
+    g->ring = kRing;
+    while (g->ring > 1 && adj + sizeof(float) * g->ring * (size_t)g->stage > (size_t)(g->ring > 2 ? 100 * 1024 : optin)) g->ring /= 2;
+    g->smem_adj = adj + sizeof(float) * g->ring * (size_t)g->stage;
+    if (std::max(g->smem, g->smem_adj) > (size_t)optin)
         return g->fail(EDEN_GPU_E_INVALID, "largest cell (%d compartments, %d gates) needs %zu bytes of shared memory, "
-                                           "the device allows %d", dm.c, dm.g, g->smem, optin);
-    if (g->smem > 48 * 1024) {
-        // (the limit belongs to the kernels, which every context launches: the
-        // device's own, so that no context lowers another's)
-        GTRY(g, cudaFuncSetAttribute(k_grad_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-        GTRY(g, cudaFuncSetAttribute(k_grad_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    }
+                                           "the device allows %d", dm.c, dm.g, std::max(g->smem, g->smem_adj), optin);
+    // (the limit belongs to the kernels, which every context launches: the
+    // device's own, so that no context lowers another's)
+    GTRY(g, cudaFuncSetAttribute(k_grad_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    GTRY(g, cudaFuncSetAttribute(k_grad_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    GTRY(g, cudaFuncSetAttribute(k_grad_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     std::vector<EdenGpuChannelType> types(m->chan_types, m->chan_types + m->n_chan_types);
     int rc;
 #define UP(dst, src) \
@@ -1119,7 +1387,8 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     UP(rec_local, rec_local); UP(rec_col, rec_col); UP(tk, tk);
     UP(comp_gr0, comp_gr0); UP(gr_kind, gr_kind); UP(gr_it0, gr_it0); UP(it_grp, it_grp); UP(it_type, it_type);
     UP(it_param, it_param); UP(it_ev, it_ev); UP(it_ev0, it_ev0); UP(gr_erev, gr_erev); UP(it_w, it_w);
-    UP(syn, syn);
+    UP(syn, syn); UP(cell_k0, cell_k0); UP(comp_cell, comp_cell); UP(gate_map, gate_map); UP(comp_g0, comp_g0);
+    UP(comp_rc0, comp_rc0);
 #undef UP
     if (d.n_grp > 0) {
         const size_t rows = (size_t)(d.N + 1) * d.n_grp;
@@ -1129,6 +1398,8 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
         if ((rc = alloc(g, &d.it_b, (size_t)d.n_item)) != 0) return rc;
         if ((rc = alloc(g, &d.it_cur, (size_t)d.n_item)) != 0) return rc;
         if ((rc = alloc(g, &d.item_grad, (size_t)d.n_item)) != 0) return rc;
+        g->ex_rows = std::max<int64_t>(1, std::min<int64_t>(d.N, kExposureBytes / (4 * d.n_item)));
+        if ((rc = alloc(g, &d.ex, (size_t)g->ex_rows * d.n_item)) != 0) return rc;
         GTRY(g, cudaMemset(d.gbar, 0, rows * sizeof(float)));
     }
     const int64_t n_ck = d.N >= 2 ? (d.N - 2) / d.S + 1 : 1;
@@ -1136,8 +1407,27 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     d.params = g->d_params;
     if ((rc = alloc(g, &d.ck_v, (size_t)n_ck * m->n_comp)) != 0) return rc;
     if ((rc = alloc(g, &d.ck_q, (size_t)n_ck * n_gate)) != 0) return rc;
-    if ((rc = alloc(g, &d.tr_v, (size_t)(d.S + 1) * m->n_comp)) != 0) return rc;
-    if ((rc = alloc(g, &d.tr_q, (size_t)(d.S + 1) * n_gate)) != 0) return rc;
+    // the trajectory: of the whole run where it fits, else of as many segments
+    const int64_t tr_row = 4 * (2 * (int64_t)m->n_comp + n_gate);
+    g->keep = d.N * tr_row <= kTrajectoryBytes;
+    g->seg_group = g->keep ? n_ck : std::max<int64_t>(1, std::min<int64_t>({n_ck, 65535, kTrajectoryBytes / tr_row / d.S}));
+    const int64_t tr_rows = g->keep ? d.N : std::min<int64_t>(d.N, g->seg_group * d.S + 1);
+    if ((rc = alloc(g, &d.tr_v, (size_t)tr_rows * m->n_comp)) != 0) return rc;
+    if ((rc = alloc(g, &d.tr_q, (size_t)tr_rows * n_gate)) != 0) return rc;
+    if ((rc = alloc(g, &d.tr_d, (size_t)tr_rows * m->n_comp)) != 0) return rc;
+    d.co_len = cell_k0[nphys];
+    g->co_rows = std::max<int64_t>(1, std::min<int64_t>({tr_rows, kCoefBytes / (4 * ((int64_t)d.co_len + m->n_comp)), 1 << 20}));
+    if ((rc = alloc(g, &d.co, (size_t)g->co_rows * d.co_len)) != 0) return rc;
+    if ((rc = alloc(g, &d.mu, (size_t)g->co_rows * m->n_comp)) != 0) return rc;
+    if ((rc = alloc(g, &d.lv, (size_t)m->n_comp)) != 0) return rc;
+    if ((rc = alloc(g, &d.lq, (size_t)n_gate)) != 0) return rc;
+    d.n_part = (int32_t)((g->co_rows + kSumSteps - 1) / kSumSteps);
+    if ((rc = alloc(g, &d.part, g->slot_param.size() * (size_t)d.n_part)) != 0) return rc;
+    {
+        const int32_t *p = nullptr;
+        if ((rc = upload(g, &p, slot_cell)) != 0) return rc;
+        g->d_slot_cell = const_cast<int32_t *>(p);
+    }
     if ((rc = alloc(g, &g->d_trace, (size_t)d.N * std::max(s->n_rec, 1))) != 0) return rc;
     d.trace = g->d_trace;
     if ((rc = alloc(g, &g->d_tgrad, (size_t)d.N * std::max(s->n_rec, 1))) != 0) return rc;
@@ -1194,8 +1484,14 @@ extern "C" int edenGpuGradForward(EdenGpuGrad *g, const float *params, float *tr
     GTRY(g, cudaMemcpyAsync(g->d_params, g->h_params.data(), sizeof(float) * g->h_params.size(), cudaMemcpyHostToDevice,
                             g->stream));
     GTRY(g, cudaEventRecord(g->e0, g->stream));
-    if (g->d.n_grp > 0) k_grad_drive<<<(g->d.n_grp + 127) / 128, 128, 0, g->stream>>>(g->d);
-    k_grad_forward<<<g->n_cells, 32, g->smem, g->stream>>>(g->d, g->dims);
+    if (g->d.n_grp > 0)
+        for (int64_t n0 = 1; n0 <= g->d.N; n0 += g->ex_rows) {
+            const int64_t rows = std::min<int64_t>(g->ex_rows, g->d.N + 1 - n0);
+            k_grad_expose<<<(unsigned)((g->d.n_item + 127) / 128), 128, 0, g->stream>>>(g->d, n0, rows);
+            k_grad_drive<<<(unsigned)((rows * g->d.n_grp + 127) / 128), 128, 0, g->stream>>>(g->d, n0, rows);
+        }
+    g->d.tr_n0 = 1;
+    k_grad_forward<false><<<g->n_cells, g->fwd_threads, g->smem, g->stream>>>(g->d, g->dims, g->fwd_cw, 0, g->keep ? 1 : 0);
     GTRY(g, cudaGetLastError());
     GTRY(g, cudaEventRecord(g->e1, g->stream));
     if (trace && g->n_rec > 0)
@@ -1219,8 +1515,42 @@ extern "C" int edenGpuGradBackward(EdenGpuGrad *g, const float *trace_grad, floa
         GTRY(g, cudaMemcpyAsync(g->d_tgrad, trace_grad, sizeof(float) * (size_t)g->d.N * g->n_rec, cudaMemcpyDefault,
                                 g->stream));
     GTRY(g, cudaEventRecord(g->e0, g->stream));
-    k_grad_backward<<<g->n_cells, 32, g->smem, g->stream>>>(g->d, g->dims);
-    if (g->d.n_item > 0) k_grad_weights<<<(unsigned)((g->d.n_item + 127) / 128), 128, 0, g->stream>>>(g->d);
+    GradDev &d = g->d;
+    const int n_slot = (int)g->slot_param.size();
+    GTRY(g, cudaMemsetAsync(d.lv, 0, sizeof(float) * d.n_comp, g->stream));
+    GTRY(g, cudaMemsetAsync(d.lq, 0, sizeof(float) * std::max<int64_t>(d.n_gate, 1), g->stream));
+    GTRY(g, cudaMemsetAsync(g->d_slot, 0, sizeof(double) * std::max(n_slot, 1), g->stream));
+    // groups of segments, the last first; in each, blocks of steps, the last first
+    bool last = true;
+    for (int64_t hi = d.N >= 2 ? (d.N - 2) / d.S + 1 : 0; hi > 0;) {
+        const int64_t lo = std::max<int64_t>(0, hi - g->seg_group);
+        const int64_t n0 = 1 + lo * d.S, n1 = std::min<int64_t>(1 + hi * d.S, d.N);
+        d.tr_n0 = g->keep ? 1 : n0;
+        if (!g->keep)
+            k_grad_forward<true><<<dim3(g->n_cells, (unsigned)(hi - lo)), g->fwd_threads, g->smem, g->stream>>>(
+                d, g->dims, g->fwd_cw, lo, 1);
+        for (int64_t b = n1; b > n0;) {
+            const int64_t a = std::max<int64_t>(n0, b - g->co_rows), rows = b - a;
+            const int chunks = (int)((rows + kSumSteps - 1) / kSumSteps);
+            d.co_n0 = a;
+            k_grad_coef<<<(unsigned)((rows * d.n_comp + 127) / 128), 128, 0, g->stream>>>(d, rows);
+            k_grad_adjoint<<<g->n_cells, g->adj_threads, g->smem_adj, g->stream>>>(d, g->dims, rows, g->ring, g->stage, last ? 1 : 0);
+            k_grad_terms<<<dim3(g->n_cells, chunks), 64, (size_t)64 * g->dims.slots * sizeof(double), g->stream>>>(d, rows);
+            if (n_slot > 0)
+                k_grad_sum<<<(n_slot + 127) / 128, 128, 0, g->stream>>>(d, n_slot, g->d_slot_cell, chunks, a == 1 ? 1 : 0);
+            last = false;
+            b = a;
+        }
+        hi = lo;
+    }
+    if (d.n_item > 0)
+        for (int64_t n0 = 1; n0 <= d.N; n0 += g->ex_rows) {
+            const int64_t rows = std::min<int64_t>(g->ex_rows, d.N + 1 - n0);
+            // (the forward's exposures are still there where one block holds them all)
+            if (g->ex_rows < d.N)
+                k_grad_expose<<<(unsigned)((d.n_item + 127) / 128), 128, 0, g->stream>>>(d, n0, rows);
+            k_grad_weights<<<(unsigned)((d.n_item * 32 + 127) / 128), 128, 0, g->stream>>>(d, n0, rows);
+        }
     GTRY(g, cudaGetLastError());
     GTRY(g, cudaEventRecord(g->e1, g->stream));
     std::vector<double> slots(g->slot_param.size()), items((size_t)g->d.n_item);

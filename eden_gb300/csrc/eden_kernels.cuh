@@ -1299,7 +1299,7 @@ __device__ __forceinline__ void hines_forest(const DevModel &m, bool init, int64
                     }
                     X[j] = xj;
                 }
-                D[j] = __fdividef(1.0f, dj);
+                D[j] = pivot(dj);
             }
             __syncwarp();
         }
@@ -1449,7 +1449,7 @@ __device__ __forceinline__ void hines_window(float dt, float *S, float2 *XR, flo
                 dj = fmaf(-k.y, CN[q].y, dj);
                 x = fmaf(-k.y, k.x, x);
             }
-            const float inv = nonflat ? __fdividef(1.0f, dj) : c.z;
+            const float inv = nonflat ? pivot(dj) : c.z;
             if (d & kPassRoot) x = x * inv;
             if (on && nonflat) { CN[j].z = inv; XR[j].y = c.x * inv; }
         } else {

@@ -49,6 +49,16 @@ __device__ __forceinline__ float div_known(float x, float y, float r) {
     const float q = x * r;
     return fmaf(fmaf(-q, y, x), r, q);
 }
+// 1 / x for the cable solve's pivots, x = 1 + dt (...): one instruction.  It is
+// __fdividef(1, x) without that one's handling of subnormal operands, which the
+// solve's chain would wait for (29 cycles a node of a cable with it out); over
+// all 2^32 operands the two differ for subnormal ones only.
+__device__ __forceinline__ float pivot(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // RN(1 / y) for div_known, 0 where it has to divide
 __host__ __device__ __forceinline__ float known_reciprocal(float y) {
     const float a = y < 0.0f ? -y : y;

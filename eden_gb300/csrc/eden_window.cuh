@@ -309,7 +309,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             float x = init ? v : v + div_known(dt * (I + (v * G)), C, rC);
             if (!f64) {
                 d = 1.0f + d * dt;
-                if ((slot & kSlotDone) && !init) x = x * __fdividef(1.0f, d);
+                if ((slot & kSlotDone) && !init) x = x * pivot(d);
             }
             CN[ti].z = d;
             XR[ti].x = x;
