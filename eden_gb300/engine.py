@@ -195,24 +195,28 @@ class Simulation:
     def fetch(self) -> Records:
         cap = self.record_capacity_steps
         nt = max(len(self.trace_target), 1)
-        trace = np.zeros((cap, nt), np.float32)
-        tstep = np.zeros(cap, np.int64)
-        ssrc = np.zeros(self.spike_capacity, np.int32)
-        sstep = np.zeros(self.spike_capacity, np.int64)
-        stime = np.zeros(self.spike_capacity, np.float64)
+        trace = np.empty((cap, nt), np.float32)
+        tstep = np.empty(cap, np.int64)
         rec = CRecords()
         rec.trace = trace.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
         rec.trace_step = tstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
         rec.trace_capacity = cap
-        rec.spike_src = ssrc.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
-        rec.spike_step = sstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
-        rec.spike_capacity = self.spike_capacity
-        rec.spike_time_us = stime.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
-        self._check(self.lib.edenGpuFetchRecords(self.ctx, ctypes.byref(rec)))
+        # room for as many spikes as there are: a small buffer first, and, where
+        # the call says that it takes more, that many
+        room = min(4096, self.spike_capacity)
+        while True:
+            ssrc, sstep, stime = np.empty(room, np.int32), np.empty(room, np.int64), np.empty(room, np.float64)
+            rec.spike_src = ssrc.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
+            rec.spike_step = sstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+            rec.spike_capacity = room
+            rec.spike_time_us = stime.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+            rc = self.lib.edenGpuFetchRecords(self.ctx, ctypes.byref(rec))
+            if rc == 0 or not room < rec.n_spikes <= self.spike_capacity:
+                break
+            room = int(rec.n_spikes)
+        self._check(rc)
         n, m = int(rec.n_trace_samples), int(rec.n_spikes)
-        order = np.lexsort((ssrc[:m], sstep[:m]))
-        return Records(trace[:n, :len(self.trace_target)].copy(), tstep[:n].copy(),
-                       ssrc[:m][order].copy(), sstep[:m][order].copy(), stime[:m][order].copy())
+        return Records(trace[:n, :len(self.trace_target)], tstep[:n], ssrc[:m], sstep[:m], stime[:m])
 
     def run(self, n_steps: int | None = None, chunk: int | None = None) -> Records:
         """Initialise, then run n_steps non-initialisation steps (default: the
@@ -265,7 +269,7 @@ class Simulation:
 
     # -- state access ----------------------------------------------------------
     def read_v(self) -> np.ndarray:
-        v = np.zeros(self.n_target, np.float32)
+        v = np.empty(self.n_target, np.float32)
         self._check(self.lib.edenGpuReadV(self.ctx, _ptr(v), ctypes.c_int64(self.n_target)))
         return v
 

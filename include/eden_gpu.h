@@ -364,7 +364,8 @@ enum {
     EDEN_KERNEL_KINDS = 5
 };
 
-/* Records produced since the previous fetch, in step order. */
+/* Records produced since the previous fetch, in step order (spikes of one step
+ * by source). */
 typedef struct EdenGpuRecords {
     /* caller-provided host buffers and their capacities */
     float *trace;             /* [trace_capacity * n_trace], sample-major */
@@ -373,7 +374,8 @@ typedef struct EdenGpuRecords {
     int32_t *spike_src;       /* [spike_capacity] */
     int64_t *spike_step;      /* [spike_capacity] step at which the spike is logged */
     int64_t spike_capacity;
-    /* filled in */
+    /* filled in; where a buffer is too small (EDEN_GPU_E_RANGE), what it takes:
+     * nothing is fetched then, and the call can be made again */
     int64_t n_trace_samples;
     int64_t n_spikes;
     /* optional (NULL: not copied), [spike_capacity]: each spike's
