@@ -112,7 +112,7 @@ struct EdenGpuCtx {
     int max_cell_blocks = 0;               // most blocks of a k_cells_t launch
     int cell_threads = 128;                // threads of a k_cells_t block
     std::vector<int64_t> h_ext_step;       // logging steps of the spike sources' events
-    size_t smem_hines = 0;
+    size_t smem_hines = 0, smem_inputs = 0;
     struct CellClass { int cta_begin, cta_end; size_t smem; };
     std::vector<CellClass> classes;        // k_cells_t launches of one window
     double last_ms = 0.0;
@@ -1267,17 +1267,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         ck_info[c] = (bk_kind[ck_blk[c]] == BK_CLAMPV ? BK_PULSE : (bk_kind[ck_blk[c]] & BK_KIND_MASK)) |
                      ((int32_t)bk_type[ck_blk[c]] << 2) | (ck_n[c] << 8);
 
-    // each block's record in the windowed kernel, its chunks counted in its unit
-    std::vector<int4> bk_rec(n_block);
-    for (size_t u = 0; u < un_t0.size(); u++) {
-        const int b0 = t_blk0[un_t0[u]], b1 = t_blk0[un_t1[u]];
-        for (int b = b0; b < b1; b++) {
-            int32_t e;
-            memcpy(&e, &bk_erev[b], 4);
-            bk_rec[b] = make_int4(bk_c0[b] - bk_c0[b0], bk_c0[b + 1] - bk_c0[b0], bk_kind[b], e);
-        }
-    }
-
     // ---- window length: every delay must cover the window (see k_window)
     int kmax = kMaxWindow;
     if (ns > 0) {
@@ -1291,6 +1280,22 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     ctx->kernel_timing = opt && opt->kernel_timing;
     int kreq = (opt && opt->steps_per_launch > 0) ? opt->steps_per_launch : kmax;
     ctx->K = ctx->mode == EDEN_MODE_BATCHED ? std::max(1, std::min(kreq, kmax)) : 1;
+    // a chunk's series: the longest window's steps (the four initialisation
+    // passes may be one), in whole 16-byte words
+    ctx->d.gp_stride = ctx->mode == EDEN_MODE_BATCHED ? (std::max(ctx->K, 4) + 3) & ~3 : 1;
+    ctx->d.acc_stride = (ctx->mode == EDEN_MODE_BATCHED ? std::max(ctx->K, 4) : 1) | 1;
+    ctx->smem_inputs = (size_t)kInputThreads / 32 * 64 * ctx->d.acc_stride * sizeof(float);
+    // each block's record in the windowed kernel
+    std::vector<int4> bk_rec(n_block);
+    for (size_t u = 0; u < un_t0.size(); u++) {
+        const int b0 = t_blk0[un_t0[u]], b1 = t_blk0[un_t1[u]];
+        for (int b = b0; b < b1; b++) {
+            int32_t e;
+            memcpy(&e, &bk_erev[b], 4);
+            bk_rec[b] = make_int4((bk_c0[b] - bk_c0[b0]) * ctx->d.gp_stride, (bk_c0[b + 1] - bk_c0[b0]) * ctx->d.gp_stride,
+                                  bk_kind[b], e);
+        }
+    }
 
     // ---- recording
     // each column on its target's list, with the internal gate slot it
@@ -1430,7 +1435,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             const int nck = bk_c0[t_blk0[b]] - bk_c0[t_blk0[a]];
             const int f = un_f[u];
             un_words[u] = forest_words(fo_n0[f + 1] - fo_n0[f], fo_w0[f + 1] - fo_w0[f], un_nf1[u] - un_nf0[u], un_ch1[u] - un_ch0[u], un_ngt[u],
-                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, nck, std::max(ctx->K, 4),
+                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, nck, ctx->d.gp_stride,
                                        fo_f64[un_f[u]] != 0);
         } else {
             un_words[u] = izh_words(b - a);
@@ -1623,7 +1628,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload_c(ctx, &d.bk_c0, bk_c0)); TRY(upload_c(ctx, &d.ck_blk, ck_blk));
     TRY(upload_c(ctx, &d.ck_i0, ck_i0)); TRY(upload_c(ctx, &d.ck_n, ck_n));
     TRY(upload_c(ctx, &d.ck_info, ck_info));
-    TRY(upload(ctx, &d.Gp, (const float *)nullptr, (size_t)32 * (size_t)std::max(n_chunk, 1)));
+    TRY(upload(ctx, &d.Gp, (const float *)nullptr, (size_t)d.gp_stride * (size_t)std::max(n_chunk, 1)));
     TRY(upload(ctx, &d.ck_a, (const float *)nullptr, (size_t)std::max(n_chunk, 1)));
     TRY(upload(ctx, &d.ck_b, (const float *)nullptr, (size_t)std::max(n_chunk, 1)));
     TRY(upload_c(ctx, &d.c_chan0, c_chan0)); TRY(upload_c(ctx, &d.ch_type, ch_type));
@@ -1862,7 +1867,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     {
         // resident input blocks only: each warp then walks several chunks
         int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ctx->fn_inputs, kInputThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ctx->fn_inputs, kInputThreads, ctx->smem_inputs);
         ctx->grid_inputs = (int)std::max<int64_t>(
             1, std::min<int64_t>(((int64_t)ctx->d.n_chunk * 32 + kInputThreads - 1) / kInputThreads,
                                  (int64_t)ctx->n_sm * std::max(per_sm, 1)));
@@ -1873,7 +1878,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         int occ_cells = 0, occ_inputs = 0;
         if (ctx->smem_window)
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cells, ctx->fn_cells, ctx->cell_threads, max_smem_class);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_inputs, ctx->fn_inputs, kInputThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_inputs, ctx->fn_inputs, kInputThreads, ctx->smem_inputs);
         fprintf(stderr, "libeden_gpu: kernels %s%s%s (%.0f ms)\n",
                 ctx->codegen_used ? "compiled for this model" : "built in",
                 ctx->codegen_note.empty() ? "" : ": ", ctx->codegen_note.c_str(), ctx->codegen_ms);
@@ -2052,7 +2057,7 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
     cudaStream_t s = ctx->stream;
     if (ctx->mode == EDEN_MODE_BATCHED && ctx->smem_window) {
         tmark(ctx, EDEN_KERNEL_INPUTS, true);
-        launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab,
+        launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d, (const WindowArgs *)ctx->d_wtab,
                  (const WindowTimes *)ctx->d_wtimes, base, idx);
         tmark(ctx, EDEN_KERNEL_INPUTS, false);
         int n = 1;
@@ -2071,7 +2076,7 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
     }
     (void)K;
     tmark(ctx, EDEN_KERNEL_INPUTS, true);
-    launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab,
+    launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d, (const WindowArgs *)ctx->d_wtab,
              (const WindowTimes *)ctx->d_wtimes, base, idx);
     tmark(ctx, EDEN_KERNEL_INPUTS, false);
     tmark(ctx, EDEN_KERNEL_TARGETS, true);
@@ -2481,8 +2486,8 @@ extern "C" int edenGpuReadSynapses(EdenGpuCtx *ctx, float *pending_us, float *st
 // host loop that must not stall on cudaMalloc/cudaFree (both can synchronise
 // the whole device), cannot accept that.  This entry point runs the same
 // kernels in the same order as edenGpuRun, with
-//   - the input kernel's per-window conductance scratch (32 rows of n_chunk
-//     floats) in the file-scope array g_static_gp instead of the context's
+//   - the input kernel's per-window conductance scratch (gp_stride, at
+//     most 32, floats a chunk) in the file-scope array g_static_gp instead of the context's
 //     buffer, which limits it to models of at most kStaticGpChunks input
 //     chunks (16 MiB of scratch); larger models get EDEN_GPU_E_RANGE;
 //   - the window arguments and step times in the file-scope tables
@@ -2495,8 +2500,8 @@ extern "C" int edenGpuReadSynapses(EdenGpuCtx *ctx, float *pending_us, float *st
 // does only it.  The arrays belong to the library's module: every device
 // that loads it holds them (16 MiB and a few KB) until the process exits,
 // whether or not this entry point is ever called.
-// Nothing in either array has to start at zero: every window writes rows
-// 0..K-1 of every chunk before the cell kernels read them, and each launch
+// Nothing in either array has to start at zero: every window writes steps
+// 0..K-1 of every chunk before the cell kernels use them, and each launch
 // reads only table entries written by the copy before it.
 // The arrays exist once per device, not per context: calls that overlap in
 // time on one device (two threads, or two contexts on different streams)
@@ -2539,7 +2544,7 @@ static int launch_window_static(EdenGpuCtx *ctx, const DevModel &dm, const Windo
     cudaStream_t s = ctx->stream;
     const int *zero = ctx->d_zero;
     if (ctx->mode == EDEN_MODE_BATCHED && ctx->smem_window) {
-        launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, 0, s, dm, tab, times, zero, idx);
+        launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, dm, tab, times, zero, idx);
         int n = 1;
         for (const auto &cl : ctx->classes) {
             const int nb = std::min(cl.cta_end - cl.cta_begin, ctx->max_cell_blocks);
@@ -2550,7 +2555,7 @@ static int launch_window_static(EdenGpuCtx *ctx, const DevModel &dm, const Windo
         launch_k(ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, dm, tab, zero, idx);
         return n + 1;
     }
-    launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, 0, s, dm, tab, times, zero, idx);
+    launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, dm, tab, times, zero, idx);
     k_targets_t<<<ctx->grid_targets, kThreads, 0, s>>>(dm, tab, times, zero, idx);
     k_hines_t<<<ctx->grid_hines, kHinesThreads, ctx->smem_hines, s>>>(dm, tab, zero, idx, ctx->forest_cap);
     launch_k(ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, dm, tab, zero, idx);

@@ -165,7 +165,7 @@ struct DevModel {
     const float *bk_erev;
     const int32_t *in_tgt;            // targets with any block
     // blocks are cut into chunks of at most kChunkItems items, one warp each; step k's
-    // partial sum of chunk c is Gp[k * n_chunk + c] and a block's value is the
+    // partial sum of chunk c is Gp[c * gp_stride + k] and a block's value is the
     // sum of its chunks' partials in chunk order
     int32_t n_chunk;
     const int32_t *bk_c0;             // [n_block + 1] chunk range of each block
@@ -173,7 +173,9 @@ struct DevModel {
     const int32_t *ck_info;           // kind | synapse type << 2 | items << 8
     const int64_t *ck_i0;             // first item of each chunk
     const int32_t *ck_n;              // items in the chunk
-    float *Gp;                        // [32 * n_chunk]
+    float *Gp;                        // [n_chunk * gp_stride]
+    int32_t gp_stride;                // steps of the longest window, a multiple of four (1: per-step path)
+    int32_t acc_stride;               // of the input kernel's event tiles: odd, at least those steps
     const float *syn_pow;             // per synapse type: f_rise^j, then f_decay^j, j < kPowLen
     int32_t pois_exact;               // dt is a whole number of us: Poisson clocks advance exactly
     float *ck_a, *ck_b;               // aggregate synapse state of each chunk (weighted sums)
@@ -260,7 +262,8 @@ struct DevModel {
     // gate of a channel type, three 16-byte records (gate_next_p)
     const int32_t *gt_idx;
     const float4 *gate_tab;
-    // per input block: its chunks (counted in its unit), kind and reversal potential
+    // per input block: where its chunks begin and end in the unit's series
+    // (gp_stride each), kind and reversal potential
     const int4 *bk_rec;
     int32_t *status;
     // forests whose cells may lose diagonal dominance: their elimination runs
@@ -334,19 +337,19 @@ constexpr int kGateExtWords = 9;  // a non-rates gate's kind and timeCourse / st
 // one of zeros after them) and nw twig rows, what addresses refer to first:
 // pairs, V and elimination factor per node; two words per twig place, pre-updated V and V; then the 16-byte
 // records: one per node, one per twig place, two per non-flat compartment, one
-// per input block; then pairs: threshold and source per non-flat compartment;
-// then words: a twig place's addresses, V at the step's start per non-flat
-// compartment, four per channel of these, three per gate (its index word, its
-// value in alternate steps), the passes, and the window's conductance series of
-// the unit's input chunks (kcap steps).  A batch of izhikevich neurons: V twice
-// and 19 parameter / state words per neuron.
+// per input block, and the window's conductance series of the unit's input
+// chunks (gps words each); then pairs: threshold and source per non-flat
+// compartment; then words: a twig place's addresses, V at the step's start per
+// non-flat compartment, four per channel of these, three per gate (its index
+// word, its value in alternate steps), and the passes.  A batch of izhikevich
+// neurons: V twice and 19 parameter / state words per neuron.
 __host__ __device__ inline int twig_words(int n) { return (2 * n + 3) & ~3; }  // where the twigs' words start
-__host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int nck, int kcap,
+__host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int nck, int gps,
                                             bool f64 = false) {
     // a double-precision forest adds its eliminated values, pivots and
     // factors in double (6 words per compartment, 8-byte aligned)
-    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + 2 * nf + 32 * nw + nf +
-                  4 * nfch + 3 * ngt + np + kcap * nck + (f64 ? 6 * n + 2 : 0);
+    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + gps * nck + 2 * nf +
+                  32 * nw + nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
     return (w + 3) & ~3;
 }
 __host__ __device__ inline int izh_words(int n) { return ((2 + EDEN_POINT_PARAMS + 3) * n + 3) & ~3; }
@@ -444,8 +447,8 @@ __device__ __forceinline__ bool trigger_arrival(float t, float dt, float delay, 
 // is at least Kprev * dt, so none of these spikes can fall due before step0.
 __device__ __forceinline__ bool replay_mask(uint32_t mask, const WindowArgs &w, const float *tprev, float dt,
                                             float delay, float &pend) {
-    for (int b = 1; b < w.Kprev; b++)
-        if ((mask >> b) & 1u) trigger_arrival(tprev[b], dt, delay, pend);
+    for (uint32_t r = mask & ((1u << w.Kprev) - 1) & ~1u; r; r &= r - 1)
+        trigger_arrival(tprev[__ffs(r) - 1], dt, delay, pend);
     return (mask >> w.Kprev) & 1u;
 }
 
@@ -472,37 +475,57 @@ __device__ __forceinline__ float decayed(float a, float f, const float *fpow, in
 }
 
 // The contribution (dA, dB) of one synapse's event at step s to its chunk's
-// aggregate, and the synapse's own state after it.
-template <int KIND>
+// aggregate, and the synapse's own state after it.  Roundings are written out:
+// they do not depend on what the code around is contracted to.
+template <int KIND, bool SYN = false>
 __device__ __forceinline__ void input_event(const SynTypeDev &st, const float *pw, float dt, float w, int64_t s,
                                             float &a, float &b, int32_t &last, float &dA, float &dB, float js = 1.0f) {
     const int n = (int)(s - (int64_t)last) - 1;
     if (KIND == EDEN_SYN_EXPTWO) {
-        // (js: a blockingPlasticSynapse's plasticity factor for this event)
-        const float jump = st.wf_w * js;
+        // (js: a blockingPlasticSynapse's plasticity factor for this event, 1 for other connections)
+        const float jump = SYN ? st.wf_w * js : st.wf_w;
         const float ai = decayed(a, st.f_rise, pw, n), bi = decayed(b, st.f_decay, pw + kPowLen, n);
-        dA = w * (dt * div_by_tau(ai, st.tau_rise, st.r_rise) + jump);
-        dB = w * (dt * div_by_tau(bi, st.tau_decay, st.r_decay) + jump);
+        const float da = div_by_tau(ai, st.tau_rise, st.r_rise), db = div_by_tau(bi, st.tau_decay, st.r_decay);
+        dA = __fmul_rn(w, SYN ? fmaf(st.wf_w, js, __fmul_rn(dt, da)) : fmaf(dt, da, jump));
+        dB = __fmul_rn(w, SYN ? fmaf(st.wf_w, js, __fmul_rn(dt, db)) : fmaf(dt, db, jump));
         a = ai + jump;
         b = bi + jump;
     } else {
         const float gi = decayed(a, st.f_decay, pw + kPowLen, n);
-        dA = w * (dt * div_by_tau(gi, st.tau_decay, st.r_decay) + st.gbase);
+        dA = __fmul_rn(w, fmaf(dt, div_by_tau(gi, st.tau_decay, st.r_decay), st.gbase));
         dB = 0.0f;
         a = gi + st.gbase;
     }
     last = (int32_t)s;
 }
 
-// Adds an event at window step j to the lane's rows of the event tiles,
-// clearing the rows on the lane's first event of the window.
-__device__ __forceinline__ void put_event(float *rowA, float *rowB, bool &used, int K, int j, float dA, float dB) {
-    if (!used) {
-        for (int q = 0; q < K; q++) { rowA[q] = 0.0f; rowB[q] = 0.0f; }
-        used = true;
+// An item's events in the window: the first in registers, the others (an item
+// has more than one only where it fires again within the window) in its rows
+// of the tiles.
+struct ItemEvents {
+    int n, j;
+    float dA, dB;
+};
+
+// Adds an event at window step j, each in a step of its own.
+template <int KIND>
+__device__ __forceinline__ void put_event(float *rowA, float *rowB, ItemEvents &ev, int K, int j, float dA, float dB) {
+    if (ev.n == 0) {
+        ev.n = 1;
+        ev.j = j;
+        ev.dA = dA;
+        ev.dB = dB;
+        return;
     }
-    rowA[j] += dA;
-    rowB[j] += dB;
+    if (ev.n == 1) {
+        ev.n = 2;
+        for (int q = 0; q < K; q++) {
+            rowA[q] = 0.0f;
+            if (KIND == EDEN_SYN_EXPTWO) rowB[q] = 0.0f;
+        }
+    }
+    rowA[j] = __fadd_rn(rowA[j], dA);
+    if (KIND == EDEN_SYN_EXPTWO) rowB[j] = __fadd_rn(rowB[j], dB);
 }
 
 // Poisson input `it` over the K steps of a window (poissonFiringSynapse,
@@ -518,21 +541,21 @@ __device__ __forceinline__ float pois_draw(const DevModel &m, int64_t it, int64_
 }
 
 template <int KIND>
-__device__ __forceinline__ void pois_fire(const DevModel &m, int64_t it, const SynTypeDev &st, int64_t s, int j, int K,
-                                          float *rowA, float *rowB, bool &used) {
+__device__ __forceinline__ void pois_fire(const DevModel &m, int64_t it, const SynTypeDev &st, const float *pw, int64_t s,
+                                          int j, int K, float *rowA, float *rowB, ItemEvents &ev) {
     float a = m.po_a[it], b = KIND == EDEN_SYN_EXPTWO ? m.po_b[it] : 0.0f;
     int32_t last = m.po_last[it];
     float dA, dB;
-    input_event<KIND>(st, m.syn_pow + (size_t)m.po_type[it] * 2 * kPowLen, m.dt, m.po_w[it], s, a, b, last, dA, dB);
+    input_event<KIND>(st, pw, m.dt, m.po_w[it], s, a, b, last, dA, dB);
     m.po_a[it] = a;
     if (KIND == EDEN_SYN_EXPTWO) m.po_b[it] = b;
     m.po_last[it] = last;
-    put_event(rowA, rowB, used, K, j, dA, dB);
+    put_event<KIND>(rowA, rowB, ev, K, j, dA, dB);
 }
 
 template <int KIND>
 __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const WindowArgs &w, const SynTypeDev &st,
-                                            float ts, float isi, float *rowA, float *rowB, bool &used) {
+                                            const float *pw, float ts, float isi, float *rowA, float *rowB, ItemEvents &ev) {
     const float dt = m.dt;
     if (w.step0 <= 0) {
         for (int j = 0; j < w.K; j++) {
@@ -540,12 +563,7 @@ __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const
             isi = pois_draw(m, it, w.step0 + j, 0);
         }
     } else if (m.pois_exact && isi < 0x1p23f) {
-        // (exact sums: no firing in the window when even its last step's
-        // time since the spike stays within the interval)
-        if (ts + (float)(w.K - 1) * dt <= isi) {
-            m.po_ts[it] = ts + (float)w.K * dt;
-            return;
-        }
+        // (one that cannot fire in the window has been dealt with: chunk_window)
         int j = 0;
         while (true) {
             // first step from j on whose time since the last spike exceeds isi
@@ -561,7 +579,7 @@ __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const
             }
             j += jn;
             isi = pois_draw(m, it, w.step0 + j, 1);
-            pois_fire<KIND>(m, it, st, w.step0 + j, j, w.K, rowA, rowB, used);
+            pois_fire<KIND>(m, it, st, pw, w.step0 + j, j, w.K, rowA, rowB, ev);
             ts = 0.0f;
             j += 1;
             if (j >= w.K) break;
@@ -571,7 +589,7 @@ __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const
             if (ts > isi) {
                 ts = 0.0f;
                 isi = pois_draw(m, it, w.step0 + j, 1);
-                pois_fire<KIND>(m, it, st, w.step0 + j, j, w.K, rowA, rowB, used);
+                pois_fire<KIND>(m, it, st, pw, w.step0 + j, j, w.K, rowA, rowB, ev);
             } else {
                 ts = ts + dt * 1.0f;
             }
@@ -590,11 +608,22 @@ __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const
 // delay below dt.
 template <int KIND>
 __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const WindowArgs &w, const SynTypeDev &st,
-                                           const float *tk, float pend, uint32_t mask, float *rowA, float *rowB,
-                                           bool &used) {
-    if (w.step0 <= 0) return;  // no spikes reach a synapse during initialisation
+                                           const float *pw, const float *tk, float pend, uint32_t mask, float *rowA, float *rowB,
+                                           ItemEvents &ev) {
+    // (chunk_window leaves out initialisation: no spikes reach a synapse in it)
     const float dt = m.dt;
     const float pend0 = pend;
+    // a spike that is due, and so its state, is known before the replay: the
+    // loads overlap
+    const bool due = pend >= tk[0] && pend < tk[w.K - 1] + dt;
+    float a = 0.0f, b = 0.0f, wt = 0.0f;
+    int32_t last = 0;
+    if (due) {
+        a = m.sy_a[it];
+        if (KIND == EDEN_SYN_EXPTWO) b = m.sy_b[it];
+        last = m.sy_last[it];
+        wt = m.sy_w[it];
+    }
     bool trig = false;
     float delay = 0.0f;
     if (mask) {
@@ -602,19 +631,29 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
         delay = m.sy_delay[it];
         trig = replay_mask(mask, w, tk + 32, dt, delay, pend);
     }
+    // the first step j with pend < tk[j] + dt (these ends never fall), if its
+    // start is not past pend
     int jf = -1;
-    if (pend >= tk[0] && pend < tk[w.K - 1] + dt)
-        for (int j = 0; j < w.K; j++)
-            if (tk[j] <= pend && pend < tk[j] + dt) { jf = j; break; }
+    if (pend >= tk[0] && pend < tk[w.K - 1] + dt) {
+        int j = 0, e = w.K - 1;
+        while (j < e) {
+            const int h = (j + e) >> 1;
+            if (pend < tk[h] + dt) e = h;
+            else j = h + 1;
+        }
+        if (tk[j] <= pend) jf = j;
+    }
     bool now = false;
     if (trig) now = trigger_arrival(tk[0], dt, delay, pend);
     if (pend != pend0) m.sy_pend[it] = pend;
     if (jf < 0 && !now) return;
-    float a = m.sy_a[it], b = KIND == EDEN_SYN_EXPTWO ? m.sy_b[it] : 0.0f;
-    int32_t last = m.sy_last[it];
-    const float wt = m.sy_w[it];
+    if (!due) {
+        a = m.sy_a[it];
+        if (KIND == EDEN_SYN_EXPTWO) b = m.sy_b[it];
+        last = m.sy_last[it];
+        wt = m.sy_w[it];
+    }
     float dA, dB;
-    const float *pw = m.syn_pow + (size_t)m.sy_type[it] * 2 * kPowLen;
     // a blockingPlasticSynapse's Tsodyks-Markram state (LEMS_CoreComponents.inc.xml:
     // 263-312): forward Euler from the last event, 1 - R and U - p shrinking
     // by their factor each step; the event's jump scaled by R U before the
@@ -634,13 +673,13 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
     };
     if (now && jf != 0) {
         const float js = factor(w.step0);
-        input_event<KIND>(st, pw, dt, wt, w.step0, a, b, last, dA, dB, js);
-        put_event(rowA, rowB, used, w.K, 0, dA, dB);
+        input_event<KIND, true>(st, pw, dt, wt, w.step0, a, b, last, dA, dB, js);
+        put_event<KIND>(rowA, rowB, ev, w.K, 0, dA, dB);
     }
     if (jf >= 0) {
         const float js = factor(w.step0 + jf);
-        input_event<KIND>(st, pw, dt, wt, w.step0 + jf, a, b, last, dA, dB, js);
-        put_event(rowA, rowB, used, w.K, jf, dA, dB);
+        input_event<KIND, true>(st, pw, dt, wt, w.step0 + jf, a, b, last, dA, dB, js);
+        put_event<KIND>(rowA, rowB, ev, w.K, jf, dA, dB);
     }
     m.sy_a[it] = a;
     if (KIND == EDEN_SYN_EXPTWO) m.sy_b[it] = b;
@@ -674,20 +713,19 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
 // t + dt exceeds a listed time, the same step), which lowering has computed.
 template <int KIND>
 __device__ __forceinline__ void timed_window(const DevModel &m, int64_t it, const WindowArgs &w, const SynTypeDev &st,
-                                             float *rowA, float *rowB, bool &used) {
+                                             const float *pw, float *rowA, float *rowB, ItemEvents &ev) {
     int64_t c = m.tm_cur[it];
     const int64_t c1 = m.tm_off[it + 1];
     const int64_t end = w.step0 + w.K;
     if (c >= c1 || m.tm_step[c] >= end) return;
     float a = m.tm_a[it], b = KIND == EDEN_SYN_EXPTWO ? m.tm_b[it] : 0.0f;
     int32_t last = m.tm_last[it];
-    const float *pw = m.syn_pow + (size_t)m.tm_type[it] * 2 * kPowLen;
     for (; c < c1 && m.tm_step[c] < end; c++) {
         const int64_t s = m.tm_step[c];
         if (s < w.step0) continue;
         float dA, dB;
         input_event<KIND>(st, pw, m.dt, m.tm_w[it], s, a, b, last, dA, dB);
-        put_event(rowA, rowB, used, w.K, (int)(s - w.step0), dA, dB);
+        put_event<KIND>(rowA, rowB, ev, w.K, (int)(s - w.step0), dA, dB);
     }
     m.tm_a[it] = a;
     if (KIND == EDEN_SYN_EXPTWO) m.tm_b[it] = b;
@@ -695,10 +733,9 @@ __device__ __forceinline__ void timed_window(const DevModel &m, int64_t it, cons
     m.tm_cur[it] = c;
 }
 
-// Per-warp accumulation tiles: row `lane` (stride kAccStride, padded so that
+// Per-warp accumulation tiles: row `lane` (stride acc_stride, odd so that
 // both a row write and a column read are free of bank conflicts) holds the
 // lane's terms for each step of the window.
-constexpr int kAccStride = 33;
 
 // An alpha chunk's aggregate over the window (alphaSynapse: conductance g
 // and rise state A; alphaCurrentSynapse: current I and J).  Per step the
@@ -711,20 +748,15 @@ constexpr int kAccStride = 33;
 // events' part of A_j (a scan over the lanes, as for the other kinds) and
 // T_j = sum_{k<j} f^(j-1-k) S_k a second scan over S.  Lane j keeps the
 // exposure g_j of step j for Gp.
-__device__ __forceinline__ void alpha_chunk_window(const DevModel &m, int c, int type, const SynTypeDev &st,
-                                                   const WindowArgs &w, unsigned rows, float A, float B,
-                                                   const float *tileA) {
+__device__ __forceinline__ float alpha_chunk_window(const float *pd, const SynTypeDev &st, const WindowArgs &w,
+                                                    bool events, float ea, float &A, float &B) {
     const int lane = threadIdx.x & 31;
-    const float *pd = m.syn_pow + (size_t)type * 2 * kPowLen + kPowLen;
     const float cc = st.c_alpha;
     const float jf = (float)lane;
     // the parts from the window's starting state
     float gj = lane < w.K ? B * pd[lane] + (lane > 0 ? cc * (jf * pd[lane - 1]) * A : 0.0f) : 0.0f;
     float Ak = A * pd[w.K], Bk = B * pd[w.K] + cc * ((float)w.K * pd[w.K - 1]) * A;
-    if (rows != 0) {
-        float ea = 0.0f;  // lane j: the chunk's events of step j
-        if (lane < w.K)
-            for (unsigned r = rows; r; r &= r - 1) ea += tileA[(__ffs(r) - 1) * kAccStride + lane];
+    if (events) {  // (ea of lane j: the chunk's events of step j)
         // S: inclusive scan of the events with factor f, then exclusive
         float va = lane < w.K ? ea : 0.0f;
 #pragma unroll
@@ -747,25 +779,30 @@ __device__ __forceinline__ void alpha_chunk_window(const DevModel &m, int c, int
         Ak += __shfl_sync(0xffffffffu, va, w.K - 1);
         Bk += cc * __shfl_sync(0xffffffffu, vt, w.K - 1);
     }
-    if (lane < w.K) m.Gp[(size_t)lane * m.n_chunk + c] = gj;
-    if (lane == 0 && w.step0 > 0) { m.ck_a[c] = Ak; m.ck_b[c] = Bk; }
-    __syncwarp();
+    if (w.step0 > 0) { A = Ak; B = Bk; }
+    return gj;
 }
 
-// One chunk (at most kChunkItems items of one input block) over the K steps
-// of a window, lane l handling items l, l + 32, ...  Pulses add their
-// current to row l of tile A, and lane j sums column j in row order into
-// Gp[j][chunk].  Synapses and Poisson inputs add their events to the tiles;
-// lane j sums step j's events over the rows in row order, and every lane then
-// steps the chunk's aggregate state through the window, lane j keeping the
-// exposure of step j (the conductance before the step's update, as the
-// reference exposes it) for Gp[j][chunk].
-__device__ __forceinline__ void chunk_window(const DevModel &m, int c, int32_t info, int64_t ck_i0,
-                                             const WindowArgs &w, float *tileA, float *tileB, const float *tk) {
+// An item that may have an event in the window: its state, its chunk's place
+// in the warp's group, and its place in the chunk (at = chunk * kChunkItems + item).
+struct HotItem {
+    float s0, s1;
+    int at;
+};
+constexpr int kInputGroup = 16;                // chunks of a group, at most
+constexpr int kHotItems = kChunkItems + 32;    // items listed before they are worked off, at most
+
+// A chunk of pulses, clamps or generators (at most kChunkItems items of one
+// input block) over the K steps of a window: lane l adds the current of items
+// l, l + 32, ... to row l of the tile, and lane j sums column j in row order
+// into the chunk's series in Gp.
+__device__ __forceinline__ void pulse_chunk(const DevModel &m, int c, int32_t info, int64_t ck_i0, const WindowArgs &w,
+                                            float *tileA, const float *tk) {
     const int lane = threadIdx.x & 31;
     const int kind = info & 3;
     const int n = info >> 8;
-    float *rowA = tileA + lane * kAccStride, *rowB = tileB + lane * kAccStride;
+    const int kAccStride = m.acc_stride;
+    float *rowA = tileA + lane * kAccStride;
     if (EDEN_KIND_CLAMP && kind == BK_PULSE && ((info >> 2) & 63) >= kClampA) {
         // voltage clamps (LEMS_CoreComponents.inc.xml:555-620): the target
         // of the phase each step's time is in (the last OnCondition that
@@ -788,7 +825,7 @@ __device__ __forceinline__ void chunk_window(const DevModel &m, int c, int32_t i
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
             for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
-            m.Gp[(size_t)lane * m.n_chunk + c] = tot;
+            m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
         return;
@@ -818,9 +855,24 @@ __device__ __forceinline__ void chunk_window(const DevModel &m, int c, int32_t i
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
             for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
-            m.Gp[(size_t)lane * m.n_chunk + c] = tot;
+            m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
+        return;
+    }
+    if (EDEN_KIND_PULSE && kind == BK_PULSE && 2 * n <= w.K) {
+        // a few pulses: lane j evaluates step j of each.  About 10 n
+        // instructions, where the rows below take 6 K + 2 n: the line is where
+        // these meet, on the safe side.  (30,011 cells of one pulse, 31 steps:
+        // 22 us by rows, 11 by steps.)
+        float tot = 0.0f;
+        const float tf = tk[lane];
+        for (int q = 0; q < n; q++) {
+            const int64_t it = ck_i0 + q;
+            const float st = m.pu_start[it], du = m.pu_dur[it], aw = __fmul_rn(m.pu_amp[it], m.pu_w[it]);
+            tot = __fadd_rn(tot, (st <= tf && tf <= st + du) ? aw : 0.0f);
+        }
+        if (lane < w.K) m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         return;
     }
     if (EDEN_KIND_PULSE && kind == BK_PULSE) {
@@ -838,90 +890,72 @@ __device__ __forceinline__ void chunk_window(const DevModel &m, int c, int32_t i
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
             for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
-            m.Gp[(size_t)lane * m.n_chunk + c] = tot;
+            m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
         return;
     }
-    const int type = (info >> 2) & 63;
-    const SynTypeDev st = m.syn_types[type];
-    const bool two = st.kind == EDEN_SYN_EXPTWO || st.kind == EDEN_SYN_BLOCKING_PLASTIC;
-    bool used = false;
-    // the chunk's aggregate and its items' per-window state, loaded up front
-    // so the loads overlap
-    float A = m.ck_a[c], B = m.ck_b[c];
-    const int64_t i0 = ck_i0 + lane;
-    float s0v[kChunkItems / 32], s1v[kChunkItems / 32];
-#pragma unroll
-    for (int r = 0; r < kChunkItems / 32; r++) {
-        s0v[r] = 0.0f; s1v[r] = 0.0f;
-        if (lane + 32 * r < n) {
-            const int64_t it = i0 + 32 * r;
-            if (kind == BK_POIS) { s0v[r] = m.po_ts[it]; s1v[r] = m.po_isi[it]; }
-            else if (kind == BK_SYN) { s0v[r] = m.sy_pend[it]; s1v[r] = __uint_as_float(m.sy_mask[it]); }
+}
+
+// The events of a listed item in the window.
+__device__ __forceinline__ void item_window(const DevModel &m, int32_t info, int64_t it, const WindowArgs &w, const HotItem &h,
+                                            const float *tk, float *rowA, float *rowB, ItemEvents &ev) {
+    const int kind = info & 3, type = (info >> 2) & 63;
+    const SynTypeDev &st = m.syn_types[type];
+    const float *pw = m.syn_pow + (size_t)type * 2 * kPowLen;
+    const bool two = EDEN_KIND_EXPTWO && (!EDEN_KIND_EXPONE || st.kind == EDEN_SYN_EXPTWO ||
+                                          st.kind == EDEN_SYN_BLOCKING_PLASTIC);
+    // only the input kinds the kernels are compiled for (all, or the model's)
+    if (kind == BK_TIMED) {
+        if (EDEN_KIND_TIMED) {
+            if (two) { if (EDEN_KIND_EXPTWO) timed_window<EDEN_SYN_EXPTWO>(m, it, w, st, pw, rowA, rowB, ev); }
+            else if (EDEN_KIND_EXPONE) timed_window<EDEN_SYN_EXPONE>(m, it, w, st, pw, rowA, rowB, ev);
         }
-    }
-#pragma unroll
-    for (int r = 0; r < kChunkItems / 32; r++) {
-        if (lane + 32 * r < n) {
-            const int64_t it = i0 + 32 * r;
-            // only the input kinds the kernels are compiled for (all, or the model's)
-            if (kind == BK_TIMED) {
-                if (EDEN_KIND_TIMED) {
-                    if (two) { if (EDEN_KIND_EXPTWO) timed_window<EDEN_SYN_EXPTWO>(m, it, w, st, rowA, rowB, used); }
-                    else if (EDEN_KIND_EXPONE) timed_window<EDEN_SYN_EXPONE>(m, it, w, st, rowA, rowB, used);
-                }
-            } else if (kind == BK_POIS) {
-                if (EDEN_KIND_POIS) {
-                    if (two) { if (EDEN_KIND_EXPTWO) pois_window<EDEN_SYN_EXPTWO>(m, it, w, st, s0v[r], s1v[r], rowA, rowB, used); }
-                    else if (EDEN_KIND_EXPONE) pois_window<EDEN_SYN_EXPONE>(m, it, w, st, s0v[r], s1v[r], rowA, rowB, used);
-                }
-            } else if (EDEN_KIND_SYN) {
-                const uint32_t mask = __float_as_uint(s1v[r]);
-                if (two) { if (EDEN_KIND_EXPTWO) syn_window<EDEN_SYN_EXPTWO>(m, it, w, st, tk, s0v[r], mask, rowA, rowB, used); }
-                else if (EDEN_KIND_EXPONE) syn_window<EDEN_SYN_EXPONE>(m, it, w, st, tk, s0v[r], mask, rowA, rowB, used);
-            }
+    } else if (kind == BK_POIS) {
+        if (EDEN_KIND_POIS) {
+            if (two) { if (EDEN_KIND_EXPTWO) pois_window<EDEN_SYN_EXPTWO>(m, it, w, st, pw, h.s0, h.s1, rowA, rowB, ev); }
+            else if (EDEN_KIND_EXPONE) pois_window<EDEN_SYN_EXPONE>(m, it, w, st, pw, h.s0, h.s1, rowA, rowB, ev);
         }
+    } else if (EDEN_KIND_SYN) {
+        const uint32_t mask = __float_as_uint(h.s1);
+        if (two) { if (EDEN_KIND_EXPTWO) syn_window<EDEN_SYN_EXPTWO>(m, it, w, st, pw, tk, h.s0, mask, rowA, rowB, ev); }
+        else if (EDEN_KIND_EXPONE) syn_window<EDEN_SYN_EXPONE>(m, it, w, st, pw, tk, h.s0, mask, rowA, rowB, ev);
     }
-    const unsigned rows = __ballot_sync(0xffffffffu, used);
-    __syncwarp();
+}
+
+// A synapse chunk's aggregate through the window from its state (A, B) and,
+// in lane j, its events ea, eb of step j.  Returns, for lane j, the exposure of
+// step j: the conductance before the step's update, as the reference exposes
+// it.  With one step's decay factor f, X_j = f^j X_0 + sum_{i<j} f^(j-1-i) e_i,
+// the sums by a scan over the lanes; without events in closed form, A f^j,
+// from the factors' powers (syn_pow).
+__device__ __forceinline__ float chunk_series(const DevModel &m, int type, const WindowArgs &w, bool events, float ea,
+                                              float eb, float &A, float &B) {
+    const int lane = threadIdx.x & 31;
+    const SynTypeDev &st = m.syn_types[type];
+    const float *pr = m.syn_pow + (size_t)type * 2 * kPowLen, *pd = pr + kPowLen;
+    if (EDEN_KIND_ALPHA && (st.kind == EDEN_SYN_ALPHA || st.kind == EDEN_SYN_ALPHA_CURRENT))
+        return alpha_chunk_window(pd, st, w, events, ea, A, B);
+    const bool two = EDEN_KIND_EXPTWO && (!EDEN_KIND_EXPONE || st.kind == EDEN_SYN_EXPTWO ||
+                                          st.kind == EDEN_SYN_BLOCKING_PLASTIC);
     float gj = 0.0f;
-    if (EDEN_KIND_ALPHA && (st.kind == EDEN_SYN_ALPHA || st.kind == EDEN_SYN_ALPHA_CURRENT)) {
-        alpha_chunk_window(m, c, type, st, w, rows, A, B, tileA);
-        return;
-    }
-    if (rows == 0) {
-        // no event in the window: the aggregate decays in closed form,
-        // A f^j, from the factors' powers (syn_pow)
-        const float *pr = m.syn_pow + (size_t)type * 2 * kPowLen, *pd = pr + kPowLen;
+    if (!events) {
         if (lane < w.K) gj = two ? st.gbase * (B * pd[lane] - A * pr[lane]) : A * pd[lane];
         if (w.step0 > 0) {
             A = A * (two ? pr[w.K] : pd[w.K]);
             B = two ? B * pd[w.K] : B;
         }
-        if (lane < w.K) m.Gp[(size_t)lane * m.n_chunk + c] = gj;
-        if (lane == 0) { m.ck_a[c] = A; m.ck_b[c] = B; }
-        __syncwarp();
-        return;
+        return gj;
     }
-    float ea = 0.0f, eb = 0.0f;  // lane j: the chunk's events of step j
-    if (lane < w.K)
-        for (unsigned r = rows; r; r &= r - 1) {
-            const int q = __ffs(r) - 1;
-            ea += tileA[q * kAccStride + lane];
-            eb += tileB[q * kAccStride + lane];
-        }
-    // the aggregate over the window: with one step's decay factor f,
-    // X_j = f^j X_0 + sum_{i<j} f^(j-1-i) e_i, the sums by a scan over the lanes
-    const float *pr = m.syn_pow + (size_t)type * 2 * kPowLen, *pd = pr + kPowLen;
     const float *pa = two ? pr : pd;
     float va = lane < w.K ? ea : 0.0f, vb = lane < w.K ? eb : 0.0f;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const float ua = __shfl_up_sync(0xffffffffu, va, d), ub = __shfl_up_sync(0xffffffffu, vb, d);
-        if (lane >= d) {
-            va = fmaf(pa[d], ua, va);
-            vb = fmaf(pd[d], ub, vb);
+        const float ua = __shfl_up_sync(0xffffffffu, va, d);
+        if (lane >= d) va = fmaf(pa[d], ua, va);
+        if (two) {
+            const float ub = __shfl_up_sync(0xffffffffu, vb, d);
+            if (lane >= d) vb = fmaf(pd[d], ub, vb);
         }
     }
     // lane j: sums of the events before step j
@@ -934,24 +968,176 @@ __device__ __forceinline__ void chunk_window(const DevModel &m, int c, int32_t i
     const float ta = __shfl_sync(0xffffffffu, va, w.K - 1), tb = __shfl_sync(0xffffffffu, vb, w.K - 1);
     A = A * pa[w.K] + ta;
     B = two ? B * pd[w.K] + tb : B;
-    if (lane < w.K) m.Gp[(size_t)lane * m.n_chunk + c] = gj;
-    if (lane == 0) { m.ck_a[c] = A; m.ck_b[c] = B; }
+    return gj;
+}
+
+// A group of nc <= kInputGroup consecutive chunks, c0 on, over the K steps of a
+// window, by one warp.  Few of a chunk's synapses and Poisson inputs have an
+// event in a window, and the code of one that has is long; run chunk by chunk
+// it was the whole of the kernel's time with most of its lanes idle.  So the
+// warp looks at every item's state first and lists those that may have an
+// event, over all chunks of the group; then each lane works off one of the
+// list (100,000 neurons of 100 synapses, windows of 10 steps: 484 us by items
+// of a lane one after another, 186 with a list per chunk, 123 per group of 16;
+// instruction issue bounds it, 62 % of its peak, memory at 27 %); then the chunks are finished in order, lane j summing the events of
+// step j -- over the items that share a lane of the chunk (l, l + 32, ...),
+// then over these lanes in order -- and taking the aggregate through the window.
+__device__ __forceinline__ void input_group(const DevModel &m, int c0, int nc, const WindowArgs &w, float *tileA,
+                                            float *tileB, HotItem *list, const float *tk) {
+    const int lane = threadIdx.x & 31;
+    const int stride = m.acc_stride;
+    float *rowA = tileA + lane * stride, *rowB = tileB + lane * stride;
+    // lane i: chunk i of the group
+    int32_t info_l = 0;
+    int64_t i0_l = 0;
+    float A_l = 0.0f, B_l = 0.0f;
+    if (lane < nc) {
+        info_l = m.ck_info[c0 + lane];
+        i0_l = m.ck_i0[c0 + lane];
+        A_l = m.ck_a[c0 + lane];
+        B_l = m.ck_b[c0 + lane];
+    }
+    const float t_end = tk[w.K - 1] + m.dt;
+    int count = 0, done = 0;  // listed items; chunks finished
+#pragma unroll 1
+    for (int i = 0;; i++) {
+        const int32_t info = __shfl_sync(0xffffffffu, info_l, i);
+        const int64_t ck_i0 = __shfl_sync(0xffffffffu, i0_l, i);
+        const int kind = info & 3, n = info >> 8;
+        if (i < nc && kind == BK_PULSE) {
+            pulse_chunk(m, c0 + i, info, ck_i0, w, tileA, tk);
+            continue;
+        }
+        if (i == nc || count + n > kHotItems) {
+            // work off the list, and finish the chunks before i
+            __syncwarp();
+            int b = -32, last = -1;  // the list's batch, and the chunk of its last item
+            unsigned rows = 0, more = 0;
+            ItemEvents ev{0, 0, 0.0f, 0.0f};
+            int at = -1;
+#pragma unroll 1
+            for (int q = done; q < i; q++) {
+                const int32_t info_q = __shfl_sync(0xffffffffu, info_l, q);
+                if ((info_q & 3) == BK_PULSE) continue;
+                float ea = 0.0f, eb = 0.0f;  // lane j: the chunk's events of step j
+                float sa = 0.0f, sb = 0.0f;  // of the items of one lane of the chunk
+                int of = -1;
+                bool events = false;
+#pragma unroll 1
+                while (true) {
+                    const unsigned mine = rows & __ballot_sync(0xffffffffu, (at >> 7) == q);
+                    events |= mine != 0;
+                    for (unsigned r = mine; r; r &= r - 1) {
+                        const int e = __ffs(r) - 1;
+                        const int l = __shfl_sync(0xffffffffu, at, e) & 31, j = __shfl_sync(0xffffffffu, ev.j, e);
+                        float dA = __shfl_sync(0xffffffffu, ev.dA, e);
+                        float dB = EDEN_KIND_EXPTWO ? __shfl_sync(0xffffffffu, ev.dB, e) : 0.0f;
+                        if (lane != j) {
+                            dA = dB = 0.0f;
+                            if (((more >> e) & 1u) && lane < w.K) {
+                                dA = tileA[e * stride + lane];
+                                if (EDEN_KIND_EXPTWO) dB = tileB[e * stride + lane];
+                            }
+                        }
+                        if (l != of) {
+                            ea += sa;
+                            eb += sb;
+                            sa = sb = 0.0f;
+                            of = l;
+                        }
+                        sa = __fadd_rn(sa, dA);
+                        if (EDEN_KIND_EXPTWO) sb = __fadd_rn(sb, dB);
+                    }
+                    if (b + 32 >= count || last > q) break;
+                    // the next batch: this one's items are all of chunks up to q
+                    __syncwarp();
+                    b += 32;
+                    ev = ItemEvents{0, 0, 0.0f, 0.0f};
+                    HotItem h{0.0f, 0.0f, -1};
+                    if (b + lane < count) h = list[b + lane];
+                    at = h.at;
+                    const int32_t info_e = __shfl_sync(0xffffffffu, info_l, (at >> 7) & 31);
+                    const int64_t it = __shfl_sync(0xffffffffu, i0_l, (at >> 7) & 31) + (at & (kChunkItems - 1));
+                    if (at >= 0) item_window(m, info_e, it, w, h, tk, rowA, rowB, ev);
+                    rows = __ballot_sync(0xffffffffu, ev.n > 0);
+                    more = __ballot_sync(0xffffffffu, ev.n > 1);
+                    last = __shfl_sync(0xffffffffu, at, min(31, count - 1 - b)) >> 7;
+                    __syncwarp();
+                }
+                ea += sa;
+                eb += sb;
+                float A = __shfl_sync(0xffffffffu, A_l, q), B = __shfl_sync(0xffffffffu, B_l, q);
+                const float gj = chunk_series(m, (info_q >> 2) & 63, w, events, ea, eb, A, B);
+                if (lane == q) { A_l = A; B_l = B; }
+                if (lane < w.K) m.Gp[(size_t)(c0 + q) * m.gp_stride + lane] = gj;
+            }
+            __syncwarp();
+            if (i == nc) break;
+            done = i;
+            count = 0;
+        }
+        // list the chunk's items that may have an event, lane by lane and a
+        // lane's in order
+        float s0v[kChunkItems / 32], s1v[kChunkItems / 32];
+        unsigned hot[kChunkItems / 32];
+#pragma unroll
+        for (int r = 0; r < kChunkItems / 32; r++) {
+            s0v[r] = 0.0f; s1v[r] = 0.0f;
+            if (lane + 32 * r < n) {
+                const int64_t it = ck_i0 + lane + 32 * r;
+                if (kind == BK_POIS) { s0v[r] = m.po_ts[it]; s1v[r] = m.po_isi[it]; }
+                else if (kind == BK_SYN) { s0v[r] = m.sy_pend[it]; s1v[r] = __uint_as_float(m.sy_mask[it]); }
+            }
+        }
+        int at = count;
+#pragma unroll
+        for (int r = 0; r < kChunkItems / 32; r++) {
+            hot[r] = 0;
+            if (32 * r >= n) continue;
+            bool h = false;
+            if (lane + 32 * r < n) {
+                const int64_t it = ck_i0 + lane + 32 * r;
+                if (kind == BK_TIMED) {
+                    const int64_t cur = m.tm_cur[it];
+                    h = EDEN_KIND_TIMED && cur < m.tm_off[it + 1] && m.tm_step[cur] < w.step0 + w.K;
+                } else if (kind == BK_POIS) {
+                    // (exact sums: no firing in the window when even its last step's
+                    // time since the spike stays within the interval)
+                    h = !(w.step0 > 0 && m.pois_exact && s1v[r] < 0x1p23f && s0v[r] + (float)(w.K - 1) * m.dt <= s1v[r]);
+                    if (!h) m.po_ts[it] = s0v[r] + (float)w.K * m.dt;
+                } else {
+                    // (no spikes reach a synapse during initialisation)
+                    h = w.step0 > 0 && (__float_as_uint(s1v[r]) != 0 || (s0v[r] >= tk[0] && s0v[r] < t_end));
+                }
+            }
+            hot[r] = __ballot_sync(0xffffffffu, h);
+            count += __popc(hot[r]);
+            at += __popc(hot[r] & ((1u << lane) - 1));
+        }
+#pragma unroll
+        for (int r = 0; r < kChunkItems / 32; r++)
+            if ((hot[r] >> lane) & 1u) list[at++] = HotItem{s0v[r], s1v[r], i * kChunkItems + lane + 32 * r};
+    }
+    if (lane < nc && (info_l & 3) != BK_PULSE) {
+        m.ck_a[c0 + lane] = A_l;
+        m.ck_b[c0 + lane] = B_l;
+    }
     __syncwarp();
 }
 
 // Currents into target t at step j of the window from its input blocks:
 // pulses add current; conductance blocks add g*(erev - v) and g, inputs
 // first, then synapses, as eden/Eden.cpp:6057-6060 orders them.  BK_K and
-// BK_E are the blocks' kinds and reversal potentials, BC0 their chunk ranges
-// (indexed from blk0 and chk0, which may point into shared memory).
-__device__ __forceinline__ void block_currents(const float *Gpk, int b0, int b1, const int32_t *BK_K,
-                                               const float *BK_E, const int32_t *BC0, int chk0, float v, float &Iin,
-                                               float &Gin, float &Isyn, float &Gsyn,
+// BK_E are the blocks' kinds and reversal potentials, BC0 their chunk ranges;
+// Gpk is Gp at the step.
+__device__ __forceinline__ void block_currents(const float *Gpk, int stride, int b0, int b1, const int32_t *BK_K,
+                                               const float *BK_E, const int32_t *BC0, float v, float &Iin, float &Gin,
+                                               float &Isyn, float &Gsyn,
                                                const float2 *BK_B = nullptr) {
     Iin = 0.0f; Gin = 0.0f; Isyn = 0.0f; Gsyn = 0.0f;
     for (int bk = b0; bk < b1; bk++) {
         float g = 0.0f;
-        for (int c = BC0[bk]; c < BC0[bk + 1]; c++) g += Gpk[c + chk0];
+        for (int c = BC0[bk]; c < BC0[bk + 1]; c++) g += Gpk[(size_t)c * stride];
         // a blockingPlasticSynapse's voltage block (voltageConcDepBlockMechanism,
         // LEMS_CoreComponents.inc.xml:231-245) scales its conductance, so both
         // the current and the conductance term (per-step kernels only)
@@ -978,17 +1164,18 @@ __device__ __forceinline__ void block_currents(const float *Gpk, int b0, int b1,
     }
 }
 
-// block_currents from the unit's block records in shared memory (first chunk,
-// end chunk, kind, reversal potential)
-__device__ __forceinline__ void block_currents_rec(const float *Gk, const int4 *BK, int b0, int b1, float v, float &Iin,
-                                                   float &Gin, float &Isyn, float &Gsyn) {
+// block_currents from the unit's block records in shared memory (where its
+// chunks begin and end in the unit's series, `stride` apart, kind, reversal
+// potential)
+__device__ __forceinline__ void block_currents_rec(const float *Gk, int stride, const int4 *BK, int b0, int b1, float v,
+                                                   float &Iin, float &Gin, float &Isyn, float &Gsyn) {
     Iin = 0.0f; Gin = 0.0f; Isyn = 0.0f; Gsyn = 0.0f;
 #pragma unroll 1
     for (int bk = b0; bk < b1; bk++) {
         const int4 r = BK[bk];
         float g = Gk[r.x];
 #pragma unroll 1
-        for (int c = r.x + 1; c < r.y; c++) g += Gk[c];
+        for (int c = r.x + stride; c < r.y; c += stride) g += Gk[c];
         const int kind = r.z & BK_KIND_MASK;
         if (EDEN_KIND_CLAMP && kind == BK_CLAMPV) {
             Iin -= v * g;

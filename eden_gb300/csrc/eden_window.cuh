@@ -21,12 +21,16 @@ constexpr int kHinesThreads = 128;  // k_hines_t: four warps, each staging one f
 // ---------------------------------------------------------------------------
 namespace eden {
 
-// Phase 1 of both paths: input blocks over the window, one warp per target
-// with inputs (the per-step path runs it with K = 1).  Six blocks fit an SM
-// by their event tiles; the register bound lets all six run.
-__global__ void __launch_bounds__(kInputThreads, 6) k_inputs_t(DevModel m, const WindowArgs *tab,
+// Phase 1 of both paths: input blocks over the window (the per-step path runs
+// it with K = 1), a warp per group of consecutive chunks.  A group grows past
+// one chunk only when there are more chunks than resident warps: a small
+// model's chunks all run at once, a large model's items with full warps.
+// The event tiles are only as long as the model's windows (dynamic shared
+// memory), so that the registers, 32 warps an SM, bound the occupancy.
+__global__ void __launch_bounds__(kInputThreads, 8) k_inputs_t(DevModel m, const WindowArgs *tab,
                                                              const WindowTimes *ttab, const int *base, int idx) {
-    __shared__ float tiles[kInputThreads / 32][2][32 * kAccStride];
+    extern __shared__ __align__(16) float sm[];
+    __shared__ HotItem lists[kInputThreads / 32][kHotItems];
     __shared__ float tk[64];  // the window's step times, then the previous window's
     const int wi = *base + idx;
     const WindowArgs w = tab[wi];
@@ -34,20 +38,11 @@ __global__ void __launch_bounds__(kInputThreads, 6) k_inputs_t(DevModel m, const
     __syncthreads();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    float *tileA = tiles[threadIdx.x >> 5][0], *tileB = tiles[threadIdx.x >> 5][1];
-    // each warp walks its chunks with the next chunk's descriptor in flight
-    int c = warp;
-    int32_t info = 0;
-    int64_t i0 = 0;
-    if (c < m.n_chunk) { info = m.ck_info[c]; i0 = m.ck_i0[c]; }
-    while (c < m.n_chunk) {
-        const int cn = c + nwarps;
-        int32_t info_n = 0;
-        int64_t i0_n = 0;
-        if (cn < m.n_chunk) { info_n = m.ck_info[cn]; i0_n = m.ck_i0[cn]; }
-        chunk_window(m, c, info, i0, w, tileA, tileB, tk);
-        c = cn; info = info_n; i0 = i0_n;
-    }
+    float *tileA = sm + (threadIdx.x >> 5) * 64 * m.acc_stride, *tileB = tileA + 32 * m.acc_stride;
+    HotItem *list = lists[threadIdx.x >> 5];
+    const int group = min(kInputGroup, (m.n_chunk + nwarps - 1) / nwarps);
+    for (int64_t c = (int64_t)warp * group; c < m.n_chunk; c += (int64_t)nwarps * group)
+        input_group(m, (int)c, min(group, m.n_chunk - (int)c), w, tileA, tileB, list, tk);
 }
 
 // Per-step path, phase 2: one thread per target.
@@ -63,8 +58,8 @@ __global__ void __launch_bounds__(256) k_targets_t(DevModel m, const WindowArgs 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nround; i += gridDim.x * blockDim.x) {
         if (i < n) {
             float v = vin[i], Iin, Gin, Isyn, Gsyn;
-            block_currents(m.Gp, m.t_blk0[i], m.t_blk0[i + 1], m.bk_kind, m.bk_erev, m.bk_c0, 0, v, Iin, Gin, Isyn,
-                           Gsyn, m.bk_block);
+            block_currents(m.Gp, m.gp_stride, m.t_blk0[i], m.t_blk0[i + 1], m.bk_kind, m.bk_erev, m.bk_c0, v, Iin, Gin,
+                           Isyn, Gsyn, m.bk_block);
             if (EDEN_KIND_GAP) Isyn += gap_current(m, i, v, vin, init);
             const float Iax = (m.fwd_euler && !init && m.t_izh[i] < 0) ? axial_current(m, i, v, vin) : 0.0f;
             target_step(m, i, init, w.step0, tnow, v, Iin, Gin, Isyn, Gsyn, &vout[i], &m.diag[i], w.wpar, Iax);
@@ -194,7 +189,9 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     float4 *CN = reinterpret_cast<float4 *>(TV + 32 * nw), *TR = CN + n + 1;
     float4 *NF = TR + 32 * nw;
     int4 *BK = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
-    float2 *TS = reinterpret_cast<float2 *>(BK + nblk);
+    const int gps = m.gp_stride;
+    float *GS = reinterpret_cast<float *>(BK + nblk);
+    float2 *TS = reinterpret_cast<float2 *>(GS + gps * nck);
     uint32_t *TA = reinterpret_cast<uint32_t *>(TS + nf);
     float *VO = (float *)(TA + 32 * nw);
     float *CHG = VO + nf, *CHE = CHG + nch;
@@ -202,10 +199,9 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     int32_t *GI = CHI + nch;
     float *GT = (float *)(GI + ngt);  // two buffers of ngt
     int32_t *PS = (int32_t *)(GT + 2 * ngt);
-    float *GS = (float *)(PS + np);
     // a double-precision forest's eliminated values, pivots and factors
     const bool f64 = m.fo_f64[fi] != 0;
-    double *XD = reinterpret_cast<double *>((reinterpret_cast<unsigned long long>(GS + w.K * nck) + 7ull) & ~7ull);
+    double *XD = reinterpret_cast<double *>((reinterpret_cast<unsigned long long>(PS + np) + 7ull) & ~7ull);
     double *PVD = XD + n, *RTD = PVD + n;
     // the steps of a window are all initialisation passes or none is
     const bool init = w.step0 <= 0;
@@ -237,8 +233,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     }
     for (int i = lane; i < ngt; i += 32) { stage_word(&GT[i], &m.gate[gt0 + i]); stage_word(&GI[i], &m.gt_idx[gt0 + i]); }
     for (int i = lane; i < np; i += 32) stage_word(&PS[i], &m.ps[ps0 + i]);
-    for (int k = 0; k < w.K; k++)
-        for (int c = lane; c < nck; c += 32) stage_word(&GS[k * nck + c], &m.Gp[(size_t)k * m.n_chunk + uc0 + c]);
+    for (int i = 4 * lane; i < gps * nck; i += 128) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
     stage_wait();
     __syncwarp();
     for (int j = lane; j < nf; j += 32) VO[j] = XR[__float_as_int(NF[kSlotRecs * j].x) & kPassStart].x;
@@ -268,7 +263,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             }
             __syncwarp();
         }
-        const float *Gk = GS + k * nck;
+        const float *Gk = GS + k;
 #pragma unroll 1
         for (int j = lane; j < nf; j += 32) {
             // channels + voltage pre-update (eden/Eden.cpp:5013-6107)
@@ -278,7 +273,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             const int ch0 = crange & 0xffff;
             const float v = VO[j];
             float Iin, Gin, Isyn, Gsyn;
-            block_currents_rec(Gk, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
+            block_currents_rec(Gk, gps, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
             // (a model with gap junctions runs one-step windows: vsrc holds
             // every target's potential at this step's start)
             if (EDEN_KIND_GAP) Isyn += gap_current(m, t0 + m.nd_t[n0 + ti], v, vsrc, init);
@@ -412,7 +407,7 @@ __device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &
         const bool init = step <= 0;
         const float *vin = S + par * n;
         float *vout = S + (par ^ 1) * n;
-        const float *Gpk = m.Gp + (size_t)k * m.n_chunk;
+        const float *Gpk = m.Gp + k;
         const int i = lane;
         bool spike = false;
         int src = -1;
@@ -420,8 +415,8 @@ __device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &
             const int t = t0 + i;
             const float v = vin[i];
             float Iin, Gin, Isyn, Gsyn;
-            block_currents(Gpk, m.t_blk0[t], m.t_blk0[t + 1], m.bk_kind, m.bk_erev, m.bk_c0, 0, v, Iin, Gin, Isyn,
-                           Gsyn);
+            block_currents(Gpk, m.gp_stride, m.t_blk0[t], m.t_blk0[t + 1], m.bk_kind, m.bk_erev, m.bk_c0, v, Iin, Gin,
+                           Isyn, Gsyn);
             float uu = SU[i], ss = SS[i], vn;
             spike = point_update(KIND[i], P + i, n, init, tk[k], dt, v, Isyn + Iin, uu, ss, vn);
             vout[i] = vn;
