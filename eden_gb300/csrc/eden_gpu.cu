@@ -1488,23 +1488,39 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             if (w > limit) return grow;
         return true;
     };
+    // A unit's gates get a warp beside its own (forest_window) where no gate takes
+    // V after the solve, and all units' two warps are resident together; where
+    // they are not, the warps there are keep the SM busy and a second round
+    // costs more than a shorter step gives.  (A window, one warp and two: 1,000
+    // HH cells 57 and 41 us, 30,011 76 and 64, 50 trees 110 and 100, 1,200
+    // trees with active dendrites 231 and 189, 5,000 cells of 100 compartments
+    // 111 and 100.)  At most four such CTAs an SM: the kernel names its barriers
+    // at run time, so each CTA takes all 16, and with five or six, the last
+    // waited for the first (30,011 cells: 97 us, the 5,000: 155).
+    bool gate_warp = false;
     {
-        const int sms = std::max(ctx->n_sm, 1), warps = kCellThreads / 32;
+        const int sms = std::max(ctx->n_sm, 1);
+        const bool may_pair = !gate_forms && ch_gate0[c_chan0[nt]] > 0;
         bool fits = false;
-        if (n_unit <= sms) fits = pack(n_unit, 1, most, true);
-        for (int per_sm = 6; !fits && per_sm >= 1; per_sm--) {
-            const int upc = warps / per_sm;
-            if ((int64_t)sms * per_sm * upc < n_unit) continue;
-            const int ctas = std::min(sms * per_sm, n_unit);
-            // (a block's own share of the SM: its words, padding and 1 KB of the system's)
-            const int share = (int)(ctx->smem_per_sm / per_sm / sizeof(float)) - 4 * kPassPad - 256;
-            fits = pack(ctas, upc, std::min(most, share), false);
+        for (int pairs = may_pair; !fits && pairs >= 0; pairs--) {
+            gate_warp = pairs;
+            const int warps = kCellThreads / 32 / (1 + pairs);
+            if (n_unit <= sms) fits = pack(n_unit, 1, most, true);
+            for (int per_sm = pairs ? 4 : 6; !fits && per_sm >= 1; per_sm--) {
+                const int upc = warps / per_sm;
+                if ((int64_t)sms * per_sm * upc < n_unit) continue;
+                const int ctas = std::min(sms * per_sm, n_unit);
+                // (a block's own share of the SM: its words, padding and 1 KB of the system's)
+                const int share = (int)(ctx->smem_per_sm / per_sm / sizeof(float)) - 4 * kPassPad - 256;
+                fits = pack(ctas, upc, std::min(most, share), false);
+            }
         }
         if (!fits) pack((n_unit + 3) / 4, 4, most, true);
     }
+    ctx->d.gate_warp = gate_warp;
     int max_units = 1;
     for (auto &c : cta_units) max_units = std::max(max_units, (int)c.size());
-    ctx->cell_threads = 32 * max_units;
+    ctx->cell_threads = (gate_warp ? 64 : 32) * max_units;
     std::vector<int32_t> cta_u0, un_off(n_unit, 0), unit_of_slot;
     for (int c = 0; c < n_cta; c++) {
         cta_u0.push_back((int)unit_of_slot.size());
@@ -1844,6 +1860,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         }
         kinds.forest = d.n_forest > 0;
         kinds.gateforms = gate_forms;
+        kinds.gate_warps = gate_warp;
         kinds.izh = n_izh > 0;
         kinds.gap = m->n_gap > 0 || m->n_graded > 0;
         ctx->codegen_source = eden_codegen::program_source(eden_codegen::kind_defines(kinds) +

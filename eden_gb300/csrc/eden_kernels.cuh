@@ -262,6 +262,7 @@ struct DevModel {
     // gate of a channel type, three 16-byte records (gate_next_p)
     const int32_t *gt_idx;
     const float4 *gate_tab;
+    int32_t gate_warp;  // a unit's gates have a warp of their own (no gate takes V after the solve)
     // per input block: where its chunks begin and end in the unit's series
     // (gp_stride each), kind and reversal potential
     const int4 *bk_rec;
@@ -339,8 +340,8 @@ constexpr int kGateExtWords = 9;  // a non-rates gate's kind and timeCourse / st
 // records: one per node, one per twig place, two per non-flat compartment, one
 // per input block, and the window's conductance series of the unit's input
 // chunks (gps words each); then pairs: threshold and source per non-flat
-// compartment; then words: a twig place's addresses, V at the step's start per
-// non-flat compartment, four per channel of these, three per gate (its index
+// compartment; then words: a twig place's addresses, V at the start of the step,
+// the next and the last per non-flat compartment, four per channel of these, three per gate (its index
 // word, its value in alternate steps), and the passes.  A batch of izhikevich
 // neurons: V twice and 19 parameter / state words per neuron.
 __host__ __device__ inline int twig_words(int n) { return (2 * n + 3) & ~3; }  // where the twigs' words start
@@ -349,7 +350,7 @@ __host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int
     // a double-precision forest adds its eliminated values, pivots and
     // factors in double (6 words per compartment, 8-byte aligned)
     const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + gps * nck + 2 * nf +
-                  32 * nw + nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
+                  32 * nw + 3 * nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
     return (w + 3) & ~3;
 }
 __host__ __device__ inline int izh_words(int n) { return ((2 + EDEN_POINT_PARAMS + 3) * n + 3) & ~3; }
@@ -706,6 +707,9 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
 #define EDEN_KIND_GAP 1
 #define EDEN_KIND_ALPHA 1
 #define EDEN_KIND_CURRENT 1
+#endif
+#ifndef EDEN_GATE_WARPS
+#define EDEN_GATE_WARPS 1  // units' gates may have a warp of their own (DevModel::gate_warp)
 #endif
 
 // A timedSynapticInput item over the window: its synapse fires in each

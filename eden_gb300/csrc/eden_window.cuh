@@ -170,15 +170,33 @@ __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs 
 // crossings.  A lane with at most one non-flat compartment, or one gate, keeps
 // its record in registers for the whole window.
 //
+// The gates and the currents of a step both read its starting state only, so a
+// unit with gates is run by two warps: one (`gates`) updates the gates, and
+// tests the thresholds a step behind, beside the other's currents and solve,
+// with a barrier of the two a step.  With gate_warp unset one warp does all of it
+// in turn.
+//
 // With the unit in shared memory the kernel moves 15 times less than a step
 // over HBM would, and is bound by the length of a step's dependent chain and,
 // with many units, by the instructions issued: hence few instructions a pass,
 // divisions by constants done as div_known, and units sized in edenGpuCreate.
-__device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S) {
+// (A kernel compiled for a model without gate warps keeps the threshold test in
+// the loop that takes V over; with them, one body for both roles: compiled
+// apart, the solve of 50 trees took 112 us a window instead of 100.)
+__device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S, bool gates,
+                                              int barrier) {
     const int lane = threadIdx.x & 31;
     const int t0 = m.un_t0[u], fi = m.un_f[u], ub0 = m.t_blk0[t0], nblk = m.t_blk0[m.un_t1[u]] - ub0;
     const int n0 = m.fo_n0[fi], n = m.fo_n0[fi + 1] - n0, w0 = m.fo_w0[fi], nw = m.fo_w0[fi + 1] - w0;
     const int ngt = m.un_ngt[u], gt0 = m.un_gt0[u];
+    const bool pair = EDEN_GATE_WARPS && m.gate_warp && ngt > 0;
+    if (gates && !pair) return;
+    // the unit's threads, and a barrier of them
+    const int th = gates ? lane + 32 : lane, nth = pair ? 64 : 32;
+    auto unit_sync = [&]() {
+        if (pair) asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+        else __syncwarp();
+    };
     const int r0 = m.un_r0[u], r1 = m.un_r1[u];
     const int nf0 = m.un_nf0[u], nf = m.un_nf1[u] - nf0;
     const int ps0 = m.fo_p0[fi], np = m.fo_p0[fi + 1] - ps0;
@@ -193,8 +211,8 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     float *GS = reinterpret_cast<float *>(BK + nblk);
     float2 *TS = reinterpret_cast<float2 *>(GS + gps * nck);
     uint32_t *TA = reinterpret_cast<uint32_t *>(TS + nf);
-    float *VO = (float *)(TA + 32 * nw);
-    float *CHG = VO + nf, *CHE = CHG + nch;
+    float *VO = (float *)(TA + 32 * nw);  // three buffers of nf: step k starts from buffer k % 3
+    float *CHG = VO + 3 * nf, *CHE = CHG + nch;
     int32_t *CHQ = (int32_t *)(CHE + nch), *CHI = CHQ + nch;
     int32_t *GI = CHI + nch;
     float *GT = (float *)(GI + ngt);  // two buffers of ngt
@@ -207,47 +225,102 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     const bool init = w.step0 <= 0;
     // ---- stage the unit
     const float *vsrc = m.v[w.par];
-    for (int i = lane; i < n; i += 32) {
+    for (int i = th; i < n; i += nth) {
         const int t = m.nd_t[n0 + i];
         stage_rec(&CN[i], &m.c_rec[n0 + i]);
         stage_word(&XR[i].x, &vsrc[t0 + (t >= 0 ? t : -1 - t)]); stage_word(&XR[i].y, &m.nd_rt[n0 + i]);
     }
-    if (lane == 0) {
+    if (th == 0) {
         XR[n] = make_float2(0.0f, 0.0f);
         CN[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    for (int i = lane; i < 32 * nw; i += 32) {
+    for (int i = th; i < 32 * nw; i += nth) {
         const int t = m.tw_t[32 * w0 + i];
         stage_rec(&TR[i], &m.tw_rec[32 * w0 + i]);
         stage_word(&TA[i], &m.tw_adr[32 * w0 + i]);
         stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
     }
-    for (int i = lane; i < kSlotRecs * nf; i += 32) stage_rec(&NF[i], &m.nf_rec[(size_t)kSlotRecs * nf0 + i]);
-    for (int i = lane; i < nblk; i += 32) stage_rec(&BK[i], &m.bk_rec[ub0 + i]);
-    for (int j = lane; j < nf; j += 32) {
+    for (int i = th; i < kSlotRecs * nf; i += nth) stage_rec(&NF[i], &m.nf_rec[(size_t)kSlotRecs * nf0 + i]);
+    for (int i = th; i < nblk; i += nth) stage_rec(&BK[i], &m.bk_rec[ub0 + i]);
+    for (int j = th; j < nf; j += nth) {
         stage_word(&TS[j].x, &m.nf_ts[nf0 + j].x); stage_word(&TS[j].y, &m.nf_ts[nf0 + j].y);
     }
-    for (int c = lane; c < nch; c += 32) {
+    for (int c = th; c < nch; c += nth) {
         stage_word(&CHG[c], &m.nfc_g[uch0 + c]); stage_word(&CHE[c], &m.nfc_e[uch0 + c]);
         stage_word(&CHQ[c], &m.nfc_q[uch0 + c]); stage_word(&CHI[c], &m.nfc_i[uch0 + c]);
     }
-    for (int i = lane; i < ngt; i += 32) { stage_word(&GT[i], &m.gate[gt0 + i]); stage_word(&GI[i], &m.gt_idx[gt0 + i]); }
-    for (int i = lane; i < np; i += 32) stage_word(&PS[i], &m.ps[ps0 + i]);
-    for (int i = 4 * lane; i < gps * nck; i += 128) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
+    for (int i = th; i < ngt; i += nth) { stage_word(&GT[i], &m.gate[gt0 + i]); stage_word(&GI[i], &m.gt_idx[gt0 + i]); }
+    for (int i = th; i < np; i += nth) stage_word(&PS[i], &m.ps[ps0 + i]);
+    for (int i = 4 * th; i < gps * nck; i += 4 * nth) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
     stage_wait();
-    __syncwarp();
-    for (int j = lane; j < nf; j += 32) VO[j] = XR[__float_as_int(NF[kSlotRecs * j].x) & kPassStart].x;
-    for (int i = lane; i < 32 * nw; i += 32) TX[i] = TV[i] + TR[i].x;  // the first step's pre-update
+    unit_sync();
+    for (int j = th; j < nf; j += nth) VO[j] = XR[__float_as_int(NF[kSlotRecs * j].x) & kPassStart].x;
+    for (int i = th; i < 32 * nw; i += nth) TX[i] = TV[i] + TR[i].x;  // the first step's pre-update
+    unit_sync();
+    const float dt = m.dt;
+    float *Gq = GT, *Gn = GT + ngt;  // gate values at the step's start, and at the next's
+    float4 ga, gb, gc;               // the lane's only gate, where it has no more
+    int gs = 0;
+    // gate updates from step k's starting V and gate values (an instantaneous
+    // gate takes the potential after the step: one warp, after the solve)
+    auto update_gates = [&](int k, const float *Vq) {
+#pragma unroll 1
+        for (int q = lane; q < ngt; q += 32) {
+            if (k == 0 || ngt > 32) {
+                gs = GI[q];
+                const float4 *r = m.gate_tab + kGateRecs * (gs >> 10);
+                ga = r[0]; gb = r[1]; gc = r[2];
+                gs &= kPassStart;
+            }
+            Gn[q] = gate_next_p(ga, gb, gc, m.gate_ext, init, dt, Vq[gs],
+                                EDEN_KIND_GATEFORMS && !pair ? XR[__float_as_int(NF[kSlotRecs * gs].x) & kPassStart].x : 0.0f,
+                                Gq[q]);
+        }
+    };
+    // the lanes' threshold crossings in step k (eden/Eden.cpp:6247-6252)
+    auto threshold = [&](int k, bool slot, const float2 &ts, float vo, float vn) {
+        const bool spk = slot && vo < ts.x && ts.x < vn;
+        if (__any_sync(0xffffffffu, spk)) {
+            // (this step's time, accumulated in double as the host does)
+            double t = w.t0;
+            if (!init)
+                for (int i = 0; i < k; i++) t += (double)dt;
+            push_spike(m, spk, spk ? __float_as_int(ts.y) : -1, (int32_t)(w.step0 + k + 1), w.wpar,
+                       spk ? crossing_time(t, dt, vo, vn, ts.x) : 0.0);
+        }
+    };
+    auto thresholds = [&](int k, const float *Vl, const float *Vq) {
+#pragma unroll 1
+        for (int j0 = 0; j0 < nf; j0 += 32) {
+            const int j = j0 + lane;
+            threshold(k, j < nf, j < nf ? TS[j] : make_float2(0.0f, 0.0f), j < nf ? Vl[j] : 0.0f, j < nf ? Vq[j] : 0.0f);
+        }
+    };
+    if (EDEN_GATE_WARPS && gates) {
+        const float *Vl = nullptr, *Vq = VO;  // the potentials the last step and this one start from
+#pragma unroll 1
+        for (int k = 0; k < w.K; k++) {
+            update_gates(k, Vq);
+            if (k > 0) thresholds(k - 1, Vl, Vq);
+            unit_sync();
+            float *g = Gq;
+            Gq = Gn;
+            Gn = g;
+            Vl = Vq;
+            Vq = Vq == VO + 2 * nf ? VO : Vq + nf;
+        }
+        thresholds(w.K - 1, Vl, Vq);
+        for (int i = lane; i < ngt; i += 32) m.gate[gt0 + i] = Gq[i];
+        return;
+    }
     int p1 = 0;  // the first pass below the roots
     while (p1 < np && (PS[p1] & kPassRoot)) p1++;
     __syncwarp();
-    const float dt = m.dt;
     int row = 0;  // the first step's row of the trajectory buffer
     if (r1 > r0) row = (int)((w.step0 + m.trace_cap - 1) % m.trace_cap);
-    float *Gq = GT, *Gn = GT + ngt;  // gate values at the step's start, and at the next's
-    float4 sa, sb, ga, gb, gc;       // the lane's only slot and gate, where it has no more
+    float4 sa, sb;  // the lane's only slot, where it has no more
     float2 ts;
-    int gs = 0;
+    float *Vq = VO;
 #pragma unroll 1
     for (int k = 0; k < w.K; k++) {
         if (r1 > r0) {
@@ -271,7 +344,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             const int slot = __float_as_int(sa.x), ti = slot & kPassStart;
             const int brange = __float_as_int(sb.y), crange = __float_as_int(sb.z);
             const int ch0 = crange & 0xffff;
-            const float v = VO[j];
+            const float v = Vq[j];
             float Iin, Gin, Isyn, Gsyn;
             block_currents_rec(Gk, gps, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
             // (a model with gap junctions runs one-step windows: vsrc holds
@@ -309,59 +382,44 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             CN[ti].z = d;
             XR[ti].x = x;
         }
-        // gate updates from this step's starting V and gate values; an
-        // instantaneous gate takes the potential after the step, so a model
-        // with other kinds of gates updates them after the solve
-        auto update_gates = [&]() {
-#pragma unroll 1
-            for (int q = lane; q < ngt; q += 32) {
-                if (k == 0 || ngt > 32) {
-                    gs = GI[q];
-                    const float4 *r = m.gate_tab + kGateRecs * (gs >> 10);
-                    ga = r[0]; gb = r[1]; gc = r[2];
-                    gs &= kPassStart;
-                }
-                Gn[q] = gate_next_p(ga, gb, gc, m.gate_ext, init, dt, VO[gs],
-                                    EDEN_KIND_GATEFORMS ? XR[__float_as_int(NF[kSlotRecs * gs].x) & kPassStart].x : 0.0f,
-                                    Gq[q]);
-            }
-        };
-        if (!EDEN_KIND_GATEFORMS) update_gates();
+        if (!EDEN_KIND_GATEFORMS && !pair) update_gates(k, Vq);
         __syncwarp();
         if (!init) {
             // (a double-precision forest has no twigs: its nodes are its compartments)
             if (f64) hines_window_f64(dt, XR, CN, m.c_l + t0, PS, np, n, XD, PVD, RTD);
             else hines_window(dt, S, XR, CN, PS, np, p1, n, TX, TV, TR, TA, nw);
         }
-        if (EDEN_KIND_GATEFORMS) {
-            update_gates();
+        if (EDEN_KIND_GATEFORMS && !pair) {
+            update_gates(k, Vq);
             __syncwarp();
         }
-        // threshold crossings of the unit's spike sources (eden/Eden.cpp:6247-6252),
-        // and V for the next step
+        // V for the next step, and the thresholds if there is no other warp for them
+        if (EDEN_GATE_WARPS) {
+            float *Vn = Vq == VO + 2 * nf ? VO : Vq + nf;
 #pragma unroll 1
-        for (int j0 = 0; j0 < nf; j0 += 32) {
-            const int j = j0 + lane;
-            bool spk = false;
-            float vo = 0.0f, vn = 0.0f;
-            if (j < nf) {
+            for (int j = lane; j < nf; j += 32) {
                 if (nf > 32) sa.x = NF[kSlotRecs * j].x;
-                if (k == 0 || nf > 32) ts = TS[j];
-                vo = VO[j];
-                vn = XR[__float_as_int(sa.x) & kPassStart].x;
-                spk = vo < ts.x && ts.x < vn;
-                VO[j] = vn;
+                Vn[j] = XR[__float_as_int(sa.x) & kPassStart].x;
             }
-            if (__any_sync(0xffffffffu, spk)) {
-                // (this step's time, accumulated in double as the host does)
-                double t = w.t0;
-                if (!init)
-                    for (int i = 0; i < k; i++) t += (double)dt;
-                push_spike(m, spk, spk ? __float_as_int(ts.y) : -1, (int32_t)(w.step0 + k + 1), w.wpar,
-                           spk ? crossing_time(t, dt, vo, vn, ts.x) : 0.0);
+            unit_sync();
+            if (!pair) thresholds(k, Vq, Vn);
+            Vq = Vn;
+        } else {
+#pragma unroll 1
+            for (int j0 = 0; j0 < nf; j0 += 32) {
+                const int j = j0 + lane;
+                float vo = 0.0f, vn = 0.0f;
+                if (j < nf) {
+                    if (nf > 32) sa.x = NF[kSlotRecs * j].x;
+                    if (k == 0 || nf > 32) ts = TS[j];
+                    vo = Vq[j];
+                    vn = XR[__float_as_int(sa.x) & kPassStart].x;
+                    Vq[j] = vn;
+                }
+                threshold(k, j < nf, ts, vo, vn);
             }
+            __syncwarp();
         }
-        __syncwarp();
         float *g = Gq;
         Gq = Gn;
         Gn = g;
@@ -376,7 +434,8 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
         const int t = m.tw_t[32 * w0 + i];
         if (t >= 0) vdst[t0 + t] = TV[i];
     }
-    for (int i = lane; i < ngt; i += 32) m.gate[gt0 + i] = Gq[i];
+    if (!pair)
+        for (int i = lane; i < ngt; i += 32) m.gate[gt0 + i] = Gq[i];
 }
 
 // A batch of up to 32 point neurons over the window (izhikevich2007Cell,
@@ -439,7 +498,10 @@ __device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &
     }
 }
 
-// This launch runs CTAs [cta_begin, cta_end), each a few units, one per warp.
+// This launch runs CTAs [cta_begin, cta_end), each a few units, one per warp of
+// the first half of the block, where units' gates have warps of their own (the
+// other half's, unit by unit, so that each half spreads over the SM's four
+// schedulers), else one per warp.
 // A block runs several CTAs in turn when there are more CTAs than blocks;
 // their units are laid out differently in shared memory, so every warp of
 // the block finishes its unit before any starts on the next CTA.
@@ -448,12 +510,16 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(DevModel m, const W
     extern __shared__ __align__(16) float sm[];
     const WindowArgs w = tab[*base + idx];
     const float *tk = ttab[*base + idx].tk;
+    const int units = EDEN_GATE_WARPS && m.gate_warp ? blockDim.x >> 6 : blockDim.x >> 5;
     const int warp = threadIdx.x >> 5;
+    const bool gates = warp >= units;
+    const int slot = gates ? warp - units : warp;
     for (int cta = cta_begin + blockIdx.x; cta < cta_end; cta += gridDim.x) {
-        const int u = m.cta_u0[cta] + warp;
+        const int u = m.cta_u0[cta] + slot;
         if (u < m.cta_u0[cta + 1]) {
-            if (m.un_f[u] >= 0) { if (EDEN_KIND_FOREST) forest_window(m, w, u, sm + m.un_off[u]); }
-            else if (EDEN_KIND_IZH) izh_window(m, w, tk, u, sm + m.un_off[u]);
+            if (m.un_f[u] >= 0) {
+                if (EDEN_KIND_FOREST) forest_window(m, w, u, sm + m.un_off[u], gates, 1 + slot);
+            } else if (EDEN_KIND_IZH && !gates) izh_window(m, w, tk, u, sm + m.un_off[u]);
         }
         if (cta + (int)gridDim.x < cta_end) __syncthreads();
     }
