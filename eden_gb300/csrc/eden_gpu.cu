@@ -113,6 +113,7 @@ struct EdenGpuCtx {
     int cell_threads = 128;                // threads of a k_cells_t block
     std::vector<int64_t> h_ext_step;       // logging steps of the spike sources' events
     size_t smem_hines = 0, smem_inputs = 0;
+    bool inputs_early = false;             // the input kernel may start while the window before drains
     struct CellClass { int cta_begin, cta_end; size_t smem; };
     std::vector<CellClass> classes;        // k_cells_t launches of one window
     double last_ms = 0.0;
@@ -188,6 +189,23 @@ template <typename... A>
 cudaError_t launch_k(const void *fn, int grid, int block, size_t smem, cudaStream_t s, A... args) {
     void *argv[] = {(void *)&args...};
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), argv, smem, s);
+}
+// Launch of a window's kernel, which may start while the one before it drains
+// where `early` (kernel_order).
+template <typename... A>
+cudaError_t launch_order(bool early, const void *fn, int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    void *argv[] = {(void *)&args...};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, fn, argv);
 }
 }  // namespace
 
@@ -1888,6 +1906,13 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         ctx->grid_inputs = (int)std::max<int64_t>(
             1, std::min<int64_t>(((int64_t)ctx->d.n_chunk * 32 + kInputThreads - 1) / kInputThreads,
                                  (int64_t)ctx->n_sm * std::max(per_sm, 1)));
+        // A window's kernels start while the one before drains: a step of 600
+        // cells with gap junctions 14.1 us, 11.0 so, of the per-step kernels with
+        // 1,000 trees 45.5 and 38.0, a window of 31 steps of 1,000 HH cells 42.5
+        // and 39.7.  Not the first of a window where its blocks fill every SM:
+        // 100,000 izhikevich neurons took 22.2 us a step with it early, 19.5
+        // without (and the others gain nothing there: 10,000 trees 9.78 and 9.81).
+        ctx->inputs_early = ctx->grid_inputs < ctx->n_sm * std::max(per_sm, 1);
     }
     phase("done");
     if (verbose) {
@@ -2074,36 +2099,38 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
     cudaStream_t s = ctx->stream;
     if (ctx->mode == EDEN_MODE_BATCHED && ctx->smem_window) {
         tmark(ctx, EDEN_KERNEL_INPUTS, true);
-        launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d, (const WindowArgs *)ctx->d_wtab,
-                 (const WindowTimes *)ctx->d_wtimes, base, idx);
+        launch_order(ctx->inputs_early, ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d,
+                     (const WindowArgs *)ctx->d_wtab, (const WindowTimes *)ctx->d_wtimes, base, idx);
         tmark(ctx, EDEN_KERNEL_INPUTS, false);
         int n = 1;
         tmark(ctx, EDEN_KERNEL_CELLS, true);
         for (const auto &cl : ctx->classes) {
             const int nb = std::min(cl.cta_end - cl.cta_begin, ctx->max_cell_blocks);
-            launch_k(ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
+            launch_order(true, ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
                      (const WindowTimes *)ctx->d_wtimes, base, idx, cl.cta_begin, cl.cta_end);
             n++;
         }
         tmark(ctx, EDEN_KERNEL_CELLS, false);
         tmark(ctx, EDEN_KERNEL_DELIVER, true);
-        launch_k(ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab, base, idx);
+        launch_order(true, ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab, base, idx);
         tmark(ctx, EDEN_KERNEL_DELIVER, false);
         return n + 1;
     }
     (void)K;
     tmark(ctx, EDEN_KERNEL_INPUTS, true);
-    launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d, (const WindowArgs *)ctx->d_wtab,
-             (const WindowTimes *)ctx->d_wtimes, base, idx);
+    launch_order(ctx->inputs_early, ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, d,
+                 (const WindowArgs *)ctx->d_wtab, (const WindowTimes *)ctx->d_wtimes, base, idx);
     tmark(ctx, EDEN_KERNEL_INPUTS, false);
     tmark(ctx, EDEN_KERNEL_TARGETS, true);
-    k_targets_t<<<ctx->grid_targets, kThreads, 0, s>>>(d, ctx->d_wtab, ctx->d_wtimes, base, idx);
+    launch_order(true, (const void *)k_targets_t, ctx->grid_targets, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab,
+                 (const WindowTimes *)ctx->d_wtimes, base, idx);
     tmark(ctx, EDEN_KERNEL_TARGETS, false);
     tmark(ctx, EDEN_KERNEL_HINES, true);
-    k_hines_t<<<ctx->grid_hines, kHinesThreads, ctx->smem_hines, s>>>(d, ctx->d_wtab, base, idx, ctx->forest_cap);
+    launch_order(true, (const void *)k_hines_t, ctx->grid_hines, kHinesThreads, ctx->smem_hines, s, d,
+                 (const WindowArgs *)ctx->d_wtab, base, idx, ctx->forest_cap);
     tmark(ctx, EDEN_KERNEL_HINES, false);
     tmark(ctx, EDEN_KERNEL_DELIVER, true);
-    launch_k(ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab, base, idx);
+    launch_order(true, ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab, base, idx);
     tmark(ctx, EDEN_KERNEL_DELIVER, false);
     return 4;
 }

@@ -18,8 +18,20 @@ constexpr int kHinesThreads = 128;  // k_hines_t: four warps, each staging one f
 // ---------------------------------------------------------------------------
 // kernels; each reads its WindowArgs from a device table so that a captured
 // graph can be replayed over many windows
+//
+// edenGpuRun launches a window's kernels so that each may start while the one
+// before it drains: `kernel_order` waits until everything before has finished
+// and is visible, and only then lets the next kernel start, so that one kernel
+// at most is ahead of the running one.  Before it a kernel reads nothing but
+// its arguments, the window tables and the model's constants, which no kernel of
+// a window writes.  (Launched without that allowance, it does not wait.)
 // ---------------------------------------------------------------------------
 namespace eden {
+
+__device__ __forceinline__ void kernel_order() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // Phase 1 of both paths: input blocks over the window (the per-step path runs
 // it with K = 1), a warp per group of consecutive chunks.  A group grows past
@@ -34,6 +46,7 @@ __global__ void __launch_bounds__(kInputThreads, 8) k_inputs_t(DevModel m, const
     __shared__ float tk[64];  // the window's step times, then the previous window's
     const int wi = *base + idx;
     const WindowArgs w = tab[wi];
+    kernel_order();
     if (threadIdx.x < 64) tk[threadIdx.x] = threadIdx.x < 32 ? ttab[wi].tk[threadIdx.x] : ttab[wi].tprev[threadIdx.x - 32];
     __syncthreads();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -50,6 +63,7 @@ __global__ void __launch_bounds__(256) k_targets_t(DevModel m, const WindowArgs 
                                                    const int *base, int idx) {
     const WindowArgs w = tab[*base + idx];
     const float tnow = ttab[*base + idx].tk[0];
+    kernel_order();
     const bool init = w.step0 <= 0;
     const float *vin = m.v[w.par];
     float *vout = m.v[w.par ^ 1];
@@ -72,6 +86,7 @@ __global__ void __launch_bounds__(256) k_targets_t(DevModel m, const WindowArgs 
 __global__ void __launch_bounds__(kHinesThreads) k_hines_t(DevModel m, const WindowArgs *tab, const int *base, int idx, int cap) {
     extern __shared__ float sm[];
     const WindowArgs w = tab[*base + idx];
+    kernel_order();
     const bool init = w.step0 <= 0;
     const float *vin = m.v[w.par];
     float *x = m.v[w.par ^ 1];
@@ -116,6 +131,7 @@ __global__ void __launch_bounds__(kHinesThreads) k_hines_t(DevModel m, const Win
 // the trigger, eden/Eden.cpp:3964-3992) and append them to the spike log.
 __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs *tab, const int *base, int idx) {
     const WindowArgs w = tab[*base + idx];
+    kernel_order();
     const int wp = w.wpar;
     const int n = m.wspk_count[wp];
     const int lane = threadIdx.x & 31;
@@ -184,7 +200,7 @@ __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs 
 // the loop that takes V over; with them, one body for both roles: compiled
 // apart, the solve of 50 trees took 112 us a window instead of 100.)
 __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S, bool gates,
-                                              int barrier) {
+                                              int barrier, bool first) {
     const int lane = threadIdx.x & 31;
     const int t0 = m.un_t0[u], fi = m.un_f[u], ub0 = m.t_blk0[t0], nblk = m.t_blk0[m.un_t1[u]] - ub0;
     const int n0 = m.fo_n0[fi], n = m.fo_n0[fi + 1] - n0, w0 = m.fo_w0[fi], nw = m.fo_w0[fi + 1] - w0;
@@ -223,22 +239,19 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     double *PVD = XD + n, *RTD = PVD + n;
     // the steps of a window are all initialisation passes or none is
     const bool init = w.step0 <= 0;
-    // ---- stage the unit
-    const float *vsrc = m.v[w.par];
+    // ---- stage the unit: its records first, which are there before the window's
+    // inputs, then what earlier kernels wrote
     for (int i = th; i < n; i += nth) {
-        const int t = m.nd_t[n0 + i];
         stage_rec(&CN[i], &m.c_rec[n0 + i]);
-        stage_word(&XR[i].x, &vsrc[t0 + (t >= 0 ? t : -1 - t)]); stage_word(&XR[i].y, &m.nd_rt[n0 + i]);
+        stage_word(&XR[i].y, &m.nd_rt[n0 + i]);
     }
     if (th == 0) {
         XR[n] = make_float2(0.0f, 0.0f);
         CN[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     for (int i = th; i < 32 * nw; i += nth) {
-        const int t = m.tw_t[32 * w0 + i];
         stage_rec(&TR[i], &m.tw_rec[32 * w0 + i]);
         stage_word(&TA[i], &m.tw_adr[32 * w0 + i]);
-        stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
     }
     for (int i = th; i < kSlotRecs * nf; i += nth) stage_rec(&NF[i], &m.nf_rec[(size_t)kSlotRecs * nf0 + i]);
     for (int i = th; i < nblk; i += nth) stage_rec(&BK[i], &m.bk_rec[ub0 + i]);
@@ -249,8 +262,19 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
         stage_word(&CHG[c], &m.nfc_g[uch0 + c]); stage_word(&CHE[c], &m.nfc_e[uch0 + c]);
         stage_word(&CHQ[c], &m.nfc_q[uch0 + c]); stage_word(&CHI[c], &m.nfc_i[uch0 + c]);
     }
-    for (int i = th; i < ngt; i += nth) { stage_word(&GT[i], &m.gate[gt0 + i]); stage_word(&GI[i], &m.gt_idx[gt0 + i]); }
+    for (int i = th; i < ngt; i += nth) stage_word(&GI[i], &m.gt_idx[gt0 + i]);
     for (int i = th; i < np; i += nth) stage_word(&PS[i], &m.ps[ps0 + i]);
+    if (first) kernel_order();
+    const float *vsrc = m.v[w.par];
+    for (int i = th; i < n; i += nth) {
+        const int t = m.nd_t[n0 + i];
+        stage_word(&XR[i].x, &vsrc[t0 + (t >= 0 ? t : -1 - t)]);
+    }
+    for (int i = th; i < 32 * nw; i += nth) {
+        const int t = m.tw_t[32 * w0 + i];
+        stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
+    }
+    for (int i = th; i < ngt; i += nth) stage_word(&GT[i], &m.gate[gt0 + i]);
     for (int i = 4 * th; i < gps * nck; i += 4 * nth) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
     stage_wait();
     unit_sync();
@@ -440,7 +464,8 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
 
 // A batch of up to 32 point neurons over the window (izhikevich2007Cell,
 // iaf*Cell, adExIaFCell; point_update), one lane each.
-__device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &w, const float *tk, int u, float *S) {
+__device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &w, const float *tk, int u, float *S,
+                                           bool first) {
     const int lane = threadIdx.x & 31;
     const int t0 = m.un_t0[u], n = m.un_t1[u] - t0;
     const int r0 = m.un_r0[u], r1 = m.un_r1[u];
@@ -451,11 +476,15 @@ __device__ __forceinline__ void izh_window(const DevModel &m, const WindowArgs &
     const int izh0 = m.t_izh[t0];
     for (int i = lane; i < n; i += 32) {
         const int iz = izh0 + i;
-        stage_word(&S[w.par * n + i], &m.v[w.par][t0 + i]);
         for (int f = 0; f < EDEN_POINT_PARAMS; f++) stage_word(&P[f * n + i], &m.iz_p[(size_t)f * m.n_izh + iz]);
+        stage_word(&KIND[i], &m.iz_kind[iz]);
+    }
+    if (first) kernel_order();
+    for (int i = lane; i < n; i += 32) {
+        const int iz = izh0 + i;
+        stage_word(&S[w.par * n + i], &m.v[w.par][t0 + i]);
         stage_word(&SU[i], &m.iz_u[iz]);
         stage_word(&SS[i], &m.iz_s[iz]);
-        stage_word(&KIND[i], &m.iz_kind[iz]);
     }
     stage_wait();
     __syncwarp();
@@ -515,11 +544,12 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(DevModel m, const W
     const bool gates = warp >= units;
     const int slot = gates ? warp - units : warp;
     for (int cta = cta_begin + blockIdx.x; cta < cta_end; cta += gridDim.x) {
+        const bool first = cta == cta_begin + (int)blockIdx.x;
         const int u = m.cta_u0[cta] + slot;
         if (u < m.cta_u0[cta + 1]) {
             if (m.un_f[u] >= 0) {
-                if (EDEN_KIND_FOREST) forest_window(m, w, u, sm + m.un_off[u], gates, 1 + slot);
-            } else if (EDEN_KIND_IZH && !gates) izh_window(m, w, tk, u, sm + m.un_off[u]);
+                if (EDEN_KIND_FOREST) forest_window(m, w, u, sm + m.un_off[u], gates, 1 + slot, first);
+            } else if (EDEN_KIND_IZH && !gates) izh_window(m, w, tk, u, sm + m.un_off[u], first);
         }
         if (cta + (int)gridDim.x < cta_end) __syncthreads();
     }
