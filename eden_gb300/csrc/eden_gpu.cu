@@ -112,6 +112,11 @@ struct EdenGpuCtx {
     int max_cell_blocks = 0;               // most blocks of a k_cells_t launch
     int cell_threads = 128;                // threads of a k_cells_t block
     std::vector<int64_t> h_ext_step;       // logging steps of the spike sources' events
+    struct Slab {
+        char *dev;
+        std::vector<char> host;
+    };
+    std::vector<Slab> slabs;               // arrays of the context not yet on the device (upload)
     size_t smem_hines = 0, smem_inputs = 0;
     bool inputs_early = false;             // the input kernel may start while the window before drains
     struct CellClass { int cta_begin, cta_end; size_t smem; };
@@ -212,10 +217,44 @@ cudaError_t launch_order(bool early, const void *fn, int grid, int block, size_t
 // ---------------------------------------------------------------------------
 namespace {
 
+// A context's arrays: a hundred, most of them small.  Those up to kSlabArray
+// bytes lie side by side in slabs, each one allocation, filled on the host and
+// copied once (flush_slabs); until then nothing else may write or read them.  (A
+// context of 100 cells, with an allocation and a copy for each array: 1.6 ms to
+// create and 0.68 to destroy; 0.75 and 0.39 so.)
+constexpr size_t kSlabArray = 256 << 10, kSlabBytes = 1 << 20;
+
+int slab_place(EdenGpuCtx *ctx, void **p, const void *src, size_t n, size_t bytes) {
+    if (ctx->slabs.empty() || ctx->slabs.back().host.size() + bytes > kSlabBytes) {
+        void *dev = nullptr;
+        CUDA_TRY(ctx, cudaMalloc(&dev, kSlabBytes));
+        ctx->allocs.push_back(dev);
+        ctx->slabs.push_back({(char *)dev, {}});
+        ctx->slabs.back().host.reserve(kSlabBytes);
+    }
+    EdenGpuCtx::Slab &s = ctx->slabs.back();
+    const size_t at = s.host.size();
+    s.host.resize(at + ((bytes + 255) & ~(size_t)255));  // (zeroed)
+    if (n) memcpy(s.host.data() + at, src, n);
+    *p = s.dev + at;
+    return 0;
+}
+
+int flush_slabs(EdenGpuCtx *ctx) {
+    for (auto &s : ctx->slabs) CUDA_TRY(ctx, cudaMemcpy(s.dev, s.host.data(), s.host.size(), cudaMemcpyHostToDevice));
+    ctx->slabs.clear();
+    return 0;
+}
+
 template <typename T>
 int upload(EdenGpuCtx *ctx, T **dst, const T *src, size_t n) {
     size_t bytes = sizeof(T) * (n > 0 ? n : 1);
     void *p = nullptr;
+    if (bytes <= kSlabArray) {
+        const int rc = slab_place(ctx, &p, src, src ? sizeof(T) * n : 0, bytes);
+        *dst = (T *)p;
+        return rc;
+    }
     CUDA_TRY(ctx, cudaMalloc(&p, bytes));
     ctx->allocs.push_back(p);
     if (src && n) {
@@ -474,7 +513,6 @@ extern "C" void edenGpuDestroy(EdenGpuCtx *ctx) {
     for (void *p : ctx->allocs) cudaFree(p);
     for (cudaEvent_t e : ctx->tev) cudaEventDestroy(e);
     if (ctx->h_wtab) cudaFreeHost(ctx->h_wtab);
-    if (ctx->h_wtimes) cudaFreeHost(ctx->h_wtimes);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1689,14 +1727,12 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload(ctx, &d.tm_a, (const float *)nullptr, (size_t)m->n_timed));
     TRY(upload(ctx, &d.tm_b, (const float *)nullptr, (size_t)m->n_timed));
     TRY(upload(ctx, &d.tm_last, (const int32_t *)nullptr, (size_t)m->n_timed));
-    TRY(upload(ctx, &d.tm_cur, (const int64_t *)nullptr, (size_t)m->n_timed));
     TRY(upload_c(ctx, &d.tm_w, tm_w)); TRY(upload_c(ctx, &d.tm_type, tm_type));
     TRY(upload_c(ctx, &d.tm_off, tm_off)); TRY(upload_c(ctx, &d.tm_step, tm_step));
     {
         // each item's cursor starts at its first listed step
         std::vector<int64_t> cur(tm_off.begin(), tm_off.end() - 1);
-        if (!cur.empty())
-            CUDA_TRY(ctx, cudaMemcpy(d.tm_cur, cur.data(), sizeof(int64_t) * cur.size(), cudaMemcpyHostToDevice));
+        TRY(upload_vec(ctx, &d.tm_cur, cur));
     }
     TRY(upload(ctx, &d.sy_a, (const float *)nullptr, (size_t)ns));
     {
@@ -1914,6 +1950,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         // without (and the others gain nothing there: 10,000 trees 9.78 and 9.81).
         ctx->inputs_early = ctx->grid_inputs < ctx->n_sm * std::max(per_sm, 1);
     }
+    TRY(flush_slabs(ctx));
     phase("done");
     if (verbose) {
         fprintf(stderr, "libeden_gpu: set-up %s\n", timing.c_str());
@@ -1976,24 +2013,24 @@ static int ensure_wtab(EdenGpuCtx *ctx, int64_t n) {
         cudaGraphExecDestroy(ctx->graph);
         ctx->graph = nullptr;
     }
+    // (both tables in one allocation)
+    ctx->wtab_cap = 0;
+    static_assert(sizeof(WindowArgs) % alignof(WindowTimes) == 0, "tables side by side");
     if (ctx->h_wtab) cudaFreeHost(ctx->h_wtab);
-    if (ctx->h_wtimes) cudaFreeHost(ctx->h_wtimes);
     ctx->h_wtab = nullptr;
     ctx->h_wtimes = nullptr;
-    for (void *old : {(void *)ctx->d_wtab, (void *)ctx->d_wtimes}) {
-        if (!old) continue;
-        cudaFree(old);
-        ctx->allocs.erase(std::remove(ctx->allocs.begin(), ctx->allocs.end(), old), ctx->allocs.end());
+    if (ctx->d_wtab) {
+        cudaFree(ctx->d_wtab);
+        ctx->allocs.erase(std::remove(ctx->allocs.begin(), ctx->allocs.end(), (void *)ctx->d_wtab), ctx->allocs.end());
+        ctx->d_wtab = nullptr;
     }
-    CUDA_TRY(ctx, cudaMallocHost(&ctx->h_wtab, sizeof(WindowArgs) * cap));
-    CUDA_TRY(ctx, cudaMallocHost(&ctx->h_wtimes, sizeof(WindowTimes) * cap));
-    void *p = nullptr, *q = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&p, sizeof(WindowArgs) * cap));
+    CUDA_TRY(ctx, cudaMallocHost(&ctx->h_wtab, (sizeof(WindowArgs) + sizeof(WindowTimes)) * cap));
+    ctx->h_wtimes = (WindowTimes *)(ctx->h_wtab + cap);
+    void *p = nullptr;
+    CUDA_TRY(ctx, cudaMalloc(&p, (sizeof(WindowArgs) + sizeof(WindowTimes)) * cap));
     ctx->allocs.push_back(p);
-    CUDA_TRY(ctx, cudaMalloc(&q, sizeof(WindowTimes) * cap));
-    ctx->allocs.push_back(q);
     ctx->d_wtab = (WindowArgs *)p;
-    ctx->d_wtimes = (WindowTimes *)q;
+    ctx->d_wtimes = (WindowTimes *)(ctx->d_wtab + cap);
     ctx->wtab_cap = cap;
     return 0;
 }
@@ -2356,17 +2393,17 @@ static int sort_log(EdenGpuCtx *ctx, int64_t n, int64_t first, int64_t end, bool
     };
     if (words > ctx->log_words) {
         ctx->log_words = 0;
-        TRY(grow((void **)&ctx->log_bits, sizeof(uint32_t) * words));
-        TRY(grow((void **)&ctx->log_before, sizeof(uint32_t) * words));
-        TRY(grow((void **)&ctx->log_blocks, sizeof(uint32_t) * (nblk + 1)));
+        TRY(grow((void **)&ctx->log_bits, sizeof(uint32_t) * (2 * words + nblk + 1)));
+        ctx->log_before = ctx->log_bits + words;
+        ctx->log_blocks = ctx->log_before + words;
         ctx->log_words = words;
     }
     if (n > ctx->sorted_cap) {
         const int64_t cap = std::min<int64_t>(d.log_cap, std::max<int64_t>(2 * n, 1 << 16));
         ctx->sorted_cap = 0;
-        TRY(grow((void **)&ctx->sorted_src, sizeof(int32_t) * cap));
-        TRY(grow((void **)&ctx->sorted_step, sizeof(int64_t) * cap));
-        TRY(grow((void **)&ctx->sorted_time, sizeof(double) * cap));
+        TRY(grow((void **)&ctx->sorted_step, (sizeof(int64_t) + sizeof(double) + sizeof(int32_t)) * cap));
+        ctx->sorted_time = (double *)(ctx->sorted_step + cap);
+        ctx->sorted_src = (int32_t *)(ctx->sorted_time + cap);
         ctx->sorted_cap = cap;
     }
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->n_sm * 16);
