@@ -1248,6 +1248,12 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         if (m->src_target[s] >= 0) t_src[u2i[m->src_target[s]]] = s;
         src_thr[s] = m->src_threshold[s];
     }
+    std::vector<int32_t> fo_s0(1, 0), fo_s;
+    for (size_t f = 0; f < fo_t0.size(); f++) {
+        for (int t = fo_t0[f]; t < fo_t1[f]; t++)
+            if (t_src[t] >= 0) fo_s.push_back(t);
+        fo_s0.push_back((int32_t)fo_s.size());
+    }
     phase("blocks");
     // input blocks per target: pulses, then Poisson runs, timed-input runs, then synapse runs of one type
     std::vector<int32_t> t_blk0(nt + 1, 0);
@@ -1657,6 +1663,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload_c(ctx, &d.fo_p0, fo_p0)); TRY(upload_c(ctx, &d.ps, ps));
     // double-precision forests: flags and the per-step path's double scratch
     TRY(upload_c(ctx, &d.fo_f64, fo_f64));
+    TRY(upload_c(ctx, &d.fo_s0, fo_s0)); TRY(upload_c(ctx, &d.fo_s, fo_s));
     TRY(upload(ctx, &d.dscr, (const double *)nullptr, ctx->n_f64_cells > 0 ? (size_t)2 * nt : (size_t)1));
     {
         // gap-junction ends per internal target, in the model's order

@@ -207,6 +207,8 @@ struct DevModel {
     uint32_t *sy_mask;
     const float *sy_w, *sy_delay;
     const uint8_t *sy_type;
+    // the targets of forest f that spike sources watch, fo_s[fo_s0[f] .. fo_s0[f + 1])
+    const int32_t *fo_s0, *fo_s;
     // spike sources and fan-out (source -> synapses, connection order)
     const int32_t *t_src;
     const float *src_thr;
@@ -1453,22 +1455,51 @@ __device__ __forceinline__ void target_step(const DevModel &m, int t, bool init,
 // ---------------------------------------------------------------------------
 // cable solve
 // ---------------------------------------------------------------------------
+// A lane's spike source of a forest: its target, its threshold.
+struct ForestSource {
+    int t = -1, src = -1;
+    float thr = 0.0f;
+};
+__device__ __forceinline__ ForestSource forest_source(const DevModel &m, int q, int end) {
+    ForestSource s;
+    if (q < end) {
+        s.t = m.fo_s[q];
+        s.src = m.t_src[s.t];
+        s.thr = m.src_thr[s.src];
+    }
+    return s;
+}
+
+// The threshold test V < thr < V_next of forest f's spike sources (eden/Eden.cpp:
+// 6247-6252), s the lane's first; `base`: the target at index 0 of Vin and X.
+__device__ __forceinline__ void forest_spikes(const DevModel &m, int f, ForestSource s, int64_t step, double tstep,
+                                              const float *X, const float *Vin, int base, int wpar) {
+    const int lane = threadIdx.x & 31, end = m.fo_s0[f + 1];
+    for (int q = m.fo_s0[f]; q < end; q += 32) {
+        if (q > m.fo_s0[f]) s = forest_source(m, q + lane, end);
+        bool spk = false;
+        double tc = 0.0;
+        if (s.src >= 0) {
+            const float v = Vin[s.t - base], vn = X[s.t - base];
+            spk = v < s.thr && s.thr < vn;
+            if (spk) tc = crossing_time(tstep, m.dt, v, vn, s.thr);
+        }
+        push_spike(m, spk, s.src, (int32_t)(step + 1), wpar, tc);
+    }
+}
+
 // Backward-Euler Hines solve of one forest by one warp (eden/Eden.cpp:6114-6225).
 // Arrays may live in shared or global memory and share one index space:
 // D (diagonal, in), X (the pre-updated V, solved in place), U, L
 // (off-diagonals), CE (end of each node's child range), P (parent), and LV
-// (the forest's depth boundaries, nlev + 1 entries); `base` maps that index
-// space back to internal target ids for the spike check.  Depths are
+// (the forest's depth boundaries, nlev + 1 entries).  Depths are
 // processed deepest first; each node pulls its children's elimination terms
 // in increasing child order, the same sequence of operations as the
 // reference's depth-first post-order, and keeps the reciprocal of its final
-// pivot.  Back-substitution then runs root-first.  When check_spikes is set
-// it ends with the threshold test V < thr < V_next of the forest's spike
-// sources (eden/Eden.cpp:6247-6252).
-__device__ __forceinline__ void hines_forest(const DevModel &m, bool init, int64_t step, double tstep, float *D,
-                                             float *X, const float *U, const float *L, const int32_t *CE,
-                                             const int32_t *P, const int32_t *LV, int nlev, const float *Vin, int base,
-                                             int wpar, bool check_spikes) {
+// pivot.  Back-substitution then runs root-first.
+__device__ __forceinline__ void hines_forest(const DevModel &m, bool init, float *D, float *X, const float *U,
+                                             const float *L, const int32_t *CE, const int32_t *P, const int32_t *LV,
+                                             int nlev) {
     const int lane = threadIdx.x & 31;
     const int c0 = LV[0], c1 = LV[nlev];
     if (!init && c1 > c0) {
@@ -1501,22 +1532,6 @@ __device__ __forceinline__ void hines_forest(const DevModel &m, bool init, int64
             __syncwarp();
         }
     }
-    if (!check_spikes) return;
-    for (int c0w = c0; c0w < c1; c0w += 32) {
-        const int c = c0w + lane;
-        bool spk = false;
-        int src = -1;
-        double tc = 0.0;
-        if (c < c1) {
-            src = m.t_src[c + base];
-            if (src >= 0) {
-                const float thr = m.src_thr[src];
-                spk = (Vin[c] < thr && thr < X[c]);
-                if (spk) tc = crossing_time(tstep, m.dt, Vin[c], X[c], thr);
-            }
-        }
-        push_spike(m, spk, src, (int32_t)(step + 1), wpar, tc);
-    }
 }
 
 // The same solve in double precision for a forest whose rows may lose
@@ -1524,10 +1539,9 @@ __device__ __forceinline__ void hines_forest(const DevModel &m, bool init, int64
 // forest's double scratch): the pre-updated V and diagonal terms stay the
 // single-precision values the step computed, the elimination and the
 // back-substitution carry doubles, and X receives V_next rounded once.
-__device__ __forceinline__ void hines_forest_f64(const DevModel &m, bool init, int64_t step, double tstep,
-                                                 const float *D, float *X, const float *U, const float *L,
-                                                 const int32_t *CE, const int32_t *P, const int32_t *LV, int nlev,
-                                                 const float *Vin, double *XD, double *DD, int wpar) {
+__device__ __forceinline__ void hines_forest_f64(const DevModel &m, bool init, const float *D, float *X, const float *U,
+                                                 const float *L, const int32_t *CE, const int32_t *P, const int32_t *LV,
+                                                 int nlev, double *XD, double *DD) {
     const int lane = threadIdx.x & 31;
     const int c0 = LV[0], c1 = LV[nlev];
     if (!init && c1 > c0) {
@@ -1561,21 +1575,6 @@ __device__ __forceinline__ void hines_forest_f64(const DevModel &m, bool init, i
         }
         for (int c = c0 + lane; c < c1; c += 32) X[c] = (float)XD[c];
         __syncwarp();
-    }
-    for (int c0w = c0; c0w < c1; c0w += 32) {
-        const int c = c0w + lane;
-        bool spk = false;
-        int src = -1;
-        double tc = 0.0;
-        if (c < c1) {
-            src = m.t_src[c];
-            if (src >= 0) {
-                const float thr = m.src_thr[src];
-                spk = (Vin[c] < thr && thr < X[c]);
-                if (spk) tc = crossing_time(tstep, m.dt, Vin[c], X[c], thr);
-            }
-        }
-        push_spike(m, spk, src, (int32_t)(step + 1), wpar, tc);
     }
 }
 

@@ -63,6 +63,20 @@ __global__ void __launch_bounds__(256) k_targets_t(DevModel m, const WindowArgs 
                                                    const int *base, int idx) {
     const WindowArgs w = tab[*base + idx];
     const float tnow = ttab[*base + idx].tk[0];
+    // the constants of the thread's first target into L1 before the wait
+    {
+        const int i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i < m.n_target) {
+            auto fetch = [](const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); };
+            const int b0 = m.t_blk0[i], b1 = m.t_blk0[i + 1], h0 = m.c_chan0[i], h1 = m.c_chan0[i + 1];
+            fetch(&m.t_izh[i]); fetch(&m.t_trace0[i]);
+            fetch(&m.c_area[i]); fetch(&m.c_cm[i]); fetch(&m.c_inv_rc[i]);
+            if (b1 > b0) { fetch(&m.bk_kind[b0]); fetch(&m.bk_erev[b0]); fetch(&m.bk_c0[b0]); }
+            if (h1 > h0) {
+                fetch(&m.ch_type[h0]); fetch(&m.ch_gate0[h0]); fetch(&m.ch_gbase[h0]); fetch(&m.ch_erev[h0]);
+            }
+        }
+    }
     kernel_order();
     const bool init = w.step0 <= 0;
     const float *vin = m.v[w.par];
@@ -86,7 +100,6 @@ __global__ void __launch_bounds__(256) k_targets_t(DevModel m, const WindowArgs 
 __global__ void __launch_bounds__(kHinesThreads) k_hines_t(DevModel m, const WindowArgs *tab, const int *base, int idx, int cap) {
     extern __shared__ float sm[];
     const WindowArgs w = tab[*base + idx];
-    kernel_order();
     const bool init = w.step0 <= 0;
     const float *vin = m.v[w.par];
     float *x = m.v[w.par ^ 1];
@@ -97,32 +110,47 @@ __global__ void __launch_bounds__(kHinesThreads) k_hines_t(DevModel m, const Win
     int32_t *sCE = (int32_t *)(sV + cap), *sP = sCE + cap, *sLV = sP + cap;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    // What no kernel writes -- a forest's off-diagonals, its tree, its spike
+    // sources -- is loaded before the wait, beside the kernel of the targets.
+    // Bound by a step's chain of depths; a test of every compartment for a
+    // source took five rounds of loads after it.  (1,000 trees, a step of all four
+    // kernels: 38.0 us, 35.2 so and with the targets' constants fetched early.)
+    bool waited = false;
     for (int f = warp; f < m.n_forest; f += nwarps) {
         const int c0 = m.fo_t0[f], n = m.fo_t1[f] - c0, nlev = m.fo_nlev[f];
         const int32_t *lv = m.lvl + m.fo_l0[f];
-        if (m.fwd_euler) {
-            // V_next is final already: only the threshold test
-            hines_forest(m, true, w.step0, w.t0, m.diag, x, m.c_u, m.c_l, m.c_cend, m.c_parent, lv, nlev, vin, 0,
-                         w.wpar, true);
-        } else if (m.fo_f64[f]) {
-            hines_forest_f64(m, init, w.step0, w.t0, m.diag, x, m.c_u, m.c_l, m.c_cend, m.c_parent, lv, nlev, vin,
-                             m.dscr, m.dscr + m.n_target, w.wpar);
-        } else if (n <= cap && nlev < cap) {
+        const bool staged = !m.fwd_euler && !m.fo_f64[f] && n <= cap && nlev < cap;
+        if (staged) {
             for (int i = lane; i < n; i += 32) {
-                sD[i] = m.diag[c0 + i]; sX[i] = x[c0 + i]; sU[i] = m.c_u[c0 + i];
-                sL[i] = m.c_l[c0 + i]; sV[i] = vin[c0 + i];
+                sU[i] = m.c_u[c0 + i]; sL[i] = m.c_l[c0 + i];
                 sCE[i] = m.c_cend[c0 + i] - c0; sP[i] = m.c_parent[c0 + i] - c0;
             }
             for (int i = lane; i <= nlev; i += 32) sLV[i] = lv[i] - c0;
+        }
+        const ForestSource src = forest_source(m, m.fo_s0[f] + lane, m.fo_s0[f + 1]);
+        if (!waited) kernel_order();
+        waited = true;
+        if (m.fwd_euler) {
+            // V_next is final already: only the threshold test
+        } else if (m.fo_f64[f]) {
+            hines_forest_f64(m, init, m.diag, x, m.c_u, m.c_l, m.c_cend, m.c_parent, lv, nlev, m.dscr,
+                             m.dscr + m.n_target);
+        } else if (staged) {
+            for (int i = lane; i < n; i += 32) {
+                sD[i] = m.diag[c0 + i]; sX[i] = x[c0 + i]; sV[i] = vin[c0 + i];
+            }
             __syncwarp();
-            hines_forest(m, init, w.step0, w.t0, sD, sX, sU, sL, sCE, sP, sLV, nlev, sV, c0, w.wpar, true);
+            hines_forest(m, init, sD, sX, sU, sL, sCE, sP, sLV, nlev);
             __syncwarp();
             for (int i = lane; i < n; i += 32) x[c0 + i] = sX[i];
+            forest_spikes(m, f, src, w.step0, w.t0, sX, sV, c0, w.wpar);
             __syncwarp();
+            continue;
         } else {
-            hines_forest(m, init, w.step0, w.t0, m.diag, x, m.c_u, m.c_l, m.c_cend, m.c_parent, lv, nlev, vin, 0, w.wpar,
-                         true);
+            hines_forest(m, init, m.diag, x, m.c_u, m.c_l, m.c_cend, m.c_parent, lv, nlev);
         }
+        __syncwarp();
+        forest_spikes(m, f, src, w.step0, w.t0, x, vin, 0, w.wpar);
     }
 }
 
