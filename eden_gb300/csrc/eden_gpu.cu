@@ -5,12 +5,13 @@
 // cell groups for the windowed kernel) and uploads it.  edenGpuRun advances
 // the network: per step (EDEN_MODE_PLAIN: four launches a step, as the
 // reference runs one OpenMP pass a step) or in windows of K steps
-// (EDEN_MODE_BATCHED: one k_window + one k_deliver per window, replayed from
-// a captured CUDA graph).
+// (EDEN_MODE_BATCHED: k_inputs_t, k_cells_t and k_deliver_t per window, replayed
+// from a captured CUDA graph); a kernel may start while the one before it drains.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -119,6 +120,7 @@ struct EdenGpuCtx {
     std::vector<Slab> slabs;               // arrays of the context not yet on the device (upload)
     size_t smem_hines = 0, smem_inputs = 0;
     bool inputs_early = false;             // the input kernel may start while the window before drains
+    bool cells_early = false;              // the cell kernel may start while the input kernel drains
     struct CellClass { int cta_begin, cta_end; size_t smem; };
     std::vector<CellClass> classes;        // k_cells_t launches of one window
     double last_ms = 0.0;
@@ -906,7 +908,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         });
     }
 
-    // windowed-path constants (see DevModel::c_kl): a compartment is flat when
+    // windowed-path constants (a unit's node and twig records): a compartment is flat when
     // it has one gateless channel and no inputs, is no spike source, and every
     // compartment below it is flat; its pivot and elimination factor are then
     // the same every step and are computed here once, deepest first
@@ -1329,7 +1331,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         ck_info[c] = (bk_kind[ck_blk[c]] == BK_CLAMPV ? BK_PULSE : (bk_kind[ck_blk[c]] & BK_KIND_MASK)) |
                      ((int32_t)bk_type[ck_blk[c]] << 2) | (ck_n[c] << 8);
 
-    // ---- window length: every delay must cover the window (see k_window)
+    // ---- window length: every delay must cover the window (see the windowed path, eden_window.cuh)
     int kmax = kMaxWindow;
     if (ns > 0) {
         double dsteps = std::floor((double)min_delay / (double)dt);
@@ -1529,6 +1531,33 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         auto cmp = [](const std::pair<int, int> &x, const std::pair<int, int> &y) { return x > y; };
         std::make_heap(heap.begin(), heap.end(), cmp);
         for (int uu : uorder) {
+            if (!grow && !heap.empty() && heap.front().first + un_words[uu] > limit) {
+                // no room in any CTA as it is: the one of fewest words exchanges a
+                // unit for a smaller one of a CTA that has room for the difference.
+                // (The batched multicompartment network missed one round by four
+                // words of 57,984, with 1.7 % of the SMs' memory free: 13.3 us a step
+                // in two rounds.)
+                const int a = heap.front().second, need = heap.front().first + un_words[uu] - limit;
+                int bc = -1, best = INT_MAX;
+                size_t by = 0, bz = 0;
+                for (int c = 0; c < n_cta; c++)
+                    for (size_t y = 0; c != a && y < cta_units[a].size(); y++)
+                        for (size_t z = 0; z < cta_units[c].size(); z++) {
+                            const int d = un_words[cta_units[a][y]] - un_words[cta_units[c][z]];
+                            if (d >= need && d < best && cta_words[c] + d <= limit) {
+                                best = d;
+                                bc = c;
+                                by = y;
+                                bz = z;
+                            }
+                        }
+                if (bc < 0) return false;
+                std::swap(cta_units[a][by], cta_units[bc][bz]);
+                cta_words[a] -= best;
+                cta_words[bc] += best;
+                for (auto &h : heap) h.first = cta_words[h.second];
+                std::make_heap(heap.begin(), heap.end(), cmp);
+            }
             if (heap.empty() || (heap.front().first > 0 && heap.front().first + un_words[uu] > limit)) {
                 if (!grow) return false;
                 heap.push_back({0, n_cta++});
@@ -1612,6 +1641,14 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         for (int c = 0; c < n_cta; c++) mx = std::max(mx, cta_words[c]);
         mx += 4 * kPassPad;
         ctx->classes.push_back({0, n_cta, (size_t)mx * sizeof(float)});
+        // The cell kernel's CTAs start beside the input kernel's last blocks only
+        // where a hole these leave cannot cost an SM its last CTA, which would
+        // wait for a whole window: one CTA an SM, or all in half the SM's shared
+        // memory.  (9,000 trees, six CTAs of 36 KB an SM: 12.2 us a step early, 9.6
+        // not; 10,000, two of 113 KB: 9.45 and 9.54; 30,011 HH cells, four of
+        // 16 KB: 2.18 and 2.26.)
+        const int64_t sms = std::max(ctx->n_sm, 1), per_sm = (n_cta + sms - 1) / sms;
+        ctx->cells_early = per_sm <= 1 || per_sm * ((int64_t)mx * 4 + 1024) <= ctx->smem_per_sm / 2;
     }
     size_t max_smem_class = 0;
     for (auto &cl : ctx->classes) max_smem_class = std::max(max_smem_class, cl.smem);
@@ -2150,7 +2187,7 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
         tmark(ctx, EDEN_KERNEL_CELLS, true);
         for (const auto &cl : ctx->classes) {
             const int nb = std::min(cl.cta_end - cl.cta_begin, ctx->max_cell_blocks);
-            launch_order(true, ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
+            launch_order(ctx->cells_early, ctx->fn_cells, nb, ctx->cell_threads, cl.smem, s, d, (const WindowArgs *)ctx->d_wtab,
                      (const WindowTimes *)ctx->d_wtimes, base, idx, cl.cta_begin, cl.cta_end);
             n++;
         }

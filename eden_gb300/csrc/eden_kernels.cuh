@@ -1,24 +1,24 @@
 // Device functions of libeden_gpu: one step of EDEN's loop, split into the
 // phases of the reference's generated per-cell kernel, over structure-of-arrays
-// device tables.  The kernels that drive them are in eden_gpu.cu:
+// device tables.  The kernels that drive them are in eden_window.cuh:
 //   * the per-step path launches k_inputs -> k_targets -> k_hines -> k_deliver
 //     once per step (the reference runs one OpenMP pass per step);
-//   * the windowed path (k_window) advances each group of cells K steps in one
-//     CTA with its membrane state in shared memory, because within K <= min
-//     synaptic delay / dt steps no cell can affect another; one k_deliver then
-//     fans the window's spikes out.
+//   * the windowed path launches k_inputs -> k_cells -> k_deliver once per window:
+//     k_cells advances each unit K steps with its state in shared memory,
+//     because within K <= min synaptic delay / dt steps no cell can affect
+//     another.
 //
 // Internal layout (built on the host in eden_gpu.cu):
-//   groups    contiguous cell ranges, one CTA each in k_window;
-//   forests   each group's physical cells split into warp-sized "forests"; a
-//             forest's compartments are numbered breadth-first over all its
+//   units     a forest of physical cells, or up to 32 point neurons: one warp, or
+//             one and another for its gates;
+//   forests   a forest's compartments are numbered breadth-first over all its
 //             cells at once, so each tree depth is one contiguous range and
 //             every node's children are contiguous, in increasing original
 //             index; a forest is solved by one warp;
-//   targets   every membrane potential: forest compartments, then the group's
-//             izhikevich neurons;
+//   targets   every membrane potential: forest compartments, then the
+//             point neurons;
 //   inputs    connection synapses, Poisson inputs and pulses sorted by target;
-//             targets with any input are listed in `in_tgt` (one warp each).
+//             a target's are cut into blocks of a kind and chunks of a block.
 #pragma once
 #ifndef __CUDACC_RTC__
 #include <cstdint>
@@ -566,7 +566,7 @@ __device__ __forceinline__ void pois_window(const DevModel &m, int64_t it, const
             isi = pois_draw(m, it, w.step0 + j, 0);
         }
     } else if (m.pois_exact && isi < 0x1p23f) {
-        // (one that cannot fire in the window has been dealt with: chunk_window)
+        // (one that cannot fire in the window has been dealt with: input_group)
         int j = 0;
         while (true) {
             // first step from j on whose time since the last spike exceeds isi
@@ -613,7 +613,7 @@ template <int KIND>
 __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const WindowArgs &w, const SynTypeDev &st,
                                            const float *pw, const float *tk, float pend, uint32_t mask, float *rowA, float *rowB,
                                            ItemEvents &ev) {
-    // (chunk_window leaves out initialisation: no spikes reach a synapse in it)
+    // (input_group leaves out initialisation: no spikes reach a synapse in it)
     const float dt = m.dt;
     const float pend0 = pend;
     // a spike that is due, and so its state, is known before the replay: the
@@ -807,8 +807,8 @@ __device__ __forceinline__ void pulse_chunk(const DevModel &m, int c, int32_t in
     const int lane = threadIdx.x & 31;
     const int kind = info & 3;
     const int n = info >> 8;
-    const int kAccStride = m.acc_stride;
-    float *rowA = tileA + lane * kAccStride;
+    const int stride = m.acc_stride;
+    float *rowA = tileA + lane * stride;
     if (EDEN_KIND_CLAMP && kind == BK_PULSE && ((info >> 2) & 63) >= kClampA) {
         // voltage clamps (LEMS_CoreComponents.inc.xml:555-620): the target
         // of the phase each step's time is in (the last OnCondition that
@@ -830,7 +830,7 @@ __device__ __forceinline__ void pulse_chunk(const DevModel &m, int c, int32_t in
         if (lane < w.K) {
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
-            for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
+            for (int r = 0; r < rows; r++) tot += tileA[r * stride + lane];
             m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
@@ -860,7 +860,7 @@ __device__ __forceinline__ void pulse_chunk(const DevModel &m, int c, int32_t in
         if (lane < w.K) {
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
-            for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
+            for (int r = 0; r < rows; r++) tot += tileA[r * stride + lane];
             m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
@@ -895,7 +895,7 @@ __device__ __forceinline__ void pulse_chunk(const DevModel &m, int c, int32_t in
         if (lane < w.K) {
             const int rows = n < 32 ? n : 32;
             float tot = 0.0f;
-            for (int r = 0; r < rows; r++) tot += tileA[r * kAccStride + lane];
+            for (int r = 0; r < rows; r++) tot += tileA[r * stride + lane];
             m.Gp[(size_t)c * m.gp_stride + lane] = tot;
         }
         __syncwarp();
