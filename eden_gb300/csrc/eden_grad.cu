@@ -994,12 +994,23 @@ int alloc(EdenGpuGrad *g, T **dst, size_t n) {
 
 bool finite_pos(float x) { return std::isfinite(x) && x > 0.0f; }
 
-// Most bytes of the trajectory and of the adjoint's coefficients, each: 256
-// cells of 51 compartments over 8,001 steps take 2.1 GB and 5.4 GB, and run in
-// one and in three parts.
-constexpr int64_t kTrajectoryBytes = (int64_t)2200 << 20;
-constexpr int64_t kCoefBytes = (int64_t)2 << 30;
-constexpr int64_t kExposureBytes = (int64_t)256 << 20;
+// The bytes of the buffers whose rows can be cut: the trajectory, the adjoint's
+// coefficients, the unit-weight exposures.  What a caller says (buffer_mib), else
+// a 64th of the device's memory, and of what is free an eighth at most: several
+// contexts, or one beside a program that holds most of the device, each take a
+// part of the rest.  Fewer rows cost time only: 256 cells of 51 compartments over
+// 8,001 steps take 2.1 GB of trajectory and 5.4 GB of coefficients; with 4.4 GB in
+// all the first is kept whole and the second is done in three parts.
+int buffer_bytes(EdenGpuGrad *g, const EdenGpuGradSpec *s, int64_t *bytes) {
+    if (s->buffer_mib > 0) {
+        *bytes = (int64_t)s->buffer_mib << 20;
+        return 0;
+    }
+    size_t free_bytes = 0, total = 0;
+    GTRY(g, cudaMemGetInfo(&free_bytes, &total));
+    *bytes = (int64_t)std::min(total / 64, free_bytes / 8);
+    return 0;
+}
 
 int validate(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     if (m->abi_version != EDEN_GPU_ABI_VERSION)
@@ -1413,8 +1424,6 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
         if ((rc = alloc(g, &d.it_b, (size_t)d.n_item)) != 0) return rc;
         if ((rc = alloc(g, &d.it_cur, (size_t)d.n_item)) != 0) return rc;
         if ((rc = alloc(g, &d.item_grad, (size_t)d.n_item)) != 0) return rc;
-        g->ex_rows = std::max<int64_t>(1, std::min<int64_t>(d.N, kExposureBytes / (4 * d.n_item)));
-        if ((rc = alloc(g, &d.ex, (size_t)g->ex_rows * d.n_item)) != 0) return rc;
         GTRY(g, cudaMemset(d.gbar, 0, rows * sizeof(float)));
     }
     const int64_t n_ck = d.N >= 2 ? (d.N - 2) / d.S + 1 : 1;
@@ -1422,22 +1431,8 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     d.params = g->d_params;
     if ((rc = alloc(g, &d.ck_v, (size_t)n_ck * m->n_comp)) != 0) return rc;
     if ((rc = alloc(g, &d.ck_q, (size_t)n_ck * n_gate)) != 0) return rc;
-    // the trajectory: of the whole run where it fits, else of as many segments
-    const int64_t tr_row = 4 * (2 * (int64_t)m->n_comp + n_gate);
-    g->keep = d.N * tr_row <= kTrajectoryBytes;
-    g->seg_group = g->keep ? n_ck : std::max<int64_t>(1, std::min<int64_t>({n_ck, 65535, kTrajectoryBytes / tr_row / d.S}));
-    const int64_t tr_rows = g->keep ? d.N : std::min<int64_t>(d.N, g->seg_group * d.S + 1);
-    if ((rc = alloc(g, &d.tr_v, (size_t)tr_rows * m->n_comp)) != 0) return rc;
-    if ((rc = alloc(g, &d.tr_q, (size_t)tr_rows * n_gate)) != 0) return rc;
-    if ((rc = alloc(g, &d.tr_d, (size_t)tr_rows * m->n_comp)) != 0) return rc;
-    d.co_len = cell_k0[nphys];
-    g->co_rows = std::max<int64_t>(1, std::min<int64_t>({tr_rows, kCoefBytes / (4 * ((int64_t)d.co_len + m->n_comp)), 1 << 20}));
-    if ((rc = alloc(g, &d.co, (size_t)g->co_rows * d.co_len)) != 0) return rc;
-    if ((rc = alloc(g, &d.mu, (size_t)g->co_rows * m->n_comp)) != 0) return rc;
     if ((rc = alloc(g, &d.lv, (size_t)m->n_comp)) != 0) return rc;
     if ((rc = alloc(g, &d.lq, (size_t)n_gate)) != 0) return rc;
-    d.n_part = (int32_t)((g->co_rows + kSumSteps - 1) / kSumSteps);
-    if ((rc = alloc(g, &d.part, g->slot_param.size() * (size_t)d.n_part)) != 0) return rc;
     {
         const int32_t *p = nullptr;
         if ((rc = upload(g, &p, slot_cell)) != 0) return rc;
@@ -1449,6 +1444,29 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     d.trace_grad = g->d_tgrad;
     if ((rc = alloc(g, &g->d_slot, g->slot_param.size())) != 0) return rc;
     d.slot_grad = g->d_slot;
+    // then what can be cut, from what is left: half for the trajectory, of the
+    // whole run where it fits, else of as many segments; most of the rest for
+    // the coefficients; a 16th for the exposures
+    int64_t budget = 0;
+    if ((rc = buffer_bytes(g, s, &budget)) != 0) return rc;
+    const int64_t tr_row = 4 * (2 * (int64_t)m->n_comp + n_gate), tr_bytes = budget / 2;
+    g->keep = d.N * tr_row <= tr_bytes;
+    g->seg_group = g->keep ? n_ck : std::max<int64_t>(1, std::min<int64_t>({n_ck, 65535, tr_bytes / tr_row / d.S}));
+    const int64_t tr_rows = g->keep ? d.N : std::min<int64_t>(d.N, g->seg_group * d.S + 1);
+    if ((rc = alloc(g, &d.tr_v, (size_t)tr_rows * m->n_comp)) != 0) return rc;
+    if ((rc = alloc(g, &d.tr_q, (size_t)tr_rows * n_gate)) != 0) return rc;
+    if ((rc = alloc(g, &d.tr_d, (size_t)tr_rows * m->n_comp)) != 0) return rc;
+    d.co_len = cell_k0[nphys];
+    g->co_rows = std::min<int64_t>({tr_rows, 1 << 20,
+                                    std::max<int64_t>(kSumSteps, budget / 16 * 7 / (4 * ((int64_t)d.co_len + m->n_comp)))});
+    if ((rc = alloc(g, &d.co, (size_t)g->co_rows * d.co_len)) != 0) return rc;
+    if ((rc = alloc(g, &d.mu, (size_t)g->co_rows * m->n_comp)) != 0) return rc;
+    d.n_part = (int32_t)((g->co_rows + kSumSteps - 1) / kSumSteps);
+    if ((rc = alloc(g, &d.part, g->slot_param.size() * (size_t)d.n_part)) != 0) return rc;
+    if (d.n_grp > 0) {
+        g->ex_rows = std::min<int64_t>(d.N, std::max<int64_t>(kSumSteps, budget / 16 / (4 * d.n_item)));
+        if ((rc = alloc(g, &d.ex, (size_t)g->ex_rows * d.n_item)) != 0) return rc;
+    }
     g->n_params = s->n_params;
     g->n_cells = nphys;
     g->n_rec = s->n_rec;

@@ -37,7 +37,7 @@ class CGradSpec(ctypes.Structure):
                 ("n_rec", ctypes.c_int32), ("rec_comp", ctypes.c_void_p), ("n_steps", ctypes.c_int64),
                 ("checkpoint_every", ctypes.c_int32), ("device", ctypes.c_int32),
                 ("syn_param", ctypes.c_void_p), ("timed_param", ctypes.c_void_p),
-                ("reserved", ctypes.c_int32 * 4)]
+                ("buffer_mib", ctypes.c_int32), ("reserved", ctypes.c_int32 * 3)]
 
 
 def _bind(lib):
@@ -121,10 +121,12 @@ def per_cell_density_map(low: LoweredModel, densities: list[int], ra: bool = Tru
 
 
 class CableGradient:
-    """One gradient context (edenGpuGradCreate) on one GPU."""
+    """One gradient context (edenGpuGradCreate) on one GPU.  buffer_mib: device
+    memory for the buffers that can be cut (include/eden_gpu.h), 0: a share of the
+    device's and of what is free."""
 
     def __init__(self, low: LoweredModel, pmap: ParamMap, rec_comp=None, n_steps: int | None = None,
-                 checkpoint_every: int = 100, device: int = 0):
+                 checkpoint_every: int = 100, device: int = 0, buffer_mib: int = 0):
         self.lib = _bind(load_library())
         self.low = low
         self.pmap = pmap
@@ -143,7 +145,8 @@ class CableGradient:
                          n_rec=self.n_rec, rec_comp=self.rec_comp.ctypes.data, n_steps=self.n_steps,
                          checkpoint_every=checkpoint_every, device=device,
                          syn_param=None if self._sp is None or not len(self._sp) else self._sp.ctypes.data,
-                         timed_param=None if self._tp is None or not len(self._tp) else self._tp.ctypes.data)
+                         timed_param=None if self._tp is None or not len(self._tp) else self._tp.ctypes.data,
+                         buffer_mib=buffer_mib)
         h = ctypes.c_void_p()
         rc = self.lib.edenGpuGradCreate(ctypes.byref(cm), ctypes.byref(spec), ctypes.byref(h))
         self.h = h

@@ -489,8 +489,20 @@ int edenGpuAbiVersion(void);
  * steps 1..n_steps, and returns the gradient of any scalar function of that
  * trace with respect to the parameters, given the function's gradient with
  * respect to the trace: the discrete adjoint of the step, run backward in
- * time over segments recomputed from forward states stored every
- * `checkpoint_every` steps.
+ * time over the forward's states.
+ *
+ * Device memory.  The states of every `checkpoint_every`th step are kept, and
+ * the trace, its gradient, and two conductances a step for each group of
+ * synaptic inputs.  Three buffers hold as many steps as they have room for: the
+ * trajectory (8 bytes a compartment and 4 a gate for each step: kept whole where
+ * that fits, else segments of `checkpoint_every` steps are recomputed, as many at
+ * a time as fit), the adjoint's coefficients (16 bytes a compartment and 12 a
+ * gate) and the synapses' exposures (4 a synapse).  Together they take at most
+ * `buffer_mib` MiB, or, where that is 0, a 64th of the device's memory and an
+ * eighth of what is free when the context is created, whichever is less; never
+ * less than one segment of the trajectory and 32 steps of the others.  With less
+ * memory the calls take longer; the trace is the same, and gradients to the
+ * order in which double-precision sums are taken.
  *
  * Pointers to parameters, traces and gradients may be host or device
  * memory.  Calls are synchronous.
@@ -512,7 +524,9 @@ typedef struct EdenGpuGradSpec {
                                       keep syn_weight; may be null */
     const int32_t *timed_param;    /* [n_timed] parameter that is the input's weight, or -1 to keep
                                       timed_weight; may be null */
-    int32_t reserved[4];
+    int32_t buffer_mib;            /* device memory for what can be computed in parts, below; 0: as
+                                      said there */
+    int32_t reserved[3];           /* zero */
 } EdenGpuGradSpec;
 
 typedef struct EdenGpuGrad EdenGpuGrad;
