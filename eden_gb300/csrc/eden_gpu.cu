@@ -87,7 +87,7 @@ struct EdenGpuCtx {
     double t_prev0 = 0.0;
     int64_t trace_first_unfetched = 1;   // first non-init step not yet fetched
     int64_t log_first = -3;              // no unfetched spike is logged before this step
-    // the log's sorting (sort_log): made on first use, grown as needed
+    // the log's sorting (fetch_sorted): words of bits and counts, entries in order
     uint32_t *log_bits = nullptr, *log_before = nullptr, *log_blocks = nullptr;
     int64_t log_words = 0, sorted_cap = 0;
     int32_t *sorted_src = nullptr;
@@ -218,6 +218,10 @@ cudaError_t launch_order(bool early, const void *fn, int grid, int block, size_t
 
 // ---------------------------------------------------------------------------
 namespace {
+
+constexpr int kLogBlockWords = 4096;             // words of one block's count (k_log_count)
+constexpr int64_t kLogWords = (int64_t)1 << 21;  // most words at a time: steps are taken in turns beyond (fetch_sorted)
+constexpr int64_t kLogHostSort = 1024;           // spikes a turn up to which the host sorts: fewer than five launches' worth
 
 // A context's arrays: a hundred, most of them small.  Those up to kSlabArray
 // bytes lie side by side in slabs, each one allocation, filled on the host and
@@ -1820,9 +1824,25 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         TRY(upload(ctx, &d.wspk_time[b], (const double *)nullptr, wcap));
     }
     TRY(upload(ctx, &d.wspk_count, (const int32_t *)nullptr, 2));
-    TRY(upload(ctx, &d.log_src, (const int32_t *)nullptr, (size_t)log_cap));
-    TRY(upload(ctx, &d.log_step, (const int64_t *)nullptr, (size_t)log_cap));
-    TRY(upload(ctx, &d.log_time, (const double *)nullptr, (size_t)log_cap));
+    {
+        // the log and what a fetch sorts it with, in one allocation: a fetch makes none
+        const int64_t row = (m->n_src + 31) / 32;
+        ctx->sorted_cap = std::max(std::min<int64_t>(log_cap, 4096), log_cap / 8);
+        ctx->log_words = std::max(row, std::min(kLogWords, (ctx->trace_cap + 4) * row));
+        const size_t all = (size_t)(log_cap + ctx->sorted_cap);
+        const size_t blocks = (size_t)(ctx->log_words + kLogBlockWords - 1) / kLogBlockWords + 1;
+        char *p = nullptr;
+        TRY(upload(ctx, &p, (const char *)nullptr, 20 * all + sizeof(uint32_t) * (2 * (size_t)ctx->log_words + blocks)));
+        d.log_step = (int64_t *)p;
+        d.log_time = (double *)(d.log_step + all);
+        d.log_src = (int32_t *)(d.log_time + all);
+        ctx->sorted_step = d.log_step + log_cap;
+        ctx->sorted_time = d.log_time + log_cap;
+        ctx->sorted_src = d.log_src + log_cap;
+        ctx->log_bits = (uint32_t *)(d.log_src + all);
+        ctx->log_before = ctx->log_bits + ctx->log_words;
+        ctx->log_blocks = ctx->log_before + ctx->log_words;
+    }
     TRY(upload(ctx, &d.log_count, (const unsigned long long *)nullptr, 1));
     d.log_cap = log_cap;
     TRY(upload_c(ctx, &d.t_trace0, t_trace0)); TRY(upload_c(ctx, &d.trace_col, trace_col));
@@ -2340,12 +2360,6 @@ extern "C" int edenGpuLastRunStats(EdenGpuCtx *ctx, double *device_ms, int64_t *
 // k_log_scan), and every entry's place is the number of bits before its own.
 // 270,000 spikes of 100,000 sources over 500 steps take 0.05 ms; the log came
 // back unsorted before and was sorted by the caller in 34 ms.
-namespace {
-constexpr int kLogBlockWords = 4096;           // words of one block's count
-constexpr int64_t kLogWords = (int64_t)1 << 24;  // most words at a time (steps are taken in turns beyond)
-constexpr int64_t kLogHostSort = 1024;         // logs up to this are sorted on the host: fewer than five launches' worth
-}  // namespace
-
 __global__ void __launch_bounds__(256) k_log_bits(const int32_t *src, const int64_t *step, int64_t n, int64_t s0, int64_t s1,
                                                   int64_t row, uint32_t *bits) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
@@ -2402,54 +2416,36 @@ __global__ void __launch_bounds__(1024) k_log_scan(uint32_t *blocks, int n) {
     }
     if (threadIdx.x == 0) blocks[n] = base;
 }
+// the entries of these steps whose places are [p0, p0 + cap), to o_* from p0 on
 __global__ void __launch_bounds__(256) k_log_place(const int32_t *src, const int64_t *step, const double *time, int64_t n,
                                                    int64_t s0, int64_t s1, int64_t row, const uint32_t *bits,
-                                                   const uint32_t *before, const uint32_t *blocks, int64_t at, int32_t *o_src,
-                                                   int64_t *o_step, double *o_time) {
+                                                   const uint32_t *before, const uint32_t *blocks, int64_t p0, int64_t cap,
+                                                   int32_t *o_src, int64_t *o_step, double *o_time) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
         if (step[e] < s0 || step[e] >= s1) continue;
         const int64_t w = (step[e] - s0) * row + (src[e] >> 5);
-        const int64_t p = at + blocks[w / kLogBlockWords] + before[w] + __popc(bits[w] & ((1u << (src[e] & 31)) - 1));
+        const int64_t p = (int64_t)blocks[w / kLogBlockWords] + before[w] + __popc(bits[w] & ((1u << (src[e] & 31)) - 1)) - p0;
+        if (p < 0 || p >= cap) continue;
         o_src[p] = src[e];
         o_step[p] = step[e];
         o_time[p] = time[e];
     }
 }
 
-// Sorts the log's n entries, of steps [first, end), into ctx->sorted_*; *ok is
-// false if they are not all different (a spike-source list may name a source
-// twice in a step) or not all of those steps.
-static int sort_log(EdenGpuCtx *ctx, int64_t n, int64_t first, int64_t end, bool *ok) {
+// Turns of as many steps as the words hold, for steps [first, end).
+static int64_t log_turns(const EdenGpuCtx *ctx, int64_t first, int64_t end) {
+    const int64_t row = (ctx->d.n_src + 31) / 32, turn = ctx->log_words / row;
+    return (end - first + turn - 1) / turn;
+}
+
+// Copies the log's n entries, of steps [first, end), to rec in order, by turns
+// of steps and pieces of what there is room to place; *ok is false if they are
+// not all different (a spike-source list may name a source twice in a step) or
+// not all of those steps, and what was copied is then no use.  Nothing is
+// allocated: a program that may not wait for that can fetch.
+static int fetch_sorted(EdenGpuCtx *ctx, EdenGpuRecords *rec, int64_t n, int64_t first, int64_t end, bool *ok) {
     const DevModel &d = ctx->d;
-    const int64_t row = (d.n_src + 31) / 32;
-    const int64_t turn = std::max<int64_t>(1, std::min<int64_t>(end - first, kLogWords / row));
-    const int64_t words = turn * row;
-    const int nblk = (int)((words + kLogBlockWords - 1) / kLogBlockWords);
-    auto grow = [&](void **p, size_t bytes) -> int {  // (the old one's contents are not needed)
-        if (*p) {
-            cudaFree(*p);
-            ctx->allocs.erase(std::remove(ctx->allocs.begin(), ctx->allocs.end(), *p), ctx->allocs.end());
-            *p = nullptr;
-        }
-        CUDA_TRY(ctx, cudaMalloc(p, bytes));
-        ctx->allocs.push_back(*p);
-        return 0;
-    };
-    if (words > ctx->log_words) {
-        ctx->log_words = 0;
-        TRY(grow((void **)&ctx->log_bits, sizeof(uint32_t) * (2 * words + nblk + 1)));
-        ctx->log_before = ctx->log_bits + words;
-        ctx->log_blocks = ctx->log_before + words;
-        ctx->log_words = words;
-    }
-    if (n > ctx->sorted_cap) {
-        const int64_t cap = std::min<int64_t>(d.log_cap, std::max<int64_t>(2 * n, 1 << 16));
-        ctx->sorted_cap = 0;
-        TRY(grow((void **)&ctx->sorted_step, (sizeof(int64_t) + sizeof(double) + sizeof(int32_t)) * cap));
-        ctx->sorted_time = (double *)(ctx->sorted_step + cap);
-        ctx->sorted_src = (int32_t *)(ctx->sorted_time + cap);
-        ctx->sorted_cap = cap;
-    }
+    const int64_t row = (d.n_src + 31) / 32, turn = ctx->log_words / row;
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->n_sm * 16);
     int64_t at = 0;
     for (int64_t s0 = first; s0 < end; s0 += turn) {
@@ -2459,12 +2455,26 @@ static int sort_log(EdenGpuCtx *ctx, int64_t n, int64_t first, int64_t end, bool
         k_log_bits<<<grid, 256, 0, ctx->stream>>>(d.log_src, d.log_step, n, s0, s1, row, ctx->log_bits);
         k_log_count<<<nb, 256, 0, ctx->stream>>>(ctx->log_bits, w, ctx->log_before, ctx->log_blocks);
         k_log_scan<<<1, 1024, 0, ctx->stream>>>(ctx->log_blocks, nb);
-        k_log_place<<<grid, 256, 0, ctx->stream>>>(d.log_src, d.log_step, d.log_time, n, s0, s1, row, ctx->log_bits,
-                                                  ctx->log_before, ctx->log_blocks, at, ctx->sorted_src, ctx->sorted_step,
-                                                  ctx->sorted_time);
+        auto place = [&](int64_t p0) {
+            k_log_place<<<grid, 256, 0, ctx->stream>>>(d.log_src, d.log_step, d.log_time, n, s0, s1, row, ctx->log_bits,
+                                                      ctx->log_before, ctx->log_blocks, p0, ctx->sorted_cap,
+                                                      ctx->sorted_src, ctx->sorted_step, ctx->sorted_time);
+        };
+        place(0);
         uint32_t total = 0;
         CUDA_TRY(ctx, cudaMemcpyAsync(&total, ctx->log_blocks + nb, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        for (int64_t p0 = 0; p0 < total; p0 += ctx->sorted_cap) {
+            const int64_t k = std::min<int64_t>(ctx->sorted_cap, total - p0);
+            if (p0 > 0) place(p0);
+            CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_src + at + p0, ctx->sorted_src, sizeof(int32_t) * k,
+                                          cudaMemcpyDeviceToHost, ctx->stream));
+            CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_step + at + p0, ctx->sorted_step, sizeof(int64_t) * k,
+                                          cudaMemcpyDeviceToHost, ctx->stream));
+            if (rec->spike_time_us)
+                CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_time_us + at + p0, ctx->sorted_time, sizeof(double) * k,
+                                              cudaMemcpyDeviceToHost, ctx->stream));
+        }
         at += total;
     }
     CUDA_TRY(ctx, cudaGetLastError());
@@ -2501,15 +2511,16 @@ extern "C" int edenGpuFetchRecords(EdenGpuCtx *ctx, EdenGpuRecords *rec) {
         for (int64_t k = 0; k < n; k++) rec->trace_step[k] = first + k;
     bool sorted = false;
     // (spikes of the steps since the last fetch, logged a step later each)
-    if (ns > kLogHostSort) TRY(sort_log(ctx, ns, ctx->log_first, last + 2, &sorted));
-    if (ns > 0) {
-        CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_src, sorted ? ctx->sorted_src : ctx->d.log_src, sizeof(int32_t) * ns,
-                                      cudaMemcpyDeviceToHost, ctx->stream));
-        CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_step, sorted ? ctx->sorted_step : ctx->d.log_step, sizeof(int64_t) * ns,
-                                      cudaMemcpyDeviceToHost, ctx->stream));
+    if (ns > kLogHostSort * log_turns(ctx, ctx->log_first, last + 2))
+        TRY(fetch_sorted(ctx, rec, ns, ctx->log_first, last + 2, &sorted));
+    if (ns > 0 && !sorted) {
+        CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_src, ctx->d.log_src, sizeof(int32_t) * ns, cudaMemcpyDeviceToHost,
+                                      ctx->stream));
+        CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_step, ctx->d.log_step, sizeof(int64_t) * ns, cudaMemcpyDeviceToHost,
+                                      ctx->stream));
         if (rec->spike_time_us)
-            CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_time_us, sorted ? ctx->sorted_time : ctx->d.log_time,
-                                          sizeof(double) * ns, cudaMemcpyDeviceToHost, ctx->stream));
+            CUDA_TRY(ctx, cudaMemcpyAsync(rec->spike_time_us, ctx->d.log_time, sizeof(double) * ns,
+                                          cudaMemcpyDeviceToHost, ctx->stream));
     }
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->d.log_count, 0, sizeof(unsigned long long), ctx->stream));
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->d.status, 0, sizeof(int), ctx->stream));
