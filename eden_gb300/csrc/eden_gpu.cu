@@ -1360,7 +1360,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         for (int b = b0; b < b1; b++) {
             int32_t e;
             memcpy(&e, &bk_erev[b], 4);
-            bk_rec[b] = make_int4((bk_c0[b] - bk_c0[b0]) * ctx->d.gp_stride, (bk_c0[b + 1] - bk_c0[b0]) * ctx->d.gp_stride,
+            bk_rec[b] = make_int4((un_f[u] >= 0 ? b - b0 : bk_c0[b] - bk_c0[b0]) * ctx->d.gp_stride, bk_c0[b + 1] - bk_c0[b],
                                   bk_kind[b], e);
         }
     }
@@ -1500,10 +1500,9 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         un_ngt[u] = ch_gate0[c_chan0[b]] - un_gt0[u];
         if (un_f[u] >= 0) {
             const int nblk = t_blk0[b] - t_blk0[a];
-            const int nck = bk_c0[t_blk0[b]] - bk_c0[t_blk0[a]];
             const int f = un_f[u];
             un_words[u] = forest_words(fo_n0[f + 1] - fo_n0[f], fo_w0[f + 1] - fo_w0[f], un_nf1[u] - un_nf0[u], un_ch1[u] - un_ch0[u], un_ngt[u],
-                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, nck, ctx->d.gp_stride,
+                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, ctx->d.gp_stride,
                                        fo_f64[un_f[u]] != 0);
         } else {
             un_words[u] = izh_words(b - a);

@@ -265,8 +265,9 @@ struct DevModel {
     const int32_t *gt_idx;
     const float4 *gate_tab;
     int32_t gate_warp;  // a unit's gates have a warp of their own (no gate takes V after the solve)
-    // per input block: where its chunks begin and end in the unit's series
-    // (gp_stride each), kind and reversal potential
+    // per input block: where its series begins in the unit's (forests: a series
+    // of gp_stride a block, staged; point neurons: a block's first chunk's in Gp),
+    // chunks, kind and reversal potential
     const int4 *bk_rec;
     int32_t *status;
     // forests whose cells may lose diagonal dominance: their elimination runs
@@ -340,18 +341,18 @@ constexpr int kGateExtWords = 9;  // a non-rates gate's kind and timeCourse / st
 // one of zeros after them) and nw twig rows, what addresses refer to first:
 // pairs, V and elimination factor per node; two words per twig place, pre-updated V and V; then the 16-byte
 // records: one per node, one per twig place, two per non-flat compartment, one
-// per input block, and the window's conductance series of the unit's input
-// chunks (gps words each); then pairs: threshold and source per non-flat
+// per input block, and the window's conductance series of each (gps words, its
+// chunks summed); then pairs: threshold and source per non-flat
 // compartment; then words: a twig place's addresses, V at the start of the step,
 // the next and the last per non-flat compartment, four per channel of these, three per gate (its index
 // word, its value in alternate steps), and the passes.  A batch of izhikevich
 // neurons: V twice and 19 parameter / state words per neuron.
 __host__ __device__ inline int twig_words(int n) { return (2 * n + 3) & ~3; }  // where the twigs' words start
-__host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int nck, int gps,
+__host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int gps,
                                             bool f64 = false) {
     // a double-precision forest adds its eliminated values, pivots and
     // factors in double (6 words per compartment, 8-byte aligned)
-    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + gps * nck + 2 * nf +
+    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + gps * nblk + 2 * nf +
                   32 * nw + 3 * nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
     return (w + 3) & ~3;
 }
@@ -1170,18 +1171,35 @@ __device__ __forceinline__ void block_currents(const float *Gpk, int stride, int
     }
 }
 
-// block_currents from the unit's block records in shared memory (where its
-// chunks begin and end in the unit's series, `stride` apart, kind, reversal
-// potential)
-__device__ __forceinline__ void block_currents_rec(const float *Gk, int stride, const int4 *BK, int b0, int b1, float v,
-                                                   float &Iin, float &Gin, float &Isyn, float &Gsyn) {
+// Four steps' values of a block of nc chunks, summed in their order: p, the first
+// chunk's, the others gps words apart.  Loads go ahead of the chain of additions.
+__device__ __forceinline__ float4 sum_chunks(const float *p, int gps, int nc) {
+    auto at = [&](int c) { return *reinterpret_cast<const float4 *>(p + (size_t)c * gps); };
+    auto add = [](float4 &g, const float4 &x) { g.x += x.x; g.y += x.y; g.z += x.z; g.w += x.w; };
+    float4 g = at(0);
+    int c = 1;
+#pragma unroll 1
+    for (; c + 8 <= nc; c += 8) {
+        float4 x[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = at(c + j);
+#pragma unroll
+        for (int j = 0; j < 8; j++) add(g, x[j]);
+    }
+#pragma unroll 1
+    for (; c < nc; c++) add(g, at(c));
+    return g;
+}
+
+// block_currents from the unit's block records (where the block's series begins
+// in the unit's, kind, reversal potential); Gk: the unit's series at the step
+__device__ __forceinline__ void block_currents_rec(const float *Gk, const int4 *BK, int b0, int b1, float v, float &Iin,
+                                                   float &Gin, float &Isyn, float &Gsyn) {
     Iin = 0.0f; Gin = 0.0f; Isyn = 0.0f; Gsyn = 0.0f;
 #pragma unroll 1
     for (int bk = b0; bk < b1; bk++) {
         const int4 r = BK[bk];
-        float g = Gk[r.x];
-#pragma unroll 1
-        for (int c = r.x + stride; c < r.y; c += stride) g += Gk[c];
+        const float g = Gk[r.x];
         const int kind = r.z & BK_KIND_MASK;
         if (EDEN_KIND_CLAMP && kind == BK_CLAMPV) {
             Iin -= v * g;

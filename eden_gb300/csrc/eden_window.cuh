@@ -216,6 +216,36 @@ __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs 
 // already produced them for all K steps.  Everything else a step reads is
 // staged in the warp's shared-memory slice for the whole window.
 
+// The series of a unit's blocks, into shared memory, where some have several
+// chunks: those are summed over them here, a thread four steps.  In the steps it
+// would be a lane a block, one load after the other.  (One compartment of 128,000
+// inputs, a window of 29 steps: 742 us by steps, 129 so; 20 compartments with
+// 51,200 together: 102 and 87.  Called, not inlined: its registers are not the
+// steps'; one of 1,000 HH cells took 1.42 us with it inlined, 1.40 so.)
+__device__ __noinline__ void stage_sums(float *GS, const float *Gp, const int32_t *c0, int nblk, int gps, int th, int nth) {
+    const int quads = gps >> 2;
+    for (int i = th; i < nblk * quads; i += nth) {
+        const int b = i / quads, c = c0[b], nc = c0[b + 1] - c;
+        const float *p = &Gp[(size_t)c * gps + 4 * (i - b * quads)];
+        if (nc == 1) stage_rec(&GS[4 * i], p);
+        else *reinterpret_cast<float4 *>(&GS[4 * i]) = sum_chunks(p, gps, nc);
+    }
+}
+// The same of a point neuron's blocks [b0, b1), into their first chunk's series,
+// by the lane that reads it.  (100 neurons of 10,000 synapses, a window of 10 steps:
+// 218 us by steps, 80 so; 300 of 300: 28 and 28.)
+__device__ __noinline__ void sum_blocks(float *Gk, const int4 *BK, int b0, int b1, int gps, int K) {
+    for (int b = b0; b < b1; b++) {
+        const int4 r = BK[b];
+        if (r.y == 1) continue;
+#pragma unroll 2
+        for (int k = 0; k < K; k += 4) {
+            float *p = &Gk[r.x + k];
+            *reinterpret_cast<float4 *>(p) = sum_chunks(p, gps, r.y);
+        }
+    }
+}
+
 // A forest unit over the window.  At the window start the unit stages its
 // nodes', twigs' and non-flat compartments' records, its gates, its input
 // blocks, and the conductance series of its input chunks for all K steps
@@ -265,7 +295,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     int4 *BK = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
     const int gps = m.gp_stride;
     float *GS = reinterpret_cast<float *>(BK + nblk);
-    float2 *TS = reinterpret_cast<float2 *>(GS + gps * nck);
+    float2 *TS = reinterpret_cast<float2 *>(GS + gps * nblk);
     uint32_t *TA = reinterpret_cast<uint32_t *>(TS + nf);
     float *VO = (float *)(TA + 32 * nw);  // three buffers of nf: step k starts from buffer k % 3
     float *CHG = VO + 3 * nf, *CHE = CHG + nch;
@@ -315,7 +345,10 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
         stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
     }
     for (int i = th; i < ngt; i += nth) stage_word(&GT[i], &m.gate[gt0 + i]);
-    for (int i = 4 * th; i < gps * nck; i += 4 * nth) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
+    if (nck == nblk)
+        for (int i = 4 * th; i < gps * nck; i += 4 * nth) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
+    else
+        stage_sums(GS, m.Gp, m.bk_c0 + ub0, nblk, gps, th, nth);
     stage_wait();
     unit_sync();
     for (int j = th; j < nf; j += nth) VO[j] = XR[__float_as_int(NF[kSlotRecs * j].x) & kPassStart].x;
@@ -410,7 +443,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
             const int ch0 = crange & 0xffff;
             const float v = Vq[j];
             float Iin, Gin, Isyn, Gsyn;
-            block_currents_rec(Gk, gps, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
+            block_currents_rec(Gk, BK, brange & 0xffff, (int)((uint32_t)brange >> 16), v, Iin, Gin, Isyn, Gsyn);
             // (a model with gap junctions runs one-step windows: vsrc holds
             // every target's potential at this step's start)
             if (EDEN_KIND_GAP) Isyn += gap_current(m, t0 + m.nd_t[n0 + ti], v, vsrc, init);
@@ -543,7 +576,9 @@ __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w,
     const int ub0 = m.t_blk0[t0];
     const int b0 = lane < n ? m.t_blk0[t0 + lane] - ub0 : 0, b1 = lane < n ? m.t_blk0[t0 + lane + 1] - ub0 : 0;
     const int4 *BK = m.bk_rec + ub0;
-    const float *Gk = m.Gp + (size_t)m.bk_c0[ub0] * m.gp_stride;
+    const int uc0 = m.bk_c0[ub0], nblk = m.t_blk0[t0 + n] - ub0;
+    float *Gk = m.Gp + (size_t)uc0 * m.gp_stride;
+    if (m.bk_c0[ub0 + nblk] - uc0 > nblk) sum_blocks(Gk, BK, b0, b1, m.gp_stride, w.K);
     const int src = lane < n ? m.t_src[t0 + lane] : -1;
     uint32_t spikes = 0;
     for (int k = 0; k < w.K; k++) {
@@ -555,7 +590,7 @@ __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w,
         if (i < n) {
             const float v = vin[i];
             float Iin, Gin, Isyn, Gsyn;
-            block_currents_rec(Gk + k, m.gp_stride, BK, b0, b1, v, Iin, Gin, Isyn, Gsyn);
+            block_currents_rec(Gk + k, BK, b0, b1, v, Iin, Gin, Isyn, Gsyn);
             float uu = SU[i], ss = SS[i], vn;
             if (point_update(KIND[i], P + i, n, init, tk[k], dt, v, Isyn + Iin, uu, ss, vn)) spikes |= 1u << k;
             vout[i] = vn;
