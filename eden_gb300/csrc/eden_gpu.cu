@@ -1411,6 +1411,9 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     std::vector<int32_t> gr_t, gr_col;
     std::vector<int32_t> un_nf0(n_unit), un_nf1(n_unit), un_ch0(n_unit), un_ch1(n_unit), nf_t;
     std::vector<int> un_words(n_unit);
+    std::vector<uint8_t> un_far(n_unit, 0);
+    bool far = false;  // for any unit
+    const int most = (int)(ctx->smem_optin / sizeof(float)) - 4 * kPassPad;  // words of one block
     for (int u = 0; u < n_unit; u++) {
         const int a = un_t0[u], b = un_t1[u];
         un_nf0[u] = (int)nf_t.size();
@@ -1501,9 +1504,23 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         if (un_f[u] >= 0) {
             const int nblk = t_blk0[b] - t_blk0[a];
             const int f = un_f[u];
-            un_words[u] = forest_words(fo_n0[f + 1] - fo_n0[f], fo_w0[f + 1] - fo_w0[f], un_nf1[u] - un_nf0[u], un_ch1[u] - un_ch0[u], un_ngt[u],
-                                       fo_p0[un_f[u] + 1] - fo_p0[un_f[u]], nblk, ctx->d.gp_stride,
-                                       fo_f64[un_f[u]] != 0);
+            // (where the whole slice is too large for a block, the input blocks' records
+            // stay in global memory; a model with a unit that does not fit even so runs
+            // the per-step kernels.  600 cells of 1,000 compartments with an input each:
+            // 337 us a step by those, 144 so; one such cell 33.6 and 32.3, one of 300
+            // compartments with five types of inputs each 27.8 and 21.3.  The slots'
+            // records and thresholds there as well: slower than the per-step kernels.)
+            auto words = [&](bool keep_far) {
+                return forest_words(fo_n0[f + 1] - fo_n0[f], fo_w0[f + 1] - fo_w0[f], un_nf1[u] - un_nf0[u],
+                                    un_ch1[u] - un_ch0[u], un_ngt[u], fo_p0[f + 1] - fo_p0[f], nblk, ctx->d.gp_stride,
+                                    fo_f64[f] != 0, keep_far);
+            };
+            un_words[u] = words(false);
+            if (un_words[u] > most) {
+                un_words[u] = words(true);
+                un_far[u] = 1;
+                far = true;
+            }
         } else {
             un_words[u] = izh_words(b - a);
         }
@@ -1515,7 +1532,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // up to four units take turns.  Units go longest-first onto the CTA with the
     // fewest words.  (On the batched multicompartment network, 10,000 cells in
     // 35 MB, CTAs of four needed a second round for a quarter of them.)
-    const int most = (int)(ctx->smem_optin / sizeof(float)) - 4 * kPassPad;  // words of one block
     std::vector<int> uorder(n_unit);
     std::iota(uorder.begin(), uorder.end(), 0);
     std::stable_sort(uorder.begin(), uorder.end(), [&](int x, int y) { return un_words[x] > un_words[y]; });
@@ -1627,6 +1643,11 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         for (size_t j = 0; j < unit_of_slot.size(); j++) o[j] = v[unit_of_slot[j]];
         v.swap(o);
     };
+    {
+        std::vector<uint8_t> o(n_unit);
+        for (int j = 0; j < n_unit; j++) o[j] = un_far[unit_of_slot[j]];
+        un_far.swap(o);
+    }
     for (auto *v : {&un_t0, &un_t1, &un_f, &un_gt0, &un_ngt, &un_ch0, &un_ch1, &un_r0, &un_r1, &un_nf0, &un_nf1}) perm(*v);
     {
         std::vector<int> w2(n_unit);
@@ -1854,7 +1875,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload_c(ctx, &d.un_ch0, un_ch0)); TRY(upload_c(ctx, &d.un_ch1, un_ch1));
     TRY(upload_c(ctx, &d.un_r0, un_r0)); TRY(upload_c(ctx, &d.un_r1, un_r1)); TRY(upload_c(ctx, &d.cta_u0, cta_u0));
     TRY(upload_c(ctx, &d.gr_t, gr_t)); TRY(upload_c(ctx, &d.gr_col, gr_col));
-    TRY(upload_c(ctx, &d.un_nf0, un_nf0)); TRY(upload_c(ctx, &d.un_nf1, un_nf1));
+    TRY(upload_c(ctx, &d.un_nf0, un_nf0)); TRY(upload_c(ctx, &d.un_nf1, un_nf1)); TRY(upload_c(ctx, &d.un_far, un_far));
     TRY(upload_c(ctx, &d.nf_rec, nf_rec)); TRY(upload_c(ctx, &d.nf_ts, nf_ts));
     TRY(upload_c(ctx, &d.gt_idx, gt_idx)); TRY(upload_c(ctx, &d.gate_tab, gate_tab));
     TRY(upload_c(ctx, &d.bk_rec, bk_rec));
@@ -1951,7 +1972,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // batched mode uses them (codegen >= 0) and NVRTC is available, else the
     // built-in ones (codegen = 1 makes a failed compile an error)
     ctx->fn_inputs = (const void *)k_inputs_t;
-    ctx->fn_cells = (const void *)k_cells_t;
+    ctx->fn_cells = far ? (const void *)k_cells_far_t : (const void *)k_cells_t;
     ctx->fn_deliver = (const void *)k_deliver_t;
     const int codegen = opt ? opt->codegen : 0;
     if (ctx->mode == EDEN_MODE_BATCHED && ctx->smem_window && codegen >= 0) {
@@ -1978,6 +1999,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         kinds.forest = d.n_forest > 0;
         kinds.gateforms = gate_forms;
         kinds.gate_warps = gate_warp;
+        kinds.far = far;
         kinds.izh = n_izh > 0;
         kinds.gap = m->n_gap > 0 || m->n_graded > 0;
         ctx->codegen_source = eden_codegen::program_source(eden_codegen::kind_defines(kinds) +

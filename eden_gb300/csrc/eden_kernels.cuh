@@ -252,6 +252,7 @@ struct DevModel {
     // C, 1/C; sum 1/(R C), block range, channel range, channel set), and nf_ts,
     // its spike threshold (NaN: no spike source) and source
     const int32_t *un_nf0, *un_nf1;
+    const uint8_t *un_far;  // the unit's slice has no room for its blocks' records
     const float4 *nf_rec;
     const float2 *nf_ts;
     // channels of the slots, [un_ch0[u], un_ch1[u]): conductivity, reversal
@@ -349,11 +350,11 @@ constexpr int kGateExtWords = 9;  // a non-rates gate's kind and timeCourse / st
 // neurons: V twice and 19 parameter / state words per neuron.
 __host__ __device__ inline int twig_words(int n) { return (2 * n + 3) & ~3; }  // where the twigs' words start
 __host__ __device__ inline int forest_words(int n, int nw, int nf, int nfch, int ngt, int np, int nblk, int gps,
-                                            bool f64 = false) {
+                                            bool f64 = false, bool far = false) {
     // a double-precision forest adds its eliminated values, pivots and
     // factors in double (6 words per compartment, 8-byte aligned)
-    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + nblk) + gps * nblk + 2 * nf +
-                  32 * nw + 3 * nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
+    const int w = twig_words(n + 1) + 64 * nw + 4 * (n + 1 + 32 * nw + kSlotRecs * nf + (far ? 0 : nblk)) + gps * nblk +
+                  2 * nf + 32 * nw + 3 * nf + 4 * nfch + 3 * ngt + np + (f64 ? 6 * n + 2 : 0);
     return (w + 3) & ~3;
 }
 __host__ __device__ inline int izh_words(int n) { return ((2 + EDEN_POINT_PARAMS + 3) * n + 3) & ~3; }
@@ -713,6 +714,9 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
 #endif
 #ifndef EDEN_GATE_WARPS
 #define EDEN_GATE_WARPS 1  // units' gates may have a warp of their own (DevModel::gate_warp)
+#endif
+#ifndef EDEN_FAR_RECORDS
+#define EDEN_FAR_RECORDS 0  // k_cells_t: units may keep records in global memory (DevModel::un_far)
 #endif
 
 // A timedSynapticInput item over the window: its synapse fires in each

@@ -269,6 +269,10 @@ __device__ __noinline__ void sum_blocks(float *Gk, const int4 *BK, int b0, int b
 // (A kernel compiled for a model without gate warps keeps the threshold test in
 // the loop that takes V over; with them, one body for both roles: compiled
 // apart, the solve of 50 trees took 112 us a window instead of 100.)
+//
+// FAR: a unit too large for a block's shared memory (un_far) reads its blocks'
+// records where they are; a step finds them in L1.
+template <bool FAR>
 __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S, bool gates,
                                               int barrier, bool first) {
     const int lane = threadIdx.x & 31;
@@ -292,9 +296,11 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     float *TX = S + twig_words(n + 1), *TV = TX + 32 * nw;
     float4 *CN = reinterpret_cast<float4 *>(TV + 32 * nw), *TR = CN + n + 1;
     float4 *NF = TR + 32 * nw;
-    int4 *BK = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
+    const bool far = FAR && m.un_far[u] != 0;
+    int4 *BKs = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
+    const int4 *BK = far ? m.bk_rec + ub0 : BKs;
     const int gps = m.gp_stride;
-    float *GS = reinterpret_cast<float *>(BK + nblk);
+    float *GS = reinterpret_cast<float *>(BKs + (far ? 0 : nblk));
     float2 *TS = reinterpret_cast<float2 *>(GS + gps * nblk);
     uint32_t *TA = reinterpret_cast<uint32_t *>(TS + nf);
     float *VO = (float *)(TA + 32 * nw);  // three buffers of nf: step k starts from buffer k % 3
@@ -324,7 +330,8 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
         stage_word(&TA[i], &m.tw_adr[32 * w0 + i]);
     }
     for (int i = th; i < kSlotRecs * nf; i += nth) stage_rec(&NF[i], &m.nf_rec[(size_t)kSlotRecs * nf0 + i]);
-    for (int i = th; i < nblk; i += nth) stage_rec(&BK[i], &m.bk_rec[ub0 + i]);
+    if (!far)
+        for (int i = th; i < nblk; i += nth) stage_rec(&BKs[i], &m.bk_rec[ub0 + i]);
     for (int j = th; j < nf; j += nth) {
         stage_word(&TS[j].x, &m.nf_ts[nf0 + j].x); stage_word(&TS[j].y, &m.nf_ts[nf0 + j].y);
     }
@@ -640,9 +647,9 @@ __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w,
 // A block runs several CTAs in turn when there are more CTAs than blocks;
 // their units are laid out differently in shared memory, so every warp of
 // the block finishes its unit before any starts on the next CTA.
-__global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
-                                                          const WindowTimes *ttab, const int *base, int idx,
-                                                          int cta_begin, int cta_end) {
+template <bool FAR>
+__device__ __forceinline__ void cells(const DevModel &m, const WindowArgs *tab, const WindowTimes *ttab, const int *base,
+                                      int idx, int cta_begin, int cta_end) {
     extern __shared__ __align__(16) float sm[];
     const WindowArgs w = tab[*base + idx];
     const float *tk = ttab[*base + idx].tk;
@@ -655,12 +662,25 @@ __global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(const __grid_consta
         const int u = m.cta_u0[cta] + slot;
         if (u < m.cta_u0[cta + 1]) {
             if (m.un_f[u] >= 0) {
-                if (EDEN_KIND_FOREST) forest_window(m, w, u, sm + m.un_off[u], gates, 1 + slot, first);
+                if (EDEN_KIND_FOREST) forest_window<FAR>(m, w, u, sm + m.un_off[u], gates, 1 + slot, first);
             } else if (EDEN_KIND_IZH && !gates) izh_window(m, w, tk, u, sm + m.un_off[u], first);
         }
         if (cta + (int)gridDim.x < cta_end) __syncthreads();
     }
 }
+__global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
+                                                          const WindowTimes *ttab, const int *base, int idx,
+                                                          int cta_begin, int cta_end) {
+    cells<EDEN_FAR_RECORDS != 0>(m, tab, ttab, base, idx, cta_begin, cta_end);
+}
+#ifndef EDEN_RTC
+// for a model with a unit that keeps records in global memory
+__global__ void __launch_bounds__(kCellThreads, 1) k_cells_far_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
+                                                              const WindowTimes *ttab, const int *base, int idx,
+                                                              int cta_begin, int cta_end) {
+    cells<true>(m, tab, ttab, base, idx, cta_begin, cta_end);
+}
+#endif
 
 __global__ void k_bump(int *base, int by) { *base += by; }
 
