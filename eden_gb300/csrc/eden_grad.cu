@@ -159,7 +159,7 @@ struct Cell {
     float *Cc, *Ac, *IRCs;
     int32_t *P, *CB, *CE, *ch0;
     int32_t *ctype, *cg0;
-    int32_t *gmap;  // per gate: compartment | (channel type << 2 | gate of it) << 16
+    const int32_t *gmap;  // per gate: compartment | (channel type << 2 | gate of it) << 16
     float *cgb, *cerev;
     int c0, g0, nc, ng, nch, nlev;
     const int32_t *lev;
@@ -173,6 +173,9 @@ __device__ __forceinline__ float axial_scale(const GradDev &m, int cell) {
     return rp >= 0 ? m.cell_ra[cell] / m.params[rp] : 1.0f;
 }
 
+// NEAR: the gates' map is staged too (a cell that has no room for it reads it
+// where it is).
+template <bool NEAR>
 __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dims &dm) {
     extern __shared__ __align__(16) double smem_d[];
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -197,7 +200,7 @@ __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dim
     c.ch0 = i; i += dm.c + 1;
     c.ctype = i; i += dm.ch;
     c.cg0 = i; i += dm.ch;
-    c.gmap = i;
+    int32_t *gmap = i;
     c.c0 = m.cell_c0[cell];
     c.nc = m.cell_c0[cell + 1] - c.c0;
     c.g0 = m.cell_g0[cell];
@@ -237,7 +240,9 @@ __device__ __forceinline__ Cell stage_cell(const GradDev &m, int cell, const Dim
         c.cgb[k] = p >= 0 ? m.params[p] : m.ch_gbase[ch];
         c.cerev[k] = m.ch_erev[ch];
     }
-    for (int k = tid; k < c.ng; k += nt) c.gmap[k] = m.gate_map[c.g0 + k];
+    c.gmap = NEAR ? gmap : m.gate_map + c.g0;
+    if (NEAR)
+        for (int k = tid; k < c.ng; k += nt) gmap[k] = m.gate_map[c.g0 + k];
     __syncthreads();
     return c;
 }
@@ -442,10 +447,10 @@ __device__ __forceinline__ void hines_cell(const Cell &c, float *VN) {
 // compartments 2,700 cycles of the solve's chain (a product, a fused one and a
 // reciprocal a compartment) and about 500 of the rest, where one warp a cell,
 // taking its 153 gates in turns before the solve, took 16,000.
-template <bool RECOMPUTE>
+template <bool RECOMPUTE, bool NEAR>
 __global__ void __launch_bounds__(32 * kFwdWarps) k_grad_forward(GradDev m, Dims dm, int cw, int64_t seg0, int keep) {
     const int cell = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const Cell c = stage_cell(m, cell, dm);
+    const Cell c = stage_cell<NEAR>(m, cell, dm);
     const int64_t seg = RECOMPUTE ? seg0 + blockIdx.y : 0;
     const int64_t first = 1 + seg * m.S, end = RECOMPUTE && first + m.S < m.N ? first + m.S : m.N;
     float *V = c.Va, *Vn = c.Vb, *q = c.qa, *qn = c.qb;  // at the step's start, and the next's
@@ -698,7 +703,10 @@ __device__ __forceinline__ void copy4(float *smem_dst, const float *gmem_src) {
 // whose coefficients are there; lv and lq hold the adjoints of the state after
 // them and receive those of the state before.  The first warp solves; the others
 // fetch a row of coefficients, `ring` - 1 steps ahead of its use, in the
-// meantime; then every thread takes its compartments and their gates.
+// meantime; then every thread takes its compartments and their gates.  Without
+// STAGED (a cell of which not one row fits shared memory; `ring` 0) the rows are read
+// where they are.
+template <bool STAGED>
 __global__ void __launch_bounds__(256) k_grad_adjoint(GradDev m, Dims dm, int64_t rows, int ring, int stage, int last) {
     extern __shared__ __align__(16) double smem_d[];
     const int cell = blockIdx.x, tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5;
@@ -740,17 +748,17 @@ __global__ void __launch_bounds__(256) k_grad_adjoint(GradDev m, Dims dm, int64_
     if (last)
         for (int j = tid; j < nc; j += nt)
             for (int r = RC[j]; r < RC[j + 1]; r++) X[j] += m.trace_grad[(m.N - 1) * m.n_rec + m.rec_col[r0 + r]];
-    if (warp > 0) {
+    if (STAGED && warp > 0) {
         fetch(rows - 1);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         for (int k = 1; k < ring - 1; k++) fetch(rows - 1 - k);
     }
     for (int64_t row = rows - 1; row >= 0; row--) {
         __syncthreads();
-        const float *co = R + (row % ring) * stage;
+        const float *co = STAGED ? R + (row % ring) * stage : m.co + row * m.co_len + m.cell_k0[cell];
         if (warp == 0) {
             adjoint_solve(X, co, co + nc, co + 2 * nc, nc, chain, serial, P, CB, CE, lev, nlev);
-        } else if (ring > 1) {
+        } else if (STAGED && ring > 1) {
             // into the stage of the row before this one's in time, which is done
             // with; then the next row is there
             fetch(row - (ring - 1));
@@ -768,10 +776,11 @@ __global__ void __launch_bounds__(256) k_grad_adjoint(GradDev m, Dims dm, int64_
                 x += lq * gb[ng + k];
                 LQ[k] = lq * gb[k] + mu * gb[2 * ng + k];
             }
-            for (int r = RC[j]; r < RC[j + 1]; r++) x += tg[r];
+            for (int r = RC[j]; r < RC[j + 1]; r++)
+                x += STAGED ? tg[r] : m.trace_grad[(m.co_n0 + row - 1) * m.n_rec + m.rec_col[r0 + r]];
             X[j] = x;
         }
-        if (ring == 1) {  // (one row at a time)
+        if (STAGED && ring == 1) {  // (one row at a time)
             __syncthreads();
             if (warp > 0) {
                 fetch(row - 1);
@@ -937,6 +946,7 @@ struct EdenGpuGrad {
     // of coefficients in flight in the adjoint, and the floats of one
     int fwd_threads = 64, fwd_cw = 1, adj_threads = 64, ring = 1, stage = 4;
     size_t smem = 0, smem_adj = 0;
+    bool near_gates = true;  // the forward stages the gates' map
     // rows of the buffers: whether every step's trajectory is kept, the segments
     // recomputed at a time where not, the steps of coefficients, of exposures
     bool keep = false;
@@ -1390,15 +1400,20 @@ int build(EdenGpuGrad *g, const EdenGpuModel *m, const EdenGpuGradSpec *s) {
     g->adj_threads = std::min(256, std::max(64, (dm.c + 31) / 32 * 32));
     g->ring = kRing;
     while (g->ring > 1 && adj + sizeof(float) * g->ring * (size_t)g->stage > (size_t)(g->ring > 2 ? 100 * 1024 : optin)) g->ring /= 2;
+    // the largest cells: coefficients, or the gates' map, read where they are
+    if (adj + sizeof(float) * g->ring * (size_t)g->stage > (size_t)optin) g->ring = 0;
+    g->near_gates = g->smem <= (size_t)optin;
+    if (!g->near_gates) g->smem -= dm.g * sizeof(int32_t);
     g->smem_adj = adj + sizeof(float) * g->ring * (size_t)g->stage;
     if (std::max(g->smem, g->smem_adj) > (size_t)optin)
         return g->fail(EDEN_GPU_E_INVALID, "largest cell (%d compartments, %d gates) needs %zu bytes of shared memory, "
                                            "the device allows %d", dm.c, dm.g, std::max(g->smem, g->smem_adj), optin);
     // (the limit belongs to the kernels, which every context launches: the
     // device's own, so that no context lowers another's)
-    GTRY(g, cudaFuncSetAttribute(k_grad_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    GTRY(g, cudaFuncSetAttribute(k_grad_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    GTRY(g, cudaFuncSetAttribute(k_grad_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    for (const void *fn : {(const void *)k_grad_forward<false, true>, (const void *)k_grad_forward<true, true>,
+                           (const void *)k_grad_forward<false, false>, (const void *)k_grad_forward<true, false>,
+                           (const void *)k_grad_adjoint<true>, (const void *)k_grad_adjoint<false>})
+        GTRY(g, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     std::vector<EdenGpuChannelType> types(m->chan_types, m->chan_types + m->n_chan_types);
     int rc;
 #define UP(dst, src) \
@@ -1524,7 +1539,8 @@ extern "C" int edenGpuGradForward(EdenGpuGrad *g, const float *params, float *tr
             k_grad_drive<<<(unsigned)((rows * g->d.n_grp + 127) / 128), 128, 0, g->stream>>>(g->d, n0, rows);
         }
     g->d.tr_n0 = 1;
-    k_grad_forward<false><<<g->n_cells, g->fwd_threads, g->smem, g->stream>>>(g->d, g->dims, g->fwd_cw, 0, g->keep ? 1 : 0);
+    (g->near_gates ? k_grad_forward<false, true> : k_grad_forward<false, false>)<<<g->n_cells, g->fwd_threads, g->smem, g->stream>>>(
+        g->d, g->dims, g->fwd_cw, 0, g->keep ? 1 : 0);
     GTRY(g, cudaGetLastError());
     GTRY(g, cudaEventRecord(g->e1, g->stream));
     if (trace && g->n_rec > 0)
@@ -1560,14 +1576,15 @@ extern "C" int edenGpuGradBackward(EdenGpuGrad *g, const float *trace_grad, floa
         const int64_t n0 = 1 + lo * d.S, n1 = std::min<int64_t>(1 + hi * d.S, d.N);
         d.tr_n0 = g->keep ? 1 : n0;
         if (!g->keep)
-            k_grad_forward<true><<<dim3(g->n_cells, (unsigned)(hi - lo)), g->fwd_threads, g->smem, g->stream>>>(
-                d, g->dims, g->fwd_cw, lo, 1);
+            (g->near_gates ? k_grad_forward<true, true> : k_grad_forward<true, false>)
+                <<<dim3(g->n_cells, (unsigned)(hi - lo)), g->fwd_threads, g->smem, g->stream>>>(d, g->dims, g->fwd_cw, lo, 1);
         for (int64_t b = n1; b > n0;) {
             const int64_t a = std::max<int64_t>(n0, b - g->co_rows), rows = b - a;
             const int chunks = (int)((rows + kSumSteps - 1) / kSumSteps);
             d.co_n0 = a;
             k_grad_coef<<<(unsigned)((rows * d.n_comp + 127) / 128), 128, 0, g->stream>>>(d, rows);
-            k_grad_adjoint<<<g->n_cells, g->adj_threads, g->smem_adj, g->stream>>>(d, g->dims, rows, g->ring, g->stage, last ? 1 : 0);
+            (g->ring > 0 ? k_grad_adjoint<true> : k_grad_adjoint<false>)
+                <<<g->n_cells, g->adj_threads, g->smem_adj, g->stream>>>(d, g->dims, rows, g->ring, g->stage, last ? 1 : 0);
             k_grad_terms<<<dim3(g->n_cells, chunks), 64, (size_t)64 * g->dims.slots * sizeof(double), g->stream>>>(d, rows);
             if (n_slot > 0)
                 k_grad_sum<<<(n_slot + 127) / 128, 128, 0, g->stream>>>(d, n_slot, g->d_slot_cell, chunks, a == 1 ? 1 : 0);
