@@ -122,7 +122,7 @@ inline std::string channel_routines(const EdenGpuChannelType *types, const std::
 struct Kinds {
     bool pulse = false, sine = false, ramp = false, pois = false, timed = false, syn = false, expone = false,
          exptwo = false, forest = false, izh = false, gateforms = false, clamp = false, gap = false, alpha = false,
-         current = false, gate_warps = false, far = false;
+         current = false, gate_warps = false, wide = false;
 };
 
 inline std::string kind_defines(const Kinds &k) {
@@ -144,7 +144,7 @@ inline std::string kind_defines(const Kinds &k) {
     def("EDEN_KIND_ALPHA", k.alpha);
     def("EDEN_KIND_CURRENT", k.current);
     def("EDEN_GATE_WARPS", k.gate_warps);
-    def("EDEN_FAR_RECORDS", k.far);
+    def("EDEN_WIDE_INPUTS", k.wide);
     return s;
 }
 

@@ -1412,7 +1412,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     std::vector<int32_t> un_nf0(n_unit), un_nf1(n_unit), un_ch0(n_unit), un_ch1(n_unit), nf_t;
     std::vector<int> un_words(n_unit);
     std::vector<uint8_t> un_far(n_unit, 0);
-    bool far = false;  // for any unit
+    bool wide = n_chunk > n_block;  // blocks of several chunks, or units too large (forest_window)
     const int most = (int)(ctx->smem_optin / sizeof(float)) - 4 * kPassPad;  // words of one block
     for (int u = 0; u < n_unit; u++) {
         const int a = un_t0[u], b = un_t1[u];
@@ -1519,7 +1519,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             if (un_words[u] > most) {
                 un_words[u] = words(true);
                 un_far[u] = 1;
-                far = true;
+                wide = true;
             }
         } else {
             un_words[u] = izh_words(b - a);
@@ -1972,7 +1972,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // batched mode uses them (codegen >= 0) and NVRTC is available, else the
     // built-in ones (codegen = 1 makes a failed compile an error)
     ctx->fn_inputs = (const void *)k_inputs_t;
-    ctx->fn_cells = far ? (const void *)k_cells_far_t : (const void *)k_cells_t;
+    ctx->fn_cells = wide ? (const void *)k_cells_t<true> : (const void *)k_cells_t<false>;
     ctx->fn_deliver = (const void *)k_deliver_t;
     const int codegen = opt ? opt->codegen : 0;
     if (ctx->mode == EDEN_MODE_BATCHED && ctx->smem_window && codegen >= 0) {
@@ -1999,7 +1999,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         kinds.forest = d.n_forest > 0;
         kinds.gateforms = gate_forms;
         kinds.gate_warps = gate_warp;
-        kinds.far = far;
+        kinds.wide = wide;
         kinds.izh = n_izh > 0;
         kinds.gap = m->n_gap > 0 || m->n_graded > 0;
         ctx->codegen_source = eden_codegen::program_source(eden_codegen::kind_defines(kinds) +

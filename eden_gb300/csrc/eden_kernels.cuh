@@ -715,8 +715,8 @@ __device__ __forceinline__ void syn_window(const DevModel &m, int64_t it, const 
 #ifndef EDEN_GATE_WARPS
 #define EDEN_GATE_WARPS 1  // units' gates may have a warp of their own (DevModel::gate_warp)
 #endif
-#ifndef EDEN_FAR_RECORDS
-#define EDEN_FAR_RECORDS 0  // k_cells_t: units may keep records in global memory (DevModel::un_far)
+#ifndef EDEN_WIDE_INPUTS
+#define EDEN_WIDE_INPUTS 0  // a model with many inputs (k_cells_t)
 #endif
 
 // A timedSynapticInput item over the window: its synapse fires in each

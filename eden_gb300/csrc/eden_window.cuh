@@ -220,8 +220,7 @@ __global__ void __launch_bounds__(256) k_deliver_t(DevModel m, const WindowArgs 
 // chunks: those are summed over them here, a thread four steps.  In the steps it
 // would be a lane a block, one load after the other.  (One compartment of 128,000
 // inputs, a window of 29 steps: 742 us by steps, 129 so; 20 compartments with
-// 51,200 together: 102 and 87.  Called, not inlined: its registers are not the
-// steps'; one of 1,000 HH cells took 1.42 us with it inlined, 1.40 so.)
+// 51,200 together: 102 and 87.)
 __device__ __noinline__ void stage_sums(float *GS, const float *Gp, const int32_t *c0, int nblk, int gps, int th, int nth) {
     const int quads = gps >> 2;
     for (int i = th; i < nblk * quads; i += nth) {
@@ -270,9 +269,12 @@ __device__ __noinline__ void sum_blocks(float *Gk, const int4 *BK, int b0, int b
 // the loop that takes V over; with them, one body for both roles: compiled
 // apart, the solve of 50 trees took 112 us a window instead of 100.)
 //
-// FAR: a unit too large for a block's shared memory (un_far) reads its blocks'
-// records where they are; a step finds them in L1.
-template <bool FAR>
+// WIDE: for models with many inputs.  Blocks of several chunks are summed as they
+// are staged (stage_sums), and a unit too large for a block's shared memory (un_far)
+// reads its blocks' records where they are; a step finds them in L1.  (Without it
+// a block has one chunk.  One kernel for both: 2,000 trees, the built-in kernels,
+// 8.08 us a step, 7.19 apart; with the body in a function of its own the same 8.08.)
+template <bool WIDE>
 __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArgs &w, int u, float *S, bool gates,
                                               int barrier, bool first) {
     const int lane = threadIdx.x & 31;
@@ -296,7 +298,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
     float *TX = S + twig_words(n + 1), *TV = TX + 32 * nw;
     float4 *CN = reinterpret_cast<float4 *>(TV + 32 * nw), *TR = CN + n + 1;
     float4 *NF = TR + 32 * nw;
-    const bool far = FAR && m.un_far[u] != 0;
+    const bool far = WIDE && m.un_far[u] != 0;
     int4 *BKs = reinterpret_cast<int4 *>(NF + kSlotRecs * nf);
     const int4 *BK = far ? m.bk_rec + ub0 : BKs;
     const int gps = m.gp_stride;
@@ -352,7 +354,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
         stage_word(&TV[i], &vsrc[t0 + (t >= 0 ? t : 0)]);
     }
     for (int i = th; i < ngt; i += nth) stage_word(&GT[i], &m.gate[gt0 + i]);
-    if (nck == nblk)
+    if (!WIDE || nck == nblk)
         for (int i = 4 * th; i < gps * nck; i += 4 * nth) stage_rec(&GS[i], &m.Gp[(size_t)uc0 * gps + i]);
     else
         stage_sums(GS, m.Gp, m.bk_c0 + ub0, nblk, gps, th, nth);
@@ -552,6 +554,7 @@ __device__ __forceinline__ void forest_window(const DevModel &m, const WindowArg
 #else
 #define EDEN_IZH_CALL __forceinline__
 #endif
+template <bool WIDE>
 __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w, const float *tk, int u, float *S,
                                            bool first) {
     const int lane = threadIdx.x & 31;
@@ -583,9 +586,8 @@ __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w,
     const int ub0 = m.t_blk0[t0];
     const int b0 = lane < n ? m.t_blk0[t0 + lane] - ub0 : 0, b1 = lane < n ? m.t_blk0[t0 + lane + 1] - ub0 : 0;
     const int4 *BK = m.bk_rec + ub0;
-    const int uc0 = m.bk_c0[ub0], nblk = m.t_blk0[t0 + n] - ub0;
-    float *Gk = m.Gp + (size_t)uc0 * m.gp_stride;
-    if (m.bk_c0[ub0 + nblk] - uc0 > nblk) sum_blocks(Gk, BK, b0, b1, m.gp_stride, w.K);
+    float *Gk = m.Gp + (size_t)m.bk_c0[ub0] * m.gp_stride;
+    if (WIDE) sum_blocks(Gk, BK, b0, b1, m.gp_stride, w.K);
     const int src = lane < n ? m.t_src[t0 + lane] : -1;
     uint32_t spikes = 0;
     for (int k = 0; k < w.K; k++) {
@@ -647,9 +649,15 @@ __device__ EDEN_IZH_CALL void izh_window(const DevModel &m, const WindowArgs &w,
 // A block runs several CTAs in turn when there are more CTAs than blocks;
 // their units are laid out differently in shared memory, so every warp of
 // the block finishes its unit before any starts on the next CTA.
-template <bool FAR>
-__device__ __forceinline__ void cells(const DevModel &m, const WindowArgs *tab, const WindowTimes *ttab, const int *base,
-                                      int idx, int cta_begin, int cta_end) {
+// WIDE: for models with many inputs (forest_window); compiled for a model, as it is.
+#ifdef EDEN_RTC
+constexpr bool WIDE = EDEN_WIDE_INPUTS != 0;
+#else
+template <bool WIDE>
+#endif
+__global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
+                                                          const WindowTimes *ttab, const int *base, int idx,
+                                                          int cta_begin, int cta_end) {
     extern __shared__ __align__(16) float sm[];
     const WindowArgs w = tab[*base + idx];
     const float *tk = ttab[*base + idx].tk;
@@ -662,25 +670,12 @@ __device__ __forceinline__ void cells(const DevModel &m, const WindowArgs *tab, 
         const int u = m.cta_u0[cta] + slot;
         if (u < m.cta_u0[cta + 1]) {
             if (m.un_f[u] >= 0) {
-                if (EDEN_KIND_FOREST) forest_window<FAR>(m, w, u, sm + m.un_off[u], gates, 1 + slot, first);
-            } else if (EDEN_KIND_IZH && !gates) izh_window(m, w, tk, u, sm + m.un_off[u], first);
+                if (EDEN_KIND_FOREST) forest_window<WIDE>(m, w, u, sm + m.un_off[u], gates, 1 + slot, first);
+            } else if (EDEN_KIND_IZH && !gates) izh_window<WIDE>(m, w, tk, u, sm + m.un_off[u], first);
         }
         if (cta + (int)gridDim.x < cta_end) __syncthreads();
     }
 }
-__global__ void __launch_bounds__(kCellThreads, 1) k_cells_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
-                                                          const WindowTimes *ttab, const int *base, int idx,
-                                                          int cta_begin, int cta_end) {
-    cells<EDEN_FAR_RECORDS != 0>(m, tab, ttab, base, idx, cta_begin, cta_end);
-}
-#ifndef EDEN_RTC
-// for a model with a unit that keeps records in global memory
-__global__ void __launch_bounds__(kCellThreads, 1) k_cells_far_t(const __grid_constant__ DevModel m, const WindowArgs *tab,
-                                                              const WindowTimes *ttab, const int *base, int idx,
-                                                              int cta_begin, int cta_end) {
-    cells<true>(m, tab, ttab, base, idx, cta_begin, cta_end);
-}
-#endif
 
 __global__ void k_bump(int *base, int by) { *base += by; }
 
