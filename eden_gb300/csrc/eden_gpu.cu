@@ -2247,14 +2247,17 @@ static int launch_window(EdenGpuCtx *ctx, const int *base, int idx, int K) {
     launch_order(true, (const void *)k_targets_t, ctx->grid_targets, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab,
                  (const WindowTimes *)ctx->d_wtimes, base, idx);
     tmark(ctx, EDEN_KERNEL_TARGETS, false);
-    tmark(ctx, EDEN_KERNEL_HINES, true);
-    launch_order(true, (const void *)k_hines_t, ctx->grid_hines, kHinesThreads, ctx->smem_hines, s, d,
-                 (const WindowArgs *)ctx->d_wtab, base, idx, ctx->forest_cap);
-    tmark(ctx, EDEN_KERNEL_HINES, false);
+    // (a network of point neurons alone has nothing to solve)
+    if (d.n_forest > 0) {
+        tmark(ctx, EDEN_KERNEL_HINES, true);
+        launch_order(true, (const void *)k_hines_t, ctx->grid_hines, kHinesThreads, ctx->smem_hines, s, d,
+                     (const WindowArgs *)ctx->d_wtab, base, idx, ctx->forest_cap);
+        tmark(ctx, EDEN_KERNEL_HINES, false);
+    }
     tmark(ctx, EDEN_KERNEL_DELIVER, true);
     launch_order(true, ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, d, (const WindowArgs *)ctx->d_wtab, base, idx);
     tmark(ctx, EDEN_KERNEL_DELIVER, false);
-    return 4;
+    return d.n_forest > 0 ? 4 : 3;
 }
 
 static int run_windows(EdenGpuCtx *ctx, int64_t first_step, int64_t n_steps);
@@ -2714,9 +2717,10 @@ static int launch_window_static(EdenGpuCtx *ctx, const DevModel &dm, const Windo
     }
     launch_k(ctx->fn_inputs, ctx->grid_inputs, kInputThreads, ctx->smem_inputs, s, dm, tab, times, zero, idx);
     k_targets_t<<<ctx->grid_targets, kThreads, 0, s>>>(dm, tab, times, zero, idx);
-    k_hines_t<<<ctx->grid_hines, kHinesThreads, ctx->smem_hines, s>>>(dm, tab, zero, idx, ctx->forest_cap);
+    if (dm.n_forest > 0)
+        k_hines_t<<<ctx->grid_hines, kHinesThreads, ctx->smem_hines, s>>>(dm, tab, zero, idx, ctx->forest_cap);
     launch_k(ctx->fn_deliver, ctx->grid_deliver, kThreads, 0, s, dm, tab, zero, idx);
-    return 4;
+    return dm.n_forest > 0 ? 4 : 3;
 }
 
 static int run_static(EdenGpuCtx *ctx, int64_t first_step, int64_t n_steps);

@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kHinesThreads) k_hines_t(DevModel m, const Win
         __syncwarp();
         forest_spikes(m, f, src, w.step0, w.t0, x, vin, 0, w.wpar);
     }
-    // Warps without a forest wait as well, and in a network without any all do: a
-    // grid that ended without it would let the delivery, which waits for this
-    // grid only, start while the targets' kernel still runs.
+    // Warps without a forest wait as well: a grid that ended without it would let
+    // the delivery, which waits for this grid only, start while the targets' kernel
+    // still runs.  (Of a network without any forest it is not launched.)
     if (!waited) kernel_order();
 }
 

@@ -19,6 +19,8 @@ def _run(low, pieces, **options):
     out = []
     for n in pieces:
         sim.run_steps(n)
+        # inputs, neurons, delivery: nothing is launched for the cables that are not there
+        assert sim.last_launches == 3 * n
         rec = sim.fetch()
         out += [rec.spike_src, rec.spike_step, rec.trace, sim.read_v()]
     sim.close()
