@@ -106,3 +106,28 @@ def test_a_refused_fetch_takes_nothing():
         np.testing.assert_array_equal(getattr(b, name), getattr(a, name))
     want.close()
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 4096, 4097])
+def test_potentials_in_the_callers_order(n):
+    """Few potentials are put in order on the host, many on the device: written,
+    read, and written again between steps, they are the ones the next steps start
+    from."""
+    low = lowering.lower(workloads.single_comp_hh(n_cells=n, length_ms=5.0, n_recorded=1))
+    v = np.random.default_rng(n).uniform(-75.0, -55.0, n).astype(np.float32)
+    traces = []
+    for target in (0, n - 1):
+        sim = Simulation(low, trace_target=[target], record_capacity_steps=64)
+        sim.initialize()
+        np.testing.assert_array_equal(sim.read_v(), np.float32(-65.0))
+        sim.write_v(v)
+        w = v.copy()
+        v[:] = 0.0      # the caller's array is its own again
+        np.testing.assert_array_equal(sim.read_v(), w)
+        sim.write_v(w)
+        sim.run_steps(20)
+        traces.append(sim.fetch().trace[0, 0])
+        assert traces[-1] == w[target]
+        assert not np.array_equal(sim.read_v(), w)
+        v[:] = w
+        sim.close()
