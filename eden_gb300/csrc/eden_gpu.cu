@@ -942,6 +942,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             }
         }, 32);
     }
+    phase("nodes");
     // ---- nodes and twigs of each forest (DevModel::c_rec, hines_window), forests
     // on the host's threads.  A twig is a flat subtree of at most `most`
     // compartments; the twigs go to the lanes, large ones first, each to the
@@ -956,16 +957,26 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         std::vector<uint32_t> adr;
     };
     std::vector<ForestRec> frec(fo_t0.size());
+    // (a thread for every 8,192 compartments)
+    const int64_t grain = std::max<int64_t>(1, (int64_t)fo_t0.size() * 8192 / std::max(n_comp, 1));
     std::vector<int32_t> node_of(nt, -1), place_of(nt, -1);  // each compartment's node or twig place
     std::vector<char> no_pass(nt, 0);
-    const bool make_twigs = !opt || opt->mode == EDEN_MODE_BATCHED;
+    const bool windows = opt && opt->mode == EDEN_MODE_BATCHED;
     parallel_for((int64_t)fo_t0.size(), [&](int64_t f) {
         const int a = fo_t0[f], n = fo_t1[f] - a;
-        if (n > 1023) return;  // (such a forest runs the per-step kernels)
+        // (the per-step kernels, which run such a forest and this mode, do without)
+        if (n > 1023 || !windows) return;
         ForestRec &fr = frec[f];
-        std::vector<int32_t> size(n, 1), depth(n, 0);  // (non-flat compartments: size over any limit)
+        // (scratch of the thread, for all its forests)
+        static thread_local std::vector<int32_t> size, depth, count, kids, twigs, load, nodes, tops;
+        static thread_local std::vector<int32_t> lane[32];
+        static thread_local std::vector<std::pair<int32_t, int32_t>> stack;
+        size.assign(n, 1);  // (non-flat compartments: size over any limit)
+        depth.assign(n, 0);
+        int flat = 0;  // compartments of the largest flat subtree
         for (int i = n - 1; i >= 0; i--) {
             if (nonflat[a + i]) size[i] = 1 << 20;
+            else flat = std::max(flat, size[i]);
             if (c_parent[a + i] >= 0) size[c_parent[a + i] - a] += size[i];
         }
         for (int i = 0; i < n; i++)
@@ -976,40 +987,50 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             return size[c_parent[a + i] - a] > most ? 1 : 2;
         };
         int best = 0;
-        if (!fo_f64[f] && make_twigs) {
+        if (!fo_f64[f] && flat > 0) {
             int64_t cheapest = INT64_MAX;
             for (int most : {0, 3, 6, 9, 12, 16, 20, 26, 32, 40, 50, 64}) {
-                std::vector<int32_t> count(fo_nlev[f], 0), kids(fo_nlev[f], 0);
-                std::vector<int32_t> twigs;
+                count.assign(fo_nlev[f], 0);
+                kids.assign(fo_nlev[f], 0);
+                twigs.clear();
+                int places = 0;
                 for (int i = 0; i < n; i++) {
                     const int q = part(most, i);
                     if (q == 0) { count[depth[i]]++; kids[depth[i]] = std::max(kids[depth[i]], c_nchild[a + i]); }
-                    else if (q == 1) twigs.push_back(size[i]);
+                    else if (q == 1) { twigs.push_back(size[i]); places += size[i]; }
                 }
-                std::sort(twigs.begin(), twigs.end(), std::greater<int>());
-                int rows = 0;
-                {
-                    std::vector<int> load(32, 0);
-                    for (int t : twigs) {
-                        auto l = std::min_element(load.begin(), load.end());
-                        *l += t;
-                        rows = std::max(rows, *l);
-                    }
-                }
-                int64_t cost = 22 * (int64_t)rows;
+                int64_t cost = 0;
                 for (int l = 0; l < fo_nlev[f]; l++) cost += (count[l] + 31) / 32 * (42 + 5 * kids[l]);
-                // (addresses of twig places have 15 bits)
-                const int words = twig_words(n + 1) + 64 * rows;
-                if (cost < cheapest && words < (int)kTwigTop) { cheapest = cost; best = most; }
+                // (rows are at least these; the twigs are dealt out only where that can be cheapest)
+                std::sort(twigs.begin(), twigs.end(), std::greater<int>());
+                int rows = twigs.empty() ? 0 : std::max((places + 31) / 32, twigs[0]);
+                if (cost + 22 * (int64_t)rows < cheapest) {
+                    load.assign(32, 0);  // a heap of the lanes' loads, the least first
+                    for (int t : twigs) {
+                        std::pop_heap(load.begin(), load.end(), std::greater<int>());
+                        load.back() += t;
+                        rows = std::max(rows, load.back());
+                        std::push_heap(load.begin(), load.end(), std::greater<int>());
+                    }
+                    cost += 22 * (int64_t)rows;
+                    // (addresses of twig places have 15 bits)
+                    const int words = twig_words(n + 1) + 64 * rows;
+                    if (cost < cheapest && words < (int)kTwigTop) { cheapest = cost; best = most; }
+                }
+                if (most >= flat) break;  // (a larger one makes the same twigs)
             }
         }
         // nodes, in the compartments' order: a depth's are consecutive, and a node's children
-        std::vector<int32_t> nodes, tops;
+        nodes.clear();
+        tops.clear();
         for (int i = 0; i < n; i++) {
             const int q = part(best, i);
             if (q < 2) { node_of[a + i] = (int)nodes.size(); nodes.push_back(i); }
             if (q == 1) tops.push_back(i);
         }
+        fr.node.reserve(nodes.size());
+        fr.rt.reserve(nodes.size());
+        fr.nd_t.reserve(nodes.size());
         for (int i : nodes) {
             const int it = a + i, q = part(best, i);
             const uint32_t nk = q == 0 ? (uint32_t)c_nchild[it] : 0u;
@@ -1053,11 +1074,11 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         }
         // the twigs' places
         std::stable_sort(tops.begin(), tops.end(), [&](int x, int y) { return size[x] > size[y]; });
-        std::vector<std::vector<int32_t>> lane(32);
+        for (auto &l : lane) l.clear();
         for (int t : tops) {
-            auto l = std::min_element(lane.begin(), lane.end(), [](const auto &x, const auto &y) { return x.size() < y.size(); });
+            auto l = std::min_element(std::begin(lane), std::end(lane), [](const auto &x, const auto &y) { return x.size() < y.size(); });
             // children first, in increasing order
-            std::vector<std::pair<int32_t, int32_t>> stack{{t, 0}};
+            stack.assign(1, {t, 0});
             while (!stack.empty()) {
                 auto &[i, k] = stack.back();
                 if (k < c_nchild[a + i]) {
@@ -1076,6 +1097,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             for (size_t r = 0; r < lane[l].size(); r++) place_of[a + lane[l][r]] = (int32_t)(32 * r + l);
         fr.place.assign(32 * rows, make_float4(0.f, 0.f, 0.f, 0.f));
         fr.tw_t.assign(32 * rows, -1);
+        fr.adr.reserve(32 * rows);
         // (an empty place works on itself, with zeros)
         for (size_t k = 0; k < 32 * rows; k++) fr.adr.push_back((uint32_t)(base + k) | (uint32_t)(tv + k) << 16);
         for (int l = 0; l < 32; l++)
@@ -1088,24 +1110,29 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                 fr.adr[k] = top ? (uint32_t)(2 * node_of[it]) | kTwigTop | (uint32_t)(2 * node_of[up]) << 16
                                 : (uint32_t)(base + place_of[up]) | (uint32_t)(tv + place_of[up]) << 16;
             }
-    }, 32);
-    std::vector<float4> c_rec, tw_rec;
-    std::vector<float> nd_rt;
-    std::vector<int32_t> fo_n0(fo_t0.size() + 1, 0), fo_w0(fo_t0.size() + 1, 0), fo_p0(fo_t0.size() + 1, 0), nd_t, tw_t, ps;
-    std::vector<uint32_t> tw_adr;
+    }, grain);
+    std::vector<int32_t> fo_n0(fo_t0.size() + 1, 0), fo_w0(fo_t0.size() + 1, 0), fo_p0(fo_t0.size() + 1, 0);
     for (size_t f = 0; f < fo_t0.size(); f++) {
-        const ForestRec &fr = frec[f];
-        c_rec.insert(c_rec.end(), fr.node.begin(), fr.node.end());
-        nd_rt.insert(nd_rt.end(), fr.rt.begin(), fr.rt.end());
-        nd_t.insert(nd_t.end(), fr.nd_t.begin(), fr.nd_t.end());
-        ps.insert(ps.end(), fr.ps.begin(), fr.ps.end());
-        tw_rec.insert(tw_rec.end(), fr.place.begin(), fr.place.end());
-        tw_t.insert(tw_t.end(), fr.tw_t.begin(), fr.tw_t.end());
-        tw_adr.insert(tw_adr.end(), fr.adr.begin(), fr.adr.end());
-        fo_n0[f + 1] = (int32_t)c_rec.size();
-        fo_w0[f + 1] = (int32_t)(tw_t.size() / 32);
-        fo_p0[f + 1] = (int32_t)ps.size();
+        fo_n0[f + 1] = fo_n0[f] + (int32_t)frec[f].node.size();
+        fo_w0[f + 1] = fo_w0[f] + (int32_t)(frec[f].tw_t.size() / 32);
+        fo_p0[f + 1] = fo_p0[f] + (int32_t)frec[f].ps.size();
     }
+    const size_t nn = fo_n0.back(), nw = 32 * (size_t)fo_w0.back();
+    std::vector<float4> c_rec(nn), tw_rec(nw);
+    std::vector<float> nd_rt(nn);
+    std::vector<int32_t> nd_t(nn), tw_t(nw), ps(fo_p0.back());
+    std::vector<uint32_t> tw_adr(nw);
+    parallel_for((int64_t)fo_t0.size(), [&](int64_t f) {
+        ForestRec &fr = frec[f];
+        std::copy(fr.node.begin(), fr.node.end(), c_rec.begin() + fo_n0[f]);
+        std::copy(fr.rt.begin(), fr.rt.end(), nd_rt.begin() + fo_n0[f]);
+        std::copy(fr.nd_t.begin(), fr.nd_t.end(), nd_t.begin() + fo_n0[f]);
+        std::copy(fr.ps.begin(), fr.ps.end(), ps.begin() + fo_p0[f]);
+        std::copy(fr.place.begin(), fr.place.end(), tw_rec.begin() + 32 * (size_t)fo_w0[f]);
+        std::copy(fr.tw_t.begin(), fr.tw_t.end(), tw_t.begin() + 32 * (size_t)fo_w0[f]);
+        std::copy(fr.adr.begin(), fr.adr.end(), tw_adr.begin() + 32 * (size_t)fo_w0[f]);
+        fr = ForestRec();
+    }, grain);
     frec.clear();
 
     // kinds and timeCourse / steadyState forms of the gates of other kinds
