@@ -151,6 +151,7 @@ class Simulation:
             self.close()
             raise EdenGpuError(rc, msg)
         self.next_step = -3
+        self._first_row = 1  # the first step not yet fetched
         self.n_target = lowered.n_target
 
     def _err(self) -> str:
@@ -193,30 +194,31 @@ class Simulation:
         return float(ms.value)
 
     def fetch(self) -> Records:
-        cap = self.record_capacity_steps
-        nt = max(len(self.trace_target), 1)
-        trace = np.empty((cap, nt), np.float32)
-        tstep = np.empty(cap, np.int64)
+        nt = len(self.trace_target)
         rec = CRecords()
-        rec.trace = trace.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
-        rec.trace_step = tstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
-        rec.trace_capacity = cap
-        # room for as many spikes as there are: a small buffer first, and, where
-        # the call says that it takes more, that many
+        # room for the rows there should be, and for a few spikes; where the call says
+        # that it takes more, that much, up to the capacities
+        rows = min(max(self.next_step - self._first_row, 0), self.record_capacity_steps)
         room = min(4096, self.spike_capacity)
         while True:
+            trace, tstep = np.empty((rows, max(nt, 1)), np.float32), np.empty(rows, np.int64)
             ssrc, sstep, stime = np.empty(room, np.int32), np.empty(room, np.int64), np.empty(room, np.float64)
+            rec.trace = trace.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
+            rec.trace_step = tstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+            rec.trace_capacity = rows
             rec.spike_src = ssrc.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
             rec.spike_step = sstep.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
             rec.spike_capacity = room
             rec.spike_time_us = stime.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
             rc = self.lib.edenGpuFetchRecords(self.ctx, ctypes.byref(rec))
-            if rc == 0 or not room < rec.n_spikes <= self.spike_capacity:
+            n, m = int(rec.n_trace_samples), int(rec.n_spikes)
+            if rc == 0 or not (rows < n <= self.record_capacity_steps or room < m <= self.spike_capacity):
                 break
-            room = int(rec.n_spikes)
+            rows, room = max(rows, min(n, self.record_capacity_steps)), max(room, min(m, self.spike_capacity))
+        self._first_row = max(1, self.next_step)
         self._check(rc)
-        n, m = int(rec.n_trace_samples), int(rec.n_spikes)
-        return Records(trace[:n, :len(self.trace_target)], tstep[:n], ssrc[:m], sstep[:m], stime[:m])
+        # (a few spikes do not keep the buffers)
+        return Records(trace[:n, :nt], tstep[:n], *(a[:m] if 4 * m >= room else a[:m].copy() for a in (ssrc, sstep, stime)))
 
     def run(self, n_steps: int | None = None, chunk: int | None = None) -> Records:
         """Initialise, then run n_steps non-initialisation steps (default: the

@@ -131,3 +131,17 @@ def test_potentials_in_the_callers_order(n):
         assert not np.array_equal(sim.read_v(), w)
         v[:] = w
         sim.close()
+
+
+def test_records_do_not_keep_the_buffers():
+    """A program that fetches often and keeps the records holds what is in them."""
+    low = lowering.lower(workloads.single_comp_hh(n_cells=50, length_ms=20.0, n_recorded=10))
+    sim = Simulation(low, record_capacity_steps=4096)
+    sim.initialize()
+    sim.run_steps(7)
+    rec = sim.fetch()
+    sim.close()
+    assert rec.trace.shape == (7, 10)
+    for a in (rec.trace, rec.trace_step, rec.spike_src, rec.spike_step, rec.spike_time):
+        held = a if a.base is None else a.base
+        assert held.nbytes == a.nbytes
