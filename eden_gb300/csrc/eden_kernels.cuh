@@ -1209,15 +1209,14 @@ __device__ __forceinline__ void block_currents_rec(const float *Gk, const int4 *
             Iin -= v * g;
             continue;
         }
-        // a current is its value times 1, and adds no conductance; the sums a
-        // block is not part of take 0 * anything finite: no branches
-        const bool current = kind == BK_PULSE || (EDEN_KIND_CURRENT && (r.z & BK_CURRENT));
-        const float t = current ? 1.0f : __int_as_float(r.w) - v;
-        const float gi = kind == BK_SYN ? 0.0f : g, gs = kind == BK_SYN ? g : 0.0f;
-        Iin = fmaf(gi, t, Iin);
-        Isyn = fmaf(gs, t, Isyn);
-        Gin += current ? 0.0f : gi;
-        Gsyn += current ? 0.0f : gs;
+        // a current is its value times 1, and adds no conductance; the sum a block
+        // is not part of stays as it is, whatever the potential: no branches
+        const bool current = kind == BK_PULSE || (EDEN_KIND_CURRENT && (r.z & BK_CURRENT)), syn = kind == BK_SYN;
+        const float sum = fmaf(g, current ? 1.0f : __int_as_float(r.w) - v, syn ? Isyn : Iin);
+        Iin = syn ? Iin : sum;
+        Isyn = syn ? sum : Isyn;
+        Gin += current || syn ? 0.0f : g;
+        Gsyn += current || !syn ? 0.0f : g;
     }
 }
 

@@ -11,7 +11,7 @@ import pytest
 import eden_port
 from criteria import box_violations, samecount
 from eden_gb300 import lowering
-from eden_gb300.engine import Simulation
+from eden_gb300.engine import MODE_PLAIN, Simulation
 from eden_gb300.network import (SYN_EXPONE, SYN_EXPTWO, ChannelDensity, Izhikevich2007Cell, NetworkSpec, OutputColumn,
                                 PhysicalCell, PoissonInputs, Population, PulseInputs, SynapseType, hh_channels)
 from helpers import spike_trains
@@ -66,3 +66,24 @@ def test_blocks_of_many_chunks(point, K):
     assert not wrong and not far
     nbad, worst = box_violations(ref["trace"], a.trace, dt_ms, 0.1, 0.5)
     assert nbad == 0, f"{nbad} samples outside box(0.1 ms, 0.5 mV), worst by {worst} mV"
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_potentials_that_are_not_finite(value):
+    """An input adds nothing to a sum it is not part of, whatever the potential:
+    what overflows to infinity or NaN in windows is what does step by step."""
+    low = _network(True)
+    out = []
+    for options in (dict(mode=MODE_PLAIN), dict(steps_per_launch=1)):
+        sim = Simulation(low, **options)
+        sim.initialize()
+        sim.run_steps(100)
+        v = sim.read_v()
+        v[::2] = value
+        sim.write_v(v)
+        sim.run_steps(1)
+        out.append(sim.read_v())
+        sim.close()
+    for f in (np.isnan, np.isposinf, np.isneginf):
+        np.testing.assert_array_equal(f(out[0]), f(out[1]))
+    assert np.isfinite(out[0][1::2]).all()
