@@ -106,10 +106,10 @@ struct EdenGpuCtx {
     int *d_base = nullptr;      // chunk base read by graph-launched kernels
     int *d_zero = nullptr;      // always 0, for direct launches
     cudaGraphExec_t graph = nullptr;
-    int grid_inputs = 0, grid_targets = 0, grid_hines = 0, grid_deliver = 0, grid_window = 0;
+    int grid_inputs = 0, grid_targets = 0, grid_hines = 0, grid_deliver = 0;
     int n_sm_unused = 0;
     int smem_per_sm = 0, smem_optin = 0;   // bytes
-    int gcap = 0, forest_cap = 0;           // largest cell / compartments per staged forest
+    int forest_cap = 0;                    // compartments per staged forest
     bool smem_window = false;              // groups fit shared memory
     int max_cell_blocks = 0;               // most blocks of a k_cells_t launch
     int cell_threads = 128;                // threads of a k_cells_t block
@@ -574,32 +574,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             }
         }
     }
-    // per-cell work estimate (inputs dominate) to balance groups
-    std::vector<int64_t> n_in_user(nt, 0);
-    for (int64_t s = 0; s < m->n_syn; s++) n_in_user[m->syn_target[s]]++;
-    for (int64_t k = 0; k < m->n_pois; k++) n_in_user[m->pois_target[k]]++;
-    for (int64_t k = 0; k < m->n_timed; k++) n_in_user[m->timed_target[k]]++;
-    for (int64_t k = 0; k < m->n_pulse; k++) n_in_user[m->pulse_target[k]]++;
-    for (int64_t k = 0; k < m->n_wave; k++) n_in_user[m->wave_target[k]]++;
-    for (int64_t k = 0; k < m->n_clamp; k++) n_in_user[m->clamp_target[k]] += 2;
-    for (int64_t k = 0; k < m->n_gap; k++) n_in_user[m->gap_target[k]]++;
-    for (int64_t k = 0; k < m->n_graded; k++) n_in_user[m->graded_target[k]]++;
-    std::vector<double> cost(n_cells, 0.0);
-    double total = 0;
-    int max_cell = 1;
-    for (int g = 0; g < n_cells; g++) {
-        double c = 0;
-        if (cell_phys[g] >= 0) {
-            int a = m->phys_comp_off[cell_phys[g]], b = m->phys_comp_off[cell_phys[g] + 1];
-            for (int i = a; i < b; i++)
-                c += 6.0 + n_in_user[i] + 8.0 * (m->comp_chan_off[i + 1] - m->comp_chan_off[i]);
-            max_cell = std::max(max_cell, b - a);
-        } else if (cell_izh[g] >= 0) {
-            c = 6.0 + n_in_user[n_comp + cell_izh[g]];
-        }
-        cost[g] = c;
-        total += c;
-    }
 
     // ---- diagonal dominance: row i of a cell's backward-Euler cable matrix
     // (eden/Eden.cpp:6114-6225) has 1 + dt (G_i / C_i + sum_j 1/(R_ij C_i))
@@ -841,7 +815,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             c_cend[it] = run;
         }
     }
-    ctx->gcap = max_cell;
     ctx->forest_cap = max_forest;
     phase("constants");
     // ---- per-target constants in internal order
@@ -1295,7 +1268,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     std::vector<uint8_t> bk_type;
     std::vector<float> bk_erev;
     std::vector<int64_t> bk_i0, bk_i1;
-    std::vector<int32_t> in_tgt;
+    int n_in = 0;  // targets with inputs
     for (int t = 0; t < nt; t++) {
         t_blk0[t] = (int32_t)bk_kind.size();
         if (qoff[t + 1] > qoff[t]) {
@@ -1341,7 +1314,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
             bk_i0.push_back(k); bk_i1.push_back(k1);
             k = k1;
         }
-        if ((int)bk_kind.size() > t_blk0[t]) in_tgt.push_back(t);
+        n_in += (int)bk_kind.size() > t_blk0[t];
     }
     t_blk0[nt] = (int32_t)bk_kind.size();
     const int n_block = (int)bk_kind.size();
@@ -1717,11 +1690,9 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     phase("upload");
     // ---- upload
     DevModel &d = ctx->d;
-    d.n_target = nt; d.n_src = m->n_src; d.n_unit = n_unit; d.n_forest = (int)fo_t0.size();
-    d.n_in = (int)in_tgt.size();
-    d.n_block = n_block;
+    d.n_target = nt; d.n_src = m->n_src; d.n_forest = (int)fo_t0.size();
     d.n_chunk = n_chunk;
-    d.n_syn = ns; d.n_pois = m->n_pois; d.dt = dt;
+    d.dt = dt;
     d.pois_exact = (dt == std::floor(dt) && dt <= 1048576.0f) ? 1 : 0;
     ctx->user_to_internal = u2i;
     TRY(upload_vec(ctx, &ctx->d_u2i, u2i));
@@ -1791,11 +1762,10 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
         TRY(upload_c(ctx, &d.gr_par, gr_par)); TRY(upload_c(ctx, &d.gr_w, gr_w));
         TRY(upload_vec(ctx, &d.gr_s, gr_s));
     }
-    TRY(upload_c(ctx, &d.in_tgt, in_tgt));
     TRY(upload_c(ctx, &d.t_blk0, t_blk0)); TRY(upload_c(ctx, &d.bk_kind, bk_kind));
-    TRY(upload_c(ctx, &d.bk_type, bk_type)); TRY(upload_c(ctx, &d.bk_erev, bk_erev));
-    TRY(upload_c(ctx, &d.bk_c0, bk_c0)); TRY(upload_c(ctx, &d.ck_blk, ck_blk));
-    TRY(upload_c(ctx, &d.ck_i0, ck_i0)); TRY(upload_c(ctx, &d.ck_n, ck_n));
+    TRY(upload_c(ctx, &d.bk_erev, bk_erev));
+    TRY(upload_c(ctx, &d.bk_c0, bk_c0));
+    TRY(upload_c(ctx, &d.ck_i0, ck_i0));
     TRY(upload_c(ctx, &d.ck_info, ck_info));
     TRY(upload(ctx, &d.Gp, (const float *)nullptr, (size_t)d.gp_stride * (size_t)std::max(n_chunk, 1)));
     TRY(upload(ctx, &d.ck_a, (const float *)nullptr, (size_t)std::max(n_chunk, 1)));
@@ -1820,11 +1790,10 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload_c(ctx, &d.po_rng, po_rng));
     TRY(upload_c(ctx, &d.wv_p, wv_p));
     TRY(upload_c(ctx, &d.cl_p, cl_p));
-    TRY(upload_c(ctx, &d.po_type, po_type));
     TRY(upload(ctx, &d.tm_a, (const float *)nullptr, (size_t)m->n_timed));
     TRY(upload(ctx, &d.tm_b, (const float *)nullptr, (size_t)m->n_timed));
     TRY(upload(ctx, &d.tm_last, (const int32_t *)nullptr, (size_t)m->n_timed));
-    TRY(upload_c(ctx, &d.tm_w, tm_w)); TRY(upload_c(ctx, &d.tm_type, tm_type));
+    TRY(upload_c(ctx, &d.tm_w, tm_w));
     TRY(upload_c(ctx, &d.tm_off, tm_off)); TRY(upload_c(ctx, &d.tm_step, tm_step));
     {
         // each item's cursor starts at its first listed step
@@ -1854,7 +1823,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     TRY(upload_vec(ctx, &d.sy_pend, sy_pend));
     TRY(upload(ctx, &d.sy_mask, (const uint32_t *)nullptr, (size_t)ns));
     TRY(upload_c(ctx, &d.sy_w, sy_w)); TRY(upload_c(ctx, &d.sy_delay, sy_d));
-    TRY(upload_c(ctx, &d.sy_type, sy_type));
     ctx->h_sy_type = sy_type;
     TRY(upload_c(ctx, &d.t_src, t_src)); TRY(upload_c(ctx, &d.src_thr, src_thr));
     TRY(upload_c(ctx, &d.fan0, fan0)); TRY(upload_c(ctx, &d.fan_syn, fan_syn));
@@ -1982,7 +1950,6 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     ctx->grid_hines = (int)std::max<int64_t>(1, ((int64_t)d.n_forest * 32 + kHinesThreads - 1) / kHinesThreads);
     ctx->grid_deliver = ctx->n_sm * 4;
     ctx->max_cell_blocks = (opt && opt->max_cell_blocks > 0) ? opt->max_cell_blocks : ctx->n_sm * 32;
-    ctx->grid_window = 0;
     // per-step Hines: each warp stages a forest of up to forest_cap compartments
     // (7 arrays plus depth boundaries); larger forests are solved in place
     const int hines_warps = kHinesThreads / 32;
@@ -2082,7 +2049,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
                 "libeden_gpu: K=%d, %d CTAs (%d thr, up to %zu B smem, %d/SM at the largest), %zu forests "
                 "(%.1f nodes, %.1f levels avg)\n"
                 "libeden_gpu: %d units, %zu size classes; inputs grid %d (%d/SM)\n",
-                nt, m->n_src, (long long)ns, (long long)m->n_pois, n_block, (int)in_tgt.size(), ctx->K,
+                nt, m->n_src, (long long)ns, (long long)m->n_pois, n_block, n_in, ctx->K,
                 (int)cta_words.size(), ctx->cell_threads, max_smem_class, occ_cells, fo_t0.size(),
                 fo_t0.empty() ? 0.0 : (double)fnodes / fo_t0.size(), fo_t0.empty() ? 0.0 : (double)flev / fo_t0.size(),
                 n_unit, ctx->classes.size(), ctx->grid_inputs, occ_inputs);

@@ -92,12 +92,11 @@ constexpr int kWaveWords = 8;    // waveform input record: delay, duration, 3 sh
 constexpr int kClampWords = 8;   // clamp record: delay, duration, 3 phase targets, R, weight, spare
 
 struct DevModel {
-    int32_t n_target, n_src, n_group, n_forest, n_in;
+    int32_t n_target, n_src, n_forest;
     // channel and synapse type tables (per context, so that contexts of
     // different models can run side by side)
     const ChanTypeDev *chan_types;
     const SynTypeDev *syn_types;
-    int64_t n_syn, n_pois;
     float dt;
     // targets
     float *v[2];
@@ -156,23 +155,18 @@ struct DevModel {
     const float *iz_p;
     float *iz_u, *iz_s;
     // input blocks: each target's pulses, then Poisson inputs and connection
-    // synapses in runs of one synapse type; a block's conductance (or, for
-    // pulses, current) for step k of the window is G[k * n_block + block]
-    int32_t n_block;
+    // synapses in runs of one synapse type; a block's value for a step of the window
+    // is its conductance (of pulses and currents, the current)
     const int32_t *t_blk0;            // [n_target + 1]
     const int32_t *bk_kind;           // BK_PULSE, BK_POIS, BK_SYN, BK_TIMED
-    const uint8_t *bk_type;           // synapse type of a Poisson / synapse block
     const float *bk_erev;
-    const int32_t *in_tgt;            // targets with any block
     // blocks are cut into chunks of at most kChunkItems items, one warp each; step k's
     // partial sum of chunk c is Gp[c * gp_stride + k] and a block's value is the
     // sum of its chunks' partials in chunk order
     int32_t n_chunk;
-    const int32_t *bk_c0;             // [n_block + 1] chunk range of each block
-    const int32_t *ck_blk;            // block of each chunk
+    const int32_t *bk_c0;             // [blocks + 1] chunk range of each block
     const int32_t *ck_info;           // kind | synapse type << 2 | items << 8
     const int64_t *ck_i0;             // first item of each chunk
-    const int32_t *ck_n;              // items in the chunk
     float *Gp;                        // [n_chunk * gp_stride]
     int32_t gp_stride;                // steps of the longest window, a multiple of four (1: per-step path)
     int32_t acc_stride;               // of the input kernel's event tiles: odd, at least those steps
@@ -189,14 +183,12 @@ struct DevModel {
     const float *po_rate, *po_w;
     const int32_t *po_seed, *po_inst;
     const int32_t *po_rng;                 // random-call id of the input's first draw
-    const uint8_t *po_type;
     // timedSynapticInput items: own synapse state (as Poisson items), weight,
     // type, the steps each fires in (tm_step[tm_off[i] .. tm_off[i+1]]) and
     // the next one due
     float *tm_a, *tm_b;
     int32_t *tm_last;
     const float *tm_w;
-    const uint8_t *tm_type;
     const int64_t *tm_off, *tm_step;
     int64_t *tm_cur;
     // connection synapses
@@ -206,7 +198,6 @@ struct DevModel {
     int32_t *sy_last;                 // step of that event
     uint32_t *sy_mask;
     const float *sy_w, *sy_delay;
-    const uint8_t *sy_type;
     // the targets of forest f that spike sources watch, fo_s[fo_s0[f] .. fo_s0[f + 1])
     const int32_t *fo_s0, *fo_s;
     // spike sources and fan-out (source -> synapses, connection order)
@@ -240,7 +231,6 @@ struct DevModel {
     // word un_off of its CTA, gates [un_gt0, un_gt0 + un_ngt) and recorded
     // targets gr_*[un_r0 .. un_r1) (target indices local to the unit); CTA c
     // runs units [cta_u0[c], cta_u0[c+1])
-    int32_t n_unit;
     const int32_t *un_t0, *un_t1, *un_f, *un_off, *un_gt0, *un_ngt, *un_r0, *un_r1;
     const int32_t *cta_u0;
     // per unit: trace columns [un_r0, un_r1): gr_t is the node << 1 or the twig
@@ -379,12 +369,6 @@ struct WindowTimes {
     float tk[32];
     float tprev[32];
 };
-
-__device__ __forceinline__ float warp_sum(float x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-}
 
 // ---------------------------------------------------------------------------
 // spike compaction: warp ballot, one atomic per warp
