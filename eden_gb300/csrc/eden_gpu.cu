@@ -1603,7 +1603,7 @@ static int build_and_upload(EdenGpuCtx *ctx, const EdenGpuModel *m, const EdenGp
     // V after the solve, and all units' two warps are resident together; where
     // they are not, the warps there are keep the SM busy and a second round
     // costs more than a shorter step gives.  (A window, one warp and two: 1,000
-    // HH cells 57 and 41 us, 30,011 76 and 64, 50 trees 110 and 100, 1,200
+    // HH cells 57 and 41 us, 30,011 76 and 62, 50 trees 110 and 100, 1,200
     // trees with active dendrites 231 and 189, 5,000 cells of 100 compartments
     // 111 and 100.)  At most four such CTAs an SM: the kernel names its barriers
     // at run time, so each CTA takes all 16, and with five or six, the last

@@ -430,7 +430,8 @@ int edenGpuRun(EdenGpuCtx *ctx, int64_t first_step, int64_t n_steps);
  * one that fails after (edenGpuRun too) leaves it refusing further runs. */
 int edenGpuRunStaticScratch(EdenGpuCtx *ctx, int64_t first_step, int64_t n_steps);
 
-/* Copy records accumulated since the last fetch into caller buffers. */
+/* Copy records accumulated since the last fetch into caller buffers.  Allocates
+ * no device memory: the log is put in order with what the context holds. */
 int edenGpuFetchRecords(EdenGpuCtx *ctx, EdenGpuRecords *rec);
 
 /* Read / write membrane potentials of all targets (n_comp + n_izh floats). */
