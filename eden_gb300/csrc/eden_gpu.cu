@@ -228,7 +228,8 @@ constexpr int64_t kLogHostSort = 1024;           // spikes a turn up to which th
 // bytes lie side by side in slabs, each one allocation, filled on the host and
 // copied once (flush_slabs); until then nothing else may write or read them.  (A
 // context of 100 cells, with an allocation and a copy for each array: 1.6 ms to
-// create and 0.68 to destroy; 0.75 and 0.39 so.)
+// create and 0.68 to destroy; 0.75 and 0.39 so, 0.8 together with the spike log
+// in one allocation.)
 constexpr size_t kSlabArray = 256 << 10, kSlabBytes = 1 << 20;
 
 int slab_place(EdenGpuCtx *ctx, void **p, const void *src, size_t n, size_t bytes) {
